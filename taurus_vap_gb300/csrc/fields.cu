@@ -380,6 +380,104 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock)
   }
 }
 
+// The fields of a few columns (CP = 1, 2, 4, 8 or 16 >= ncol): the lanes of a
+// warp split into CP columns x 32 / CP slots, slot t takes the entries t,
+// t + 32 / CP, ... of the row, and the partial sums of the slots meet in a
+// shuffle tree.  Blocks [0, gblocks) hold the rows of Gamma, the rest the
+// strict-lower entries of Delta.  With one column the kernels above keep one
+// lane busy on a serial chain of ~370 dependent FMAs per row; here the entry
+// list streams coalesced (12 B an entry, 106 MB at n = 140) and its rate is
+// the bound.  One column, n = 140: 978 + 480 us -> 82 us (cold).
+template <int CP>
+__global__ void __launch_bounds__(32 * kWarpsPerBlock)
+    gather_few_kernel(int n, int ncol, int ldc, unsigned gblocks, const int* __restrict__ g_rowptr,
+                      const int* __restrict__ g_src, const double* __restrict__ g_coef,
+                      const int* __restrict__ d_rowptr, const int* __restrict__ d_src,
+                      const double* __restrict__ d_coef, const double2* __restrict__ rho,
+                      const double2* __restrict__ kLR, const double2* __restrict__ kRL,
+                      const double2* __restrict__ H1, double2* __restrict__ gamma, double2* __restrict__ hsp,
+                      double2* __restrict__ dLR, double2* __restrict__ dRL) {
+  constexpr int kSlots = 32 / CP;
+  const int lane = threadIdx.x & 31;
+  const int col = lane % CP, slot = lane / CP;
+  const bool live = col < ncol;
+  auto total = [](double v) {
+#pragma unroll
+    for (int off = CP; off < 32; off <<= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
+    return v;
+  };
+  if (blockIdx.x < gblocks) {
+    const long long r = blockIdx.x * (long long)kWarpsPerBlock + (threadIdx.x >> 5);
+    if (r >= (long long)n * n) return;
+    double2 acc = make_double2(0.0, 0.0);
+    const int beg = g_rowptr[r], end = g_rowptr[r + 1];
+    if (live) {
+#pragma unroll 4
+      for (int e = beg + slot; e < end; e += kSlots) {
+        const double w = g_coef[e];
+        const double2 v = rho[(long long)g_src[e] * ldc + col];
+        acc.x = fma(w, v.x, acc.x);
+        acc.y = fma(w, v.y, acc.y);
+      }
+    }
+    acc.x = total(acc.x);
+    acc.y = total(acc.y);
+    if (slot == 0 && live) {
+      gamma[r * ldc + col] = acc;
+      hsp[r * ldc + col] = cadd(acc, H1[r]);
+    }
+    return;
+  }
+  // Delta: warp w holds entry (b, a), b >= a, of the row-wise lower triangle
+  const long long w = (blockIdx.x - gblocks) * (long long)kWarpsPerBlock + (threadIdx.x >> 5);
+  if (w >= (long long)n * (n + 1) / 2) return;
+  int b = int((sqrtf(8.0f * float(w) + 1.0f) - 1.0f) * 0.5f);
+  while ((long long)b * (b + 1) / 2 > w) --b;
+  while ((long long)(b + 1) * (b + 2) / 2 <= w) ++b;
+  const int a = int(w - (long long)b * (b + 1) / 2);
+  const long long r = b + (long long)a * n, rt = a + (long long)b * n;
+  double2 al = make_double2(0.0, 0.0), ar = make_double2(0.0, 0.0);
+  if (live && a != b) {
+    const int beg = d_rowptr[r], end = d_rowptr[r + 1];
+#pragma unroll 4
+    for (int e = beg + slot; e < end; e += kSlots) {
+      const double wt = d_coef[e];
+      const long long at = (long long)d_src[e] * ldc + col;
+      const double2 u = kLR[at], v = kRL[at];
+      al.x = fma(wt, u.x, al.x);
+      al.y = fma(wt, u.y, al.y);
+      ar.x = fma(wt, v.x, ar.x);
+      ar.y = fma(wt, v.y, ar.y);
+    }
+  }
+  al.x = total(al.x);
+  al.y = total(al.y);
+  ar.x = total(ar.x);
+  ar.y = total(ar.y);
+  if (slot == 0 && live) {
+    dLR[r * ldc + col] = al;
+    dRL[r * ldc + col] = ar;
+    if (a != b) {
+      dLR[rt * ldc + col] = make_double2(-al.x, -al.y);
+      dRL[rt * ldc + col] = make_double2(-ar.x, -ar.y);
+    }
+  }
+}
+
+template <int CP>
+void launch_fields_few(tvap_ctx* c, int ncol, int ldc, const double2* rho, const double2* kLR, const double2* kRL,
+                       double2* gamma, double2* hsp, double2* dLR, double2* dRL, cudaStream_t s) {
+  const int n = c->n;
+  const long long rows = (long long)n * n, tri = (long long)n * (n + 1) / 2;
+  const unsigned gb = unsigned((rows + kWarpsPerBlock - 1) / kWarpsPerBlock);
+  const unsigned db = unsigned((tri + kWarpsPerBlock - 1) / kWarpsPerBlock);
+  sec_begin_on(c, SEC_FIELDS_GAMMA, s);  // Gamma and Delta in one launch
+  gather_few_kernel<CP><<<gb + db, 32 * kWarpsPerBlock, 0, tvap::counted(s)>>>(
+      n, ncol, ldc, gb, c->csr.g_rowptr, c->csr.g_src, c->csr.g_coef, c->csr.d_rowptr, c->csr.d_src, c->csr.d_coef,
+      rho, kLR, kRL, c->d_H1, gamma, hsp, dLR, dRL);
+  sec_end_on(c, SEC_FIELDS_GAMMA, s);
+}
+
 template <int CPL>
 void launch_fields(tvap_ctx* c, int ncol, int ldc, const double2* rho, const double2* kLR, const double2* kRL,
                    double2* gamma, double2* hsp, double2* dLR, double2* dRL, cudaStream_t s) {
@@ -408,7 +506,17 @@ int fields_batched(tvap_ctx* c, int ncol, int ldc, const double2* rho, const dou
   // many gauge angles at once: dense symmetry blocks on the tensor cores
   if (c->gemm_mode >= 1 && c->csr.dense_ok && ncol >= kDenseMinCols)
     return fields_dense(c, ncol, ldc, rho, kLR, kRL, gamma, hsp, dLR, dRL, s);
-  if (ncol <= 32)
+  if (ncol == 1)
+    launch_fields_few<1>(c, ncol, ldc, rho, kLR, kRL, gamma, hsp, dLR, dRL, s);
+  else if (ncol == 2)
+    launch_fields_few<2>(c, ncol, ldc, rho, kLR, kRL, gamma, hsp, dLR, dRL, s);
+  else if (ncol <= 4)
+    launch_fields_few<4>(c, ncol, ldc, rho, kLR, kRL, gamma, hsp, dLR, dRL, s);
+  else if (ncol <= 8)
+    launch_fields_few<8>(c, ncol, ldc, rho, kLR, kRL, gamma, hsp, dLR, dRL, s);
+  else if (ncol <= 16)
+    launch_fields_few<16>(c, ncol, ldc, rho, kLR, kRL, gamma, hsp, dLR, dRL, s);
+  else if (ncol <= 32)
     launch_fields<1>(c, ncol, ldc, rho, kLR, kRL, gamma, hsp, dLR, dRL, s);
   else if (ncol <= 64)
     launch_fields<2>(c, ncol, ldc, rho, kLR, kRL, gamma, hsp, dLR, dRL, s);
