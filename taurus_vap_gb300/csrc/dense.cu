@@ -216,6 +216,128 @@ __global__ void __launch_bounds__((TM / 2) * (TN / 2)) gemm3m_kernel(GemmArgs g)
     }
 }
 
+// Small products (single matrices up to n ~ 220, batches of very small ones):
+// 8 x 8 outputs per CTA of 128 threads, one output per thread with K split
+// between the two warp pairs, the operands' rows staged for up to 96 - 192
+// values of k at once.  An FP64 warp instruction holds its sub-partition's
+// FP64 unit for about 64 cycles on this part, so a product of this size is
+// bound by how evenly its FMAs spread over the 4 x 152 units: four warps per
+// CTA (one per sub-partition), tiles of 64 outputs (324 CTAs at n = 140) and
+// one load latency per staging.  Measured (cold): real n = 24 10.1 -> 5.0 us
+// and n = 80 27.8 -> 8.7 us against 16 x 16 tiles with two warps of 4 outputs
+// a thread; real n = 140 27 us (two slicing passes and an mma.sync product)
+// -> 15.6 us.  M3: complex x complex with three real products (the sums
+// Re + Im formed once when the tile is staged).
+constexpr int kSmallT = 8;          // outputs per CTA side
+constexpr int kSmallLd = kSmallT + 1;
+constexpr int kSmallThreads = 128;
+// k per staging: the operands (and the sums of the 3M form) within 48 KB
+template <typename TA, typename TB>
+__host__ __device__ constexpr int small_kc() {
+  return sizeof(TA) + sizeof(TB) > 24 ? 96 : sizeof(TA) + sizeof(TB) > 16 ? 128 : 192;
+}
+// double precision multiply-adds of a product up to which it runs here
+constexpr double kSmallWork = 1.2e7;
+
+template <typename T>
+__device__ __forceinline__ void stage_small(T* dst, const View& v, bool rows_first, int r0, int rows, int k0, int kt,
+                                            long long b, bool conj) {
+  // rows_first: element (r0 + r, k0 + k); otherwise (k0 + k, r0 + r).
+  // Consecutive threads run along the operand's contiguous direction.
+  const long long r_step = rows_first ? v.rs : v.cs, k_step = rows_first ? v.cs : v.rs;
+  const bool k_fast = k_step < r_step;
+  for (int idx = threadIdx.x; idx < kSmallT * kt; idx += kSmallThreads) {
+    const int r = k_fast ? idx / kt : idx % kSmallT;
+    const int k = k_fast ? idx - r * kt : idx / kSmallT;
+    T x = zero_of<T>();
+    if (r0 + r < rows) {
+      x = static_cast<const T*>(v.p)[(r0 + r) * r_step + (k0 + k) * k_step + b * v.bs];
+      if constexpr (sizeof(T) == sizeof(double2))
+        if (conj) x.y = -x.y;
+    }
+    dst[k * kSmallLd + r] = x;
+  }
+}
+
+template <typename TA, typename TB, bool M3>
+__global__ void __launch_bounds__(kSmallThreads) small_gemm_kernel(GemmArgs g, unsigned tiles_n) {
+  typedef typename AccT<TA, TB>::type TC;
+  constexpr int kSmallKc = small_kc<TA, TB>();
+  __shared__ TA As[kSmallKc * kSmallLd];
+  __shared__ TB Bs[kSmallKc * kSmallLd];
+  __shared__ double Sa[M3 ? kSmallKc * kSmallLd : 1], Sb[M3 ? kSmallKc * kSmallLd : 1];
+  __shared__ TC half[kSmallT * kSmallT];
+  const int i0 = int(blockIdx.x / tiles_n) * kSmallT, j0 = int(blockIdx.x % tiles_n) * kSmallT;
+  if (g.upper_only && j0 + kSmallT <= i0) return;  // wholly below the diagonal
+  const long long b = blockIdx.y;
+  const int out = threadIdx.x & 63, part = threadIdx.x >> 6;
+  const int i = out & 7, j = out >> 3;
+  TC acc = zero_of<TC>();
+  double t1 = 0.0, t2 = 0.0, t3 = 0.0;
+  for (int k0 = 0; k0 < g.K; k0 += kSmallKc) {
+    const int kt = min(kSmallKc, g.K - k0);
+    if (k0 > 0) __syncthreads();
+    stage_small<TA>(As, g.A, true, i0, g.M, k0, kt, b, g.conj_a);
+    stage_small<TB>(Bs, g.B, false, j0, g.N, k0, kt, b, g.conj_b);
+    __syncthreads();
+    if constexpr (M3) {
+      for (int idx = threadIdx.x; idx < kt * kSmallLd; idx += kSmallThreads) {
+        if (idx % kSmallLd == kSmallT) continue;
+        Sa[idx] = As[idx].x + As[idx].y;
+        Sb[idx] = Bs[idx].x + Bs[idx].y;
+      }
+      __syncthreads();
+#pragma unroll 4
+      for (int k = part; k < kt; k += 2) {
+        const TA a = As[k * kSmallLd + i];
+        const TB c = Bs[k * kSmallLd + j];
+        t1 = fma(a.x, c.x, t1);
+        t2 = fma(a.y, c.y, t2);
+        t3 = fma(Sa[k * kSmallLd + i], Sb[k * kSmallLd + j], t3);
+      }
+    } else {
+#pragma unroll 4
+      for (int k = part; k < kt; k += 2) mac(acc, As[k * kSmallLd + i], Bs[k * kSmallLd + j]);
+    }
+  }
+  if constexpr (M3) acc = make_double2(t1 - t2, t3 - t1 - t2);
+  if (part == 1) half[out] = acc;
+  __syncthreads();
+  if (part == 1 || i0 + i >= g.M || j0 + j >= g.N) return;
+  double2 alpha = g.alpha;
+  if (g.alpha_vec) alpha = cmul(alpha, g.alpha_vec[b]);
+  const long long idx = (i0 + i) * g.crs + (j0 + j) * g.ccs + b * g.cbs;
+  if constexpr (sizeof(TC) == sizeof(double)) {
+    store_out(g, idx, acc + half[out], alpha);
+  } else {
+    const double2 v = cadd(acc, half[out]);
+    if (g.c_real)
+      store_out_real_from_complex(g, idx, v, alpha);
+    else
+      store_out(g, idx, v, alpha);
+  }
+}
+
+// FP64 multiply-adds of a product (a complex one in the 3M form)
+double real_work(const GemmArgs& g) {
+  return double(g.M) * g.N * (double(g.K) + g.K2) * g.batch * ((g.a_real ? 1 : 2) + (g.b_real ? 1 : 2) - 1);
+}
+
+void launch_small_gemm(const GemmArgs& g, cudaStream_t s) {
+  const unsigned tn = unsigned(g.N + kSmallT - 1) / kSmallT, tm = unsigned(g.M + kSmallT - 1) / kSmallT;
+  const dim3 grid(tn * tm, g.batch);
+  if (g.a_real && g.b_real)
+    small_gemm_kernel<double, double, false><<<grid, kSmallThreads, 0, tvap::counted(s)>>>(g, tn);
+  else if (g.a_real)
+    small_gemm_kernel<double, double2, false><<<grid, kSmallThreads, 0, tvap::counted(s)>>>(g, tn);
+  else if (g.b_real)
+    small_gemm_kernel<double2, double, false><<<grid, kSmallThreads, 0, tvap::counted(s)>>>(g, tn);
+  else if (g.three_m && !g.c_real)
+    small_gemm_kernel<double2, double2, true><<<grid, kSmallThreads, 0, tvap::counted(s)>>>(g, tn);
+  else
+    small_gemm_kernel<double2, double2, false><<<grid, kSmallThreads, 0, tvap::counted(s)>>>(g, tn);
+}
+
 template <int T, typename TA, typename TB>
 void launch_gemm_t(const GemmArgs& g, cudaStream_t s) {
   dim3 grid((g.N + T - 1) / T, (g.M + T - 1) / T, g.batch);
@@ -283,14 +405,22 @@ int gemm_split_k2(const GemmArgs& g, cudaStream_t s) {
 
 int gemm(const GemmArgs& g, cudaStream_t s) {
   if (g.M <= 0 || g.N <= 0 || g.batch <= 0) return TVAP_OK;
+  // Up to kSmallWork FP64 multiply-adds a product runs on the FP64 pipe in
+  // every mode (small_gemm_kernel): 1.2e7 take 20 us on the whole chip, about
+  // what the emulated form's two slicing passes and its product need at least
+  // (real n = 140, 2.7e6: 15.6 us against 27; n = 336, 3.8e7: at least 63 us
+  // against 50).  Larger ones run emulated on the tensor cores.
+  const bool small = real_work(g) <= kSmallWork;
   if (g.K2 > 0) {
-    const double kk = double(g.K) + g.K2;
-    if (g_gemm_mode == 2 && double(g.M) * g.N * kk * g.batch >= 1.0e6) return gemm_ozaki(g, s);
+    if (g_gemm_mode == 2 && !small) return gemm_ozaki(g, s);
     return gemm_split_k2(g, s);
   }
-  // every product of at least 10^6 multiply-adds runs emulated on the tensor
-  // cores; the smaller ones (few-column blocks, short K) stay on the FP64 pipe
-  if (g_gemm_mode >= 1 && g.K >= 16 && double(g.M) * g.N * g.K * g.batch >= 1.0e6) return gemm_ozaki(g, s);
+  if (small) {
+    launch_small_gemm(g, s);
+    TVAP_CUDA(cudaGetLastError());
+    return TVAP_OK;
+  }
+  if (g_gemm_mode >= 1 && g.K >= 16) return gemm_ozaki(g, s);
   // few tiles in all (single small products): the smallest tile, to spread
   // the latency-bound work over more SMs
   const long long t28 = (long long)((g.M + 27) / 28) * ((g.N + 27) / 28) * g.batch;
