@@ -26,7 +26,7 @@ GPU_LIB = os.path.join(PKG_DIR, "libtvap_gpu.so")
 GPU_SOURCES = [
     "tvap_context.cu",
     "fields.cu",
-    "dense.cu",
+    "dense.cu", "evolve.cu",
     "projection.cu",
     "gradient.cu",
     "ozaki.cu",

@@ -138,16 +138,15 @@ int tvap_adjust_constraints(tvap_ctx* c, const double* U0, const double* V0, dou
   const size_t nn = size_t(n) * n;
   cudaStream_t s = c->stream;
   const int njobs = cdim + cdim * (cdim + 1) / 2;
-  // U0, V0, Z, U1, V1 (adjacent), rho, kappa, T1, T2, T3, evolution work
-  // (3 n^2 + n), the operators, C20, x, partial sums and results, the jobs
+  // U0, V0, Z, U1, V1, rho, kappa, T1, T2, T3, evolution work, the operators, C20, x, partial sums and results, the jobs
   double* buf = nullptr;
   const size_t jobs_doubles = (sizeof(DotJob) * size_t(njobs > 0 ? njobs : 1) + 7) / 8;
-  const size_t tot = 13 * nn + n + 2 * size_t(cdim) * nn + cdim + size_t(njobs) * (kDotBlocks + 1) + jobs_doubles + 2;
+  const size_t tot = 10 * nn + evolve_work(n) + 2 * size_t(cdim) * nn + cdim + size_t(njobs) * (kDotBlocks + 1) + jobs_doubles + 2;
   int rc;
   if ((rc = ctx_scratch(c, tot, &buf))) return rc;
   double *dU0 = buf, *dV0 = dU0 + nn, *dZ = dV0 + nn, *dU1 = dZ + nn, *dV1 = dU1 + nn, *rho = dV1 + nn,
          *kap = rho + nn, *T1 = kap + nn, *T2 = T1 + nn, *T3 = T2 + nn, *work = T3 + nn;
-  double* cops = work + 3 * nn + n;
+  double* cops = work + evolve_work(n);
   double* c20 = cops + size_t(cdim) * nn;
   double* dx = c20 + size_t(cdim) * nn;
   double* partial = dx + cdim;

@@ -1475,341 +1475,4 @@ int cholesky_inverse(int n, double* A, int* flags, cudaStream_t s) {
   return TVAP_OK;
 }
 
-
-// ---------------------------------------------------------------------------
-// Cholesky factorisation of S (lower, L L^T = S; S has n x n + n doubles, the
-// last n receive 1 / L_jj) and the evolution solves
-// X L^T = A for two n x n matrices A (U1 = A1 L^{-T}, V1 = A2 L^{-T}) in one
-// cooperative launch.  GB300's FP64 pipe gives one SM about 2 FMAs per clock,
-// so the factorisation is spread over the grid: panels of kCoopNb columns; CTA
-// 0 factors each diagonal block, all CTAs solve the panel rows below it and
-// apply the trailing update (CTA 0 updating and factoring the next diagonal
-// block meanwhile); then one warp per row of A1 / A2 runs the forward
-// substitution L x = a with L in shared memory.  Grid-wide barriers between
-// the phases are bounded spins (all CTAs are co-resident by the cooperative
-// launch); a barrier that gives up raises the status word and every CTA
-// returns.
-// ---------------------------------------------------------------------------
-namespace {
-
-constexpr int kCoopThreads = 256;
-constexpr int kCoopNb = 16;
-constexpr long long kCoopSpin = 1LL << 22;
-
-// bar[0] arrivals, bar[1] generation, bar[2] abort; zeroed before the launch
-__device__ bool coop_barrier(unsigned* bar, unsigned nblocks, unsigned& gen, int* flags) {
-  __shared__ int ok_s;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    int ok = 1;
-    __threadfence();
-    if (atomicAdd(&bar[0], 1u) == nblocks - 1) {
-      atomicExch(&bar[0], 0u);
-      __threadfence();
-      atomicExch(&bar[1], gen + 1);
-    } else {
-      volatile unsigned* g = &bar[1];
-      long long it = 0;
-      while (*g == gen) {
-        if (++it > kCoopSpin || *(volatile unsigned*)&bar[2]) {
-          ok = 0;
-          break;
-        }
-        __nanosleep(64);
-      }
-    }
-    if (!ok || *(volatile unsigned*)&bar[2]) {
-      if (!*(volatile unsigned*)&bar[2]) atomicOr(flags, DEV_WAIT_TIMEOUT);
-      atomicExch(&bar[2], 1u);
-      ok = 0;
-    }
-    __threadfence();
-    ok_s = ok;
-  }
-  ++gen;
-  __syncthreads();
-  return ok_s != 0;
-}
-
-// 1 / sqrt(d) for a positive normal d: an FP32 seed (of d's value with the
-// mantissa truncated to 23 bits) refined by two Newton-Raphson steps for the
-// reciprocal square root, y <- y (3 - d y^2) / 2 (each step doubles the
-// correct bits: 2^-22 -> 2^-44 -> FP64 rounding).  The range test, the seed's
-// conversions and d / 2 (an exponent decrement) run on the integer pipe, so
-// the 6 Newton instructions are all that occupy the FP64 pipe; outside the
-// range of seed_range the library routines are used.
-__device__ __forceinline__ double rsqrt_newton(double d) {
-  if (!seed_range(d)) return 1.0 / sqrt(d);
-  double y = seed_f64(rsqrtf(seed_f32(d)));
-  const double h = __longlong_as_double(__double_as_longlong(d) - (1LL << 52));  // d / 2, exact
-  y = y * fma(-h, y * y, 1.5);
-  y = y * fma(-h, y * y, 1.5);
-  return y;
-}
-
-// Unblocked Cholesky of the nb x nb diagonal block at (j0, j0) of S by the
-// whole CTA (kCoopThreads >= kCoopNb^2 threads, one entry of the block each,
-// the block in B): per step the pivot's thread forms 1 / sqrt(d), the column
-// is scaled by it (as DPBTF2 does) and the trailing entries take
-// A_ij -= L_ik L_jk, each entry in the same order as an unblocked
-// elimination.  An FP64 warp instruction holds the FP64 unit of its SM
-// sub-partition for about 64 cycles on this part: with the block's entries
-// spread over all the CTA's warps, a step's update is one instruction on
-// every sub-partition instead of up to 15 on one.  The reciprocals go to
-// rd[j0 ..] for the solves; sc (2 doubles of shared memory) carries the
-// pivot's reciprocal and the failure flag.  Elements written by other CTAs
-// are read through L2.  Every thread of the CTA calls it; the result is
-// uniform.
-__device__ bool coop_factor_diag(int n, double* S, double* rd, int j0, int nb, double (*B)[kCoopNb + 1],
-                                 double* sc) {
-  static_assert(kCoopThreads >= kCoopNb * kCoopNb, "one thread per entry of the diagonal block");
-  const int t = threadIdx.x;
-  const int i = t % kCoopNb, j = t / kCoopNb;
-  const bool mine = t < kCoopNb * kCoopNb && i < nb && j < nb && i >= j;
-  if (mine) B[i][j] = __ldcg(&S[(j0 + i) + size_t(j0 + j) * n]);
-  __syncthreads();
-  for (int k = 0; k < nb; ++k) {
-    if (t == k * kCoopNb + k) {  // the pivot's thread
-      const double d = B[k][k];
-      if (d > 0.0) {
-        const double y = rsqrt_newton(d);
-        B[k][k] = d * y;
-        rd[j0 + k] = y;
-        sc[0] = y;
-        sc[1] = 0.0;
-      } else {
-        sc[1] = 1.0;
-      }
-    }
-    __syncthreads();
-    if (sc[1] != 0.0) return false;  // uniform: read by every thread after the barrier
-    if (mine && j == k && i > k) B[i][k] *= sc[0];
-    __syncthreads();
-    if (mine && j > k) B[i][j] = fma(-B[i][k], B[j][k], B[i][j]);
-    __syncthreads();
-  }
-  if (mine) S[(j0 + i) + size_t(j0 + j) * n] = B[i][j];
-  return true;
-}
-
-template <int SLOTS>
-__global__ void __launch_bounds__(kCoopThreads, 1) cholesky_evolve_kernel(int n, double* S, const double* A,
-                                                                       long long a_stride, double* X,
-                                                                       long long x_stride, unsigned* bar,
-                                                                       int* flags, int skip_cta, int l_smem) {
-  // the panel rows; then, in the solve phase, L (n x n, when l_smem) and 1 / L_jj
-  extern __shared__ double coop_smem[];
-  __shared__ double L11[kCoopNb][kCoopNb + 1];
-  __shared__ double rdiag[kCoopNb];
-  __shared__ unsigned gen_s;
-  const int t = threadIdx.x, G = gridDim.x, cta = blockIdx.x;
-  if (t == 0) gen_s = *(volatile unsigned*)&bar[1];
-  __syncthreads();
-  unsigned gen = gen_s;  // every thread keeps its own copy of the generation
-  double* rd = S + size_t(n) * n;  // 1 / L_jj
-  if (cta == 0 && !coop_factor_diag(n, S, rd, 0, min(kCoopNb, n), L11, rdiag) && t == 0) {
-    atomicOr(flags, DEV_CHOLESKY);
-    atomicExch(&bar[2], 1u);
-  }
-  // test hook: this CTA leaves without arriving, so that the others' bounded
-  // waits at the first barrier run out (status DEV_WAIT_TIMEOUT, abort)
-  if (cta == skip_cta) return;
-  if (!coop_barrier(bar, G, gen, flags)) return;
-  for (int j0 = 0;;) {
-    const int j1 = min(j0 + kCoopNb, n);
-    if (j1 >= n) break;
-    const int nbp = j1 - j0, j2 = min(j1 + kCoopNb, n);
-    // panel rows below the diagonal block: L21 = S21 L11^{-T}, one warp per
-    // row (lane k holds x_k), rows spread over the CTAs so that their FP64
-    // work runs on different SMs
-    if (j1 + cta < n) {
-      for (int idx = t; idx < nbp * nbp; idx += blockDim.x) {
-        const int i = idx % nbp, j = idx / nbp;
-        if (i >= j) L11[i][j] = __ldcg(&S[(j0 + i) + size_t(j0 + j) * n]);
-      }
-      if (t < nbp) rdiag[t] = __ldcg(&rd[j0 + t]);
-      __syncthreads();
-      const int warp = t >> 5, lane = t & 31, warps = blockDim.x >> 5;
-      for (int i = j1 + cta + G * warp; i < n; i += G * warps) {
-        double xk = (lane < nbp) ? __ldcg(&S[i + size_t(j0 + lane) * n]) : 0.0;
-        for (int m = 0; m < nbp; ++m) {
-          if (lane == m) xk *= rdiag[m];
-          const double xm = __shfl_sync(0xffffffffu, xk, m);
-          if (lane > m && lane < nbp) xk = fma(-xm, L11[lane][m], xk);
-        }
-        if (lane < nbp) S[i + size_t(j0 + lane) * n] = xk;
-      }
-    }
-    if (!coop_barrier(bar, G, gen, flags)) return;
-    // trailing update S22 -= L21 L21^T (lower triangle).  CTA 0 takes the
-    // next diagonal block (rows and columns j1 .. j2-1) and factors it; the
-    // other CTAs take the rest, one column at a time.  The panel rows j1..n-1
-    // are staged in shared memory first (independent loads: one L2 round
-    // trip instead of one per k).
-    double* P = coop_smem;  // (n - j1) x nbp, row-major
-    const int prow = n - j1;
-    if (cta == 0 || cta - 1 < prow) {
-#pragma unroll 4
-      for (int idx = t; idx < prow * nbp; idx += blockDim.x) {
-        const int k = idx / prow, i = idx - k * prow;
-        P[i * kCoopNb + k] = __ldcg(&S[(j1 + i) + size_t(j0 + k) * n]);
-      }
-      __syncthreads();
-    }
-    if (cta == 0) {
-      const int nb2 = j2 - j1;
-      for (int idx = t; idx < nb2 * nb2; idx += blockDim.x) {
-        const int i = idx % nb2, j = idx / nb2;
-        if (i < j) continue;
-        double v = __ldcg(&S[(j1 + i) + size_t(j1 + j) * n]);
-        for (int k = 0; k < nbp; ++k) v = fma(-P[i * kCoopNb + k], P[j * kCoopNb + k], v);
-        S[(j1 + i) + size_t(j1 + j) * n] = v;
-      }
-      __syncthreads();
-      // (L11 and rdiag are free until the barrier: every CTA reloads them)
-      if (!coop_factor_diag(n, S, rd, j1, nb2, L11, rdiag) && t == 0) {
-        atomicOr(flags, DEV_CHOLESKY);
-        atomicExch(&bar[2], 1u);
-      }
-    }
-    if (cta > 0 || G == 1) {
-      const int workers = G > 1 ? G - 1 : 1, w = G > 1 ? cta - 1 : 0;
-      for (int j = j1 + w; j < n; j += workers) {
-        const double* pj = P + (j - j1) * kCoopNb;
-        const int i0 = (j < j2) ? j2 : j;
-        for (int i = i0 + t; i < n; i += blockDim.x) {
-          const double* pi = P + (i - j1) * kCoopNb;
-          double v = __ldcg(&S[i + size_t(j) * n]);
-          for (int k = 0; k < nbp; ++k) v = fma(-pi[k], pj[k], v);
-          S[i + size_t(j) * n] = v;
-        }
-      }
-    }
-    if (!coop_barrier(bar, G, gen, flags)) return;
-    j0 = j1;
-  }
-  // forward substitution L x = a for every row of A1 and A2: one warp per
-  // row, rows spread over all CTAs
-  const int warps = blockDim.x >> 5, warp = t >> 5, lane = t & 31;
-  const int rows = 2 * n;
-  if (cta >= rows) return;
-  // L from shared memory when it fits (n <= 168), else from L2 (S is
-  // written by this grid before the last barrier: read through L2, not L1)
-  double* Ls = coop_smem;
-  double* dinv = l_smem ? Ls + size_t(n) * n : coop_smem;
-  if (l_smem) {
-    if ((reinterpret_cast<uintptr_t>(S) & 15) == 0) {
-      // 16-byte loads, many in flight
-      const int nn2 = (n * n) / 2;
-      const double2* S2 = reinterpret_cast<const double2*>(S);
-      double2* L2 = reinterpret_cast<double2*>(Ls);
-#pragma unroll 16
-      for (int idx = t; idx < nn2; idx += blockDim.x) L2[idx] = __ldcg(&S2[idx]);
-      if (((n * n) & 1) && t == 0) Ls[n * n - 1] = __ldcg(&S[n * n - 1]);
-    } else {
-#pragma unroll 16
-      for (int idx = t; idx < n * n; idx += blockDim.x) Ls[idx] = __ldcg(&S[idx]);
-    }
-  }
-  __syncthreads();
-  for (int j = t; j < n; j += blockDim.x) dinv[j] = __ldcg(&rd[j]);
-  __syncthreads();
-  constexpr int kMaxPerLane = SLOTS;
-  for (int r = cta + G * warp; r < rows; r += G * warps) {
-    const int mat = r >= n ? 1 : 0, row = r - mat * n;
-    const double* a = A + mat * a_stride;
-    double* x = X + mat * x_stride;
-    double v[kMaxPerLane];
-#pragma unroll
-    for (int q = 0; q < kMaxPerLane; ++q) {
-      const int j = lane + 32 * q;
-      v[q] = (j < n) ? a[row + size_t(j) * n] : 0.0;
-    }
-    // columns j in slot qj (a compile-time index once unrolled): the slots
-    // below qj are finished, the slots above take every lane, slot qj the
-    // lanes above j -- only those FMAs are issued (each an FP64 instruction
-    // of about 64 cycles on this part), in the order of an unblocked solve
-#pragma unroll
-    for (int qj = 0; qj < kMaxPerLane; ++qj) {
-      if (32 * qj >= n) break;
-      const int jend = min(32 * qj + 32, n);
-      for (int j = 32 * qj; j < jend; ++j) {
-        const int owner = j & 31;
-        const double xj = __shfl_sync(0xffffffffu, v[qj], owner) * dinv[j];
-        if (lane == owner) v[qj] = xj;
-        const double* lc = (l_smem ? Ls : S) + size_t(j) * n;
-        {
-          const int jj = lane + 32 * qj;
-          if (jj > j && jj < n) v[qj] = fma(-xj, l_smem ? lc[jj] : __ldcg(&lc[jj]), v[qj]);
-        }
-#pragma unroll
-        for (int q = qj + 1; q < kMaxPerLane; ++q) {
-          if (32 * q >= n) break;
-          const int jj = lane + 32 * q;
-          if (jj < n) v[q] = fma(-xj, l_smem ? lc[jj] : __ldcg(&lc[jj]), v[q]);
-        }
-      }
-    }
-#pragma unroll
-    for (int q = 0; q < kMaxPerLane; ++q) {
-      const int j = lane + 32 * q;
-      if (j < n) x[row + size_t(j) * n] = v[q];
-    }
-  }
-}
-
-}  // namespace
-
-int cholesky_evolve_coop(int n, double* S, const double* A, long long a_stride, double* X, long long x_stride,
-                         unsigned* bar, int* flags, cudaStream_t s, int skip_cta) {
-  // L in shared memory for the solves when it fits; else the panel rows
-  // ((n - 1) x kCoopNb) and 1 / L_jj only, L read from L2
-  const size_t shm_full = sizeof(double) * (size_t(n) * n + n);
-  const int l_smem = shm_full <= jacobi32_smem_limit() ? 1 : 0;
-  const size_t shm = l_smem ? shm_full : sizeof(double) * (size_t(n) * kCoopNb + n);
-  if (n > 384 || shm > jacobi32_smem_limit()) return TVAP_ERR_ARG;
-  const int slots = (n + 31) / 32;
-  const void* kern = slots <= 2    ? (const void*)cholesky_evolve_kernel<2>
-                     : slots <= 4  ? (const void*)cholesky_evolve_kernel<4>
-                     : slots <= 5  ? (const void*)cholesky_evolve_kernel<5>
-                     : slots <= 6  ? (const void*)cholesky_evolve_kernel<6>
-                     : slots <= 8  ? (const void*)cholesky_evolve_kernel<8>
-                     : slots <= 11 ? (const void*)cholesky_evolve_kernel<11>
-                                   : (const void*)cholesky_evolve_kernel<12>;
-  // the co-resident grid of this instantiation and shared-memory size, found
-  // once per device
-  struct GridKey {
-    int dev;
-    const void* kern;
-    size_t shm;
-  };
-  static std::mutex m;
-  static std::vector<std::pair<GridKey, int>> grids;
-  int dev = 0;
-  TVAP_CUDA(cudaGetDevice(&dev));
-  int grid = 0;
-  {
-    std::lock_guard<std::mutex> lock(m);
-    for (const auto& e : grids)
-      if (e.first.dev == dev && e.first.kern == kern && e.first.shm == shm) grid = e.second;
-    if (grid == 0) {
-      if (int rc = smem_opt_in(kern, shm)) return rc;
-      int per_sm = 0;
-      TVAP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kCoopThreads, shm));
-      grid = std::min(per_sm * device_sms(), 128);
-      if (grid >= 1) grids.push_back({GridKey{dev, kern, shm}, grid});
-    }
-  }
-  if (grid < 1) return TVAP_ERR_ARG;
-  TVAP_CUDA(cudaMemsetAsync(bar, 0, 3 * sizeof(unsigned), s));
-  // the hook names the grid's last CTA (never CTA 0, which factors the
-  // diagonal blocks); -1 leaves every CTA in
-  int skip = (skip_cta >= 0 && grid > 1) ? grid - 1 : -1;
-  void* args[] = {&n, &S, &A, &a_stride, &X, &x_stride, &bar, &flags, &skip, const_cast<int*>(&l_smem)};
-  ++g_launch_count;
-  TVAP_CUDA(cudaLaunchCooperativeKernel(kern, dim3(grid), dim3(kCoopThreads), args,
-                                        shm, s));
-  return TVAP_OK;
-}
-
 }  // namespace tvap

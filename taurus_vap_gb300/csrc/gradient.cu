@@ -78,37 +78,29 @@ int rgemm(int M, int N, int K, View A, View B, double* C, int ldc, double alpha,
   return gemm(g, s);
 }
 
-struct EvolveBuf {
-  double *Z = nullptr, *L = nullptr, *A1 = nullptr, *A2 = nullptr, *U0 = nullptr, *V0 = nullptr;
-};
-
-// U1 = (U0 + V0 Z) L^{-T}, V1 = (V0 + U0 Z) L^{-T} with L L^T = 1 + Z^T Z.
-// With want_linv, L^{-1} is left in b.L (cholesky_inverse and two products);
-// otherwise one cooperative launch factorises and solves when n allows it.
-int evolve_device(tvap_ctx* c, EvolveBuf& b, int n, double* U1, double* V1, bool want_linv) {
+// U1 = (U0 + V0 Z) L^{-T}, V1 = (V0 + U0 Z) L^{-T} with L L^T = 1 + Z^T Z, and
+// L^{-1} when Linv is not null; work holds evolve_work(n) doubles.  One
+// cooperative launch, which also forms the products where n allows it; above
+// its range the single-CTA inverse and two products.
+int evolve_device(tvap_ctx* c, const double* Z, const double* U0, const double* V0, double* work, int n, double* U1,
+                  double* V1, double* Linv) {
   cudaStream_t s = c->stream;
   const size_t nn = size_t(n) * n;
+  double *A = work, *S = work + 2 * nn;
   int rc;
-  const View Zv = view_cm(b.Z, n, 0);
   sec_begin(c, SEC_EVOLVE);
-  if ((rc = rgemm(n, n, n, view_t(Zv), Zv, b.L, n, 1.0, 0.0, s))) return rc;
-  add_identity_kernel<<<(n + 255) / 256, 256, 0, tvap::counted(s)>>>(n, b.L);
-  TVAP_CUDA(cudaMemcpyAsync(b.A1, b.U0, sizeof(double) * nn, cudaMemcpyDeviceToDevice, s));
-  TVAP_CUDA(cudaMemcpyAsync(b.A2, b.V0, sizeof(double) * nn, cudaMemcpyDeviceToDevice, s));
-  const bool coop = !want_linv && c->d_bar;
-  if (!coop && (rc = cholesky_inverse(n, b.L, c->d_flags, s))) return rc;
-  const View LinvT = view_t(view_cm(b.L, n, 0));
-  // A1 = U0 + V0 Z, A2 = V0 + U0 Z as one batch of two when A2 follows A1
-  // (then U1 = A1 L^-T, V1 = A2 L^-T likewise when V1 follows U1)
-  const bool pair_a = (b.A2 == b.A1 + nn);
-  const bool pair_u = pair_a && (V1 == U1 + nn);
-  if (pair_a) {
+  if (!evolve_forms_products(n)) {
+    const View Zv = view_cm(Z, n, 0);
+    if ((rc = rgemm(n, n, n, view_t(Zv), Zv, S, n, 1.0, 0.0, s))) return rc;
+    add_identity_kernel<<<(n + 255) / 256, 256, 0, tvap::counted(s)>>>(n, S);
+    TVAP_CUDA(cudaMemcpyAsync(A, U0, sizeof(double) * nn, cudaMemcpyDeviceToDevice, s));
+    TVAP_CUDA(cudaMemcpyAsync(A + nn, V0, sizeof(double) * nn, cudaMemcpyDeviceToDevice, s));
     GemmArgs g{};
     g.M = g.N = g.K = n;
     g.batch = 2;
-    g.A = View{b.V0, 1, n, (long long)(b.U0 - b.V0)};
-    g.B = View{b.Z, 1, n, 0};
-    g.C = b.A1;
+    g.A = View{V0, 1, n, (long long)(U0 - V0)};
+    g.B = View{Z, 1, n, 0};
+    g.C = A;
     g.crs = 1;
     g.ccs = n;
     g.cbs = (long long)nn;
@@ -116,39 +108,18 @@ int evolve_device(tvap_ctx* c, EvolveBuf& b, int n, double* U1, double* V1, bool
     g.beta = make_double2(1.0, 0.0);
     g.a_real = g.b_real = g.c_real = true;
     if ((rc = gemm(g, s))) return rc;
-  } else {
-    if ((rc = rgemm(n, n, n, view_cm(b.V0, n, 0), Zv, b.A1, n, 1.0, 1.0, s))) return rc;
-    if ((rc = rgemm(n, n, n, view_cm(b.U0, n, 0), Zv, b.A2, n, 1.0, 1.0, s))) return rc;
   }
-  if (coop) {
-    const int skip = c->test_skip_arrival ? 1 : -1;
-    c->test_skip_arrival = false;
-    rc = cholesky_evolve_coop(n, b.L, b.A1, (long long)(b.A2 - b.A1), U1, (long long)(V1 - U1), c->d_bar,
-                              c->d_flags, s, skip);
-    if (rc == TVAP_OK) {
-      sec_end(c, SEC_EVOLVE);
-      return TVAP_OK;
-    }
-    if (rc != TVAP_ERR_ARG) return rc;
-    if ((rc = cholesky_inverse(n, b.L, c->d_flags, s))) return rc;
-  }
-  if (pair_u) {
-    GemmArgs g{};
-    g.M = g.N = g.K = n;
-    g.batch = 2;
-    g.A = View{b.A1, 1, n, (long long)nn};
-    g.B = View{LinvT.p, LinvT.rs, LinvT.cs, 0};
-    g.C = U1;
-    g.crs = 1;
-    g.ccs = n;
-    g.cbs = (long long)nn;
-    g.alpha = make_double2(1.0, 0.0);
-    g.beta = make_double2(0.0, 0.0);
-    g.a_real = g.b_real = g.c_real = true;
-    if ((rc = gemm(g, s))) return rc;
-  } else {
-    if ((rc = rgemm(n, n, n, view_cm(b.A1, n, 0), LinvT, U1, n, 1.0, 0.0, s))) return rc;
-    if ((rc = rgemm(n, n, n, view_cm(b.A2, n, 0), LinvT, V1, n, 1.0, 0.0, s))) return rc;
+  const int skip = c->test_skip_arrival ? 1 : -1;
+  c->test_skip_arrival = false;
+  rc = thouless_evolve(n, Z, U0, V0, work, U1, V1, Linv, c->d_bar, c->d_flags, s, skip);
+  if (rc == TVAP_ERR_ARG) {
+    if ((rc = cholesky_inverse(n, S, c->d_flags, s))) return rc;
+    const View LinvT = view_t(view_cm(S, n, 0));
+    if ((rc = rgemm(n, n, n, view_cm(A, n, 0), LinvT, U1, n, 1.0, 0.0, s))) return rc;
+    if ((rc = rgemm(n, n, n, view_cm(A + nn, n, 0), LinvT, V1, n, 1.0, 0.0, s))) return rc;
+    if (Linv) TVAP_CUDA(cudaMemcpyAsync(Linv, S, sizeof(double) * nn, cudaMemcpyDeviceToDevice, s));
+  } else if (rc) {
+    return rc;
   }
   sec_end(c, SEC_EVOLVE);
   return TVAP_OK;
@@ -158,20 +129,11 @@ int evolve_device(tvap_ctx* c, EvolveBuf& b, int n, double* U1, double* V1, bool
 
 // The Thouless evolution of a device state for the other translation units:
 // U1 = (U0 + V0 Z) L^-T, V1 = (V0 + U0 Z) L^-T, every matrix on the device;
-// work holds 3 n^2 + n doubles.  Runs on the context's stream in the calling
-// thread's arithmetic.
+// work holds evolve_work(n) doubles.  Runs on the context's stream in the
+// calling thread's arithmetic.
 int evolve_state(tvap_ctx* c, const double* U0, const double* V0, const double* Z, double* U1, double* V1,
                  double* work) {
-  const int n = c->n;
-  const size_t nn = size_t(n) * n;
-  EvolveBuf b;
-  b.Z = const_cast<double*>(Z);
-  b.U0 = const_cast<double*>(U0);
-  b.V0 = const_cast<double*>(V0);
-  b.A1 = work;
-  b.A2 = work + nn;
-  b.L = work + 2 * nn;
-  return evolve_device(c, b, n, U1, V1, false);
+  return evolve_device(c, Z, U0, V0, work, c->n, U1, V1, nullptr);
 }
 
 double* ws_U(tvap_ctx* c);
@@ -269,20 +231,12 @@ int tvap_evolve(tvap_ctx* c, const double* U0, const double* V0, const double* Z
   const size_t nn = size_t(n) * n;
   cudaStream_t s = c->stream;
   double* buf = nullptr;
-  if (int r0 = ctx_scratch(c, 8 * nn + n, &buf)) return r0;
-  EvolveBuf b;
-  b.Z = buf;
-  b.U0 = buf + nn;
-  b.V0 = buf + 2 * nn;
-  b.A1 = buf + 3 * nn;
-  b.A2 = buf + 4 * nn;
-  double* dU1 = buf + 5 * nn;
-  double* dV1 = buf + 6 * nn;
-  b.L = buf + 7 * nn;  // n*n + n (scratch row)
-  int rc = upload_matrix(Z, b.Z, sizeof(double) * nn, s);
-  if (!rc) rc = upload_matrix(U0, b.U0, sizeof(double) * nn, s);
-  if (!rc) rc = upload_matrix(V0, b.V0, sizeof(double) * nn, s);
-  if (!rc) rc = evolve_device(c, b, n, dU1, dV1, false);
+  if (int r0 = ctx_scratch(c, 5 * nn + evolve_work(n), &buf)) return r0;
+  double *dZ = buf, *dU0 = buf + nn, *dV0 = buf + 2 * nn, *dU1 = buf + 3 * nn, *dV1 = buf + 4 * nn;
+  int rc = upload_matrix(Z, dZ, sizeof(double) * nn, s);
+  if (!rc) rc = upload_matrix(U0, dU0, sizeof(double) * nn, s);
+  if (!rc) rc = upload_matrix(V0, dV0, sizeof(double) * nn, s);
+  if (!rc) rc = evolve_device(c, dZ, dU0, dV0, buf + 5 * nn, n, dU1, dV1, nullptr);
   if (!rc) rc = download_matrix(dU1, U1, sizeof(double) * nn, s);
   if (!rc) rc = download_matrix(dV1, V1, sizeof(double) * nn, s);
   if (!rc) rc = check_flags(c);
@@ -314,9 +268,9 @@ int tvap_iterate(tvap_ctx* c, const double* U0, const double* V0, const tvap_pro
   const int tb = 256;
   const int nblocks = int((nn + tb - 1) / tb);
   double* buf = nullptr;
-  // Z_{i-1}, Z_i, A1, A2, U1, V1 (adjacent pairs), L (n^2 + n), partial sums
-  if ((rc = ctx_scratch(c, 7 * nn + n + nblocks, &buf))) return rc;
-  double *dZm = buf, *dZ = buf + nn, *dU1 = buf + 4 * nn, *dV1 = buf + 5 * nn, *part = buf + 7 * nn + n;
+  // Z_{i-1}, Z_i, U1, V1, partial sums, the evolution's work
+  if ((rc = ctx_scratch(c, 4 * nn + nblocks + evolve_work(n), &buf))) return rc;
+  double *dZm = buf, *dZ = buf + nn, *dU1 = buf + 2 * nn, *dV1 = buf + 3 * nn, *part = buf + 4 * nn;
   if ((rc = upload_matrix(U0, ws_U(c), sizeof(double) * nn, s))) return rc;
   if ((rc = upload_matrix(V0, ws_V(c), sizeof(double) * nn, s))) return rc;
   if ((rc = upload_matrix(Zim1, dZm, sizeof(double) * nn, s))) return rc;
@@ -331,14 +285,7 @@ int tvap_iterate(tvap_ctx* c, const double* U0, const double* V0, const tvap_pro
   TVAP_CUDA(cudaGetLastError());
   sec_end(c, SEC_GRADIENT);
   // cholesky_factorization + evolve_wavefunction of the projected state
-  EvolveBuf b;
-  b.Z = dZ;
-  b.U0 = ws_U(c);
-  b.V0 = ws_V(c);
-  b.A1 = buf + 2 * nn;
-  b.A2 = buf + 3 * nn;
-  b.L = buf + 6 * nn;
-  if ((rc = evolve_device(c, b, n, dU1, dV1, false))) return rc;
+  if ((rc = evolve_device(c, dZ, ws_U(c), ws_V(c), part + nblocks, n, dU1, dV1, nullptr))) return rc;
   if ((rc = download_matrix(dZ, Zi, sizeof(double) * nn, s))) return rc;
   if ((rc = download_matrix(dU1, U1, sizeof(double) * nn, s))) return rc;
   if ((rc = download_matrix(dV1, V1, sizeof(double) * nn, s))) return rc;
@@ -432,28 +379,21 @@ int tvap_energy_adjoint(tvap_ctx* c, const double* U0, const double* V0, const d
   g_tc_pairs_min_k = c->tune_pairs_k;
   g_dev_flags = c->d_flags;
   double* buf = nullptr;
-  if ((rc = ctx_scratch(c, 7 * nn + n, &buf))) return rc;
-  EvolveBuf b;
-  b.Z = buf;
-  b.U0 = buf + nn;
-  b.V0 = buf + 2 * nn;
-  b.A1 = buf + 3 * nn;
-  b.A2 = buf + 4 * nn;
-  double* G = buf + 5 * nn;
-  b.L = buf + 6 * nn;
-  rc = upload_matrix(Z, b.Z, sizeof(double) * nn, s);
-  if (!rc) rc = upload_matrix(U0, b.U0, sizeof(double) * nn, s);
-  if (!rc) rc = upload_matrix(V0, b.V0, sizeof(double) * nn, s);
-  if (!rc) rc = evolve_device(c, b, n, ws_U(c), ws_V(c), true);
+  if ((rc = ctx_scratch(c, 6 * nn + evolve_work(n), &buf))) return rc;
+  double *dZ = buf, *dU0 = buf + nn, *dV0 = buf + 2 * nn, *Linv = buf + 3 * nn, *G = buf + 4 * nn, *dE = buf + 5 * nn;
+  rc = upload_matrix(Z, dZ, sizeof(double) * nn, s);
+  if (!rc) rc = upload_matrix(U0, dU0, sizeof(double) * nn, s);
+  if (!rc) rc = upload_matrix(V0, dV0, sizeof(double) * nn, s);
+  if (!rc) rc = evolve_device(c, dZ, dU0, dV0, buf + 6 * nn, n, ws_U(c), ws_V(c), Linv);
   if (!rc) rc = check_flags(c);
   tvap_pnp p{};
   if (!rc) rc = project_device(c, *opts, &p);
   if (!rc) {
     // dE/dZ = L^{-T} H20v L^{-1}
-    const View Li = view_cm(b.L, n, 0);
+    const View Li = view_cm(Linv, n, 0);
     rc = rgemm(n, n, n, view_cm(ws_H20v(c), n, 0), Li, G, n, 1.0, 0.0, s);
-    if (!rc) rc = rgemm(n, n, n, view_t(Li), view_cm(G, n, 0), b.A1, n, 1.0, 0.0, s);
-    if (!rc) rc = download_matrix(b.A1, dEdZ, sizeof(double) * nn, s);
+    if (!rc) rc = rgemm(n, n, n, view_t(Li), view_cm(G, n, 0), dE, n, 1.0, 0.0, s);
+    if (!rc) rc = download_matrix(dE, dEdZ, sizeof(double) * nn, s);
     if (!rc) {
       if (cudaStreamSynchronize(s) != cudaSuccess) rc = TVAP_ERR_CUDA;
       const double ore = p.over[0], oim = p.over[1], ere = p.ener[0], eim = p.ener[1];

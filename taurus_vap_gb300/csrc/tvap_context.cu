@@ -301,8 +301,8 @@ int tvap_init(tvap_ctx** ctx, int64_t n, const int32_t* sp_2mj, const int32_t* s
   if ((e = cudaMalloc(&c->d_sp_l, sizeof(int) * n)) != cudaSuccess) return fail(e);
   // the status word, then words for the non-finite check of caller matrices
   if ((e = cudaMalloc(&c->d_flags, 8 * sizeof(int))) != cudaSuccess) return fail(e);
-  if ((e = cudaMalloc(&c->d_bar, 4 * sizeof(unsigned))) != cudaSuccess) return fail(e);
-  cudaMemset(c->d_bar, 0, 4 * sizeof(unsigned));
+  if ((e = cudaMalloc(&c->d_bar, tvap::kEvolveBarWords * sizeof(unsigned))) != cudaSuccess) return fail(e);
+  cudaMemset(c->d_bar, 0, tvap::kEvolveBarWords * sizeof(unsigned));
   cudaMemcpy(c->d_sp_2mj, sp_2mj, sizeof(int) * n, cudaMemcpyHostToDevice);
   cudaMemcpy(c->d_sp_tr, sp_tr, sizeof(int) * n, cudaMemcpyHostToDevice);
   cudaMemcpy(c->d_sp_l, sp_l, sizeof(int) * n, cudaMemcpyHostToDevice);

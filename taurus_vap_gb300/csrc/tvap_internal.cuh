@@ -297,7 +297,7 @@ struct tvap_ctx {
   void* h_pin = nullptr;  // pinned host buffer (kPinnedBytes) for the status word and small results
   tvap::Workspace* ws = nullptr;
   int* d_flags = nullptr;  // device status word
-  unsigned* d_bar = nullptr;  // grid-barrier state of the cooperative kernels (3 words)
+  unsigned* d_bar = nullptr;  // grid-barrier state of the cooperative evolution (kEvolveBarWords words)
   int kernel_launches = 0;  // launches issued by the last top-level call
   int gemm_mode = 2;        // 0: FP64 pipe, 1/2: FP64 emulated on the bf16 tensor cores (mma.sync / tcgen05)
   // optional section timing with CUDA events on the context's stream
@@ -398,11 +398,16 @@ int jacobi_cluster(int n, const double* M, int m_transposed, const double* W0, d
                    cudaStream_t s);
 // Cholesky L L^T = A (lower), then L^{-1} in place
 int cholesky_inverse(int n, double* A, int* flags, cudaStream_t s);
-// Cholesky L L^T = S (S overwritten by L, lower) and X_m = A_m L^{-T} for
-// m = 0, 1 (A_1 at A + a_stride, X_1 at X + x_stride) in one cooperative
-// launch; TVAP_ERR_ARG when n is outside its range (the caller then uses
-// cholesky_inverse and two products)
-int cholesky_evolve_coop(int n, double* S, const double* A, long long a_stride, double* X, long long x_stride,
-                         unsigned* bar, int* flags, cudaStream_t s, int skip_cta = -1);
+// The Thouless evolution in one cooperative launch: U1 = (U0 + V0 Z) L^{-T},
+// V1 = (V0 + U0 Z) L^{-T}, L L^T = 1 + Z^T Z, and L^{-1} (zeros above the
+// diagonal) when Linv is not null.  work: evolve_work(n) doubles, A1, A2 (2 n^2)
+// then S (n^2 + n), which the caller fills with U0 + V0 Z, V0 + U0 Z and
+// 1 + Z^T Z unless evolve_forms_products(n).  bar: kEvolveBarWords words.
+// TVAP_ERR_ARG when n is outside its range.
+constexpr int kEvolveBarWords = 16;
+size_t evolve_work(int n);
+bool evolve_forms_products(int n);
+int thouless_evolve(int n, const double* Z, const double* U0, const double* V0, double* work, double* U1, double* V1,
+                    double* Linv, unsigned* bar, int* flags, cudaStream_t s, int skip_cta = -1);
 
 }  // namespace tvap
