@@ -4,7 +4,6 @@
 //
 // Per iteration (at most 100, as in the reference):
 //   (U1, V1) = evolve(U0, V0, Z_i)                      cholesky + evolve
-//   rho = V1 V1^T, kappa = V1 U1^T                       calculate_densities_real
 //   <C_m> = Tr(C_m rho) (one-body), Tr(C_m kappa^T) (pair)  calculate_expectval_*
 //   C20_m = f20(C_m) or g20(C_m) at (U1, V1)             set_operator_qpbasis
 //   stop when every |target_m - <C_m>| <= eps
@@ -12,6 +11,14 @@
 // Everything but the c x c solve runs on the device; the expectation values
 // and the Gram matrix come back in one read per iteration (fixed-order
 // reductions, no atomics), the c-vector x goes down.
+//
+// The densities themselves are not needed: with W_m = C_m V1 the expectation
+// value is Tr(C_m V1 V1^T) = sum V1 o W_m, and with the pair operators'
+// W_m = C_m U1 it is Tr(C_m (V1 U1^T)^T) = sum V1 o W_m as well.  The second
+// term of f20, V^T C^T U, is the transpose of the first, U^T C V = U^T W_m.  So
+// the operators of a step take two batched products (two more for pair
+// operators: V^T C V), where two densities and four single products per
+// operator took 14 products with three constraints (n = 140: 218 -> 53 us a step).
 
 #include <cmath>
 #include <vector>
@@ -23,8 +30,6 @@ namespace tvap {
 int upload_matrix(const void* src, void* dst, size_t bytes, cudaStream_t s);
 int download_matrix(const void* src, void* dst, size_t bytes, cudaStream_t s);
 int check_flags(tvap_ctx* c);
-int real_product(int M, int N, int K, View A, View B, double* C, int ldc, double alpha, double beta,
-                 cudaStream_t s);
 int evolve_state(tvap_ctx* c, const double* U0, const double* V0, const double* Z, double* U1, double* V1,
                  double* work);
 
@@ -34,22 +39,17 @@ constexpr int kDotThreads = 256;
 constexpr int kDotBlocks = 64;
 
 // partial[p * kDotBlocks + b] = sum over block b's share of x_p[i] y_p[i]
-// (y_p read transposed when tr_p: the (i, j) entry of y is at j + i n)
 struct DotJob {
   const double* x;
   const double* y;
-  int tr;
 };
-__global__ void __launch_bounds__(kDotThreads) dot_partial_kernel(int n, const DotJob* __restrict__ jobs,
+__global__ void __launch_bounds__(kDotThreads) dot_partial_kernel(size_t nn, const DotJob* __restrict__ jobs,
                                                                double* __restrict__ partial) {
   __shared__ double red[kDotThreads / 32];
   const DotJob J = jobs[blockIdx.y];
-  const size_t nn = size_t(n) * n;
   double s = 0.0;
-  for (size_t i = blockIdx.x * size_t(kDotThreads) + threadIdx.x; i < nn; i += size_t(kDotBlocks) * kDotThreads) {
-    const size_t iy = J.tr ? (i / n) + (i % n) * size_t(n) : i;
-    s = fma(J.x[i], J.y[iy], s);
-  }
+  for (size_t i = blockIdx.x * size_t(kDotThreads) + threadIdx.x; i < nn; i += size_t(kDotBlocks) * kDotThreads)
+    s = fma(J.x[i], J.y[i], s);
   for (int off = 16; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
   __syncthreads();
@@ -68,15 +68,23 @@ __global__ void dot_finish_kernel(int njobs, const double* __restrict__ partial,
   out[p] = t;
 }
 
-// B = 1/2 (A1 - A1^T) with A1 = A2 - A3 (the '20' parts of
-// set_operator_qpbasis, factor -1, module_operators.f90:49-97)
-__global__ void part20_finish_kernel(int n, const double* __restrict__ A2, const double* __restrict__ A3,
+// The '20' parts of set_operator_qpbasis (factor -1, module_operators.f90:
+// 49-97), B = 1/2 (A1 - A1^T): one-body A1 = P - P^T (P = U^T C V), pair
+// A1 = P - Q (P = U^T C U, Q = V^T C V).  blockIdx.y = operator; P and B hold
+// all of them, Q the pair operators (m >= c1).
+__global__ void part20_finish_kernel(int n, int c1, const double* __restrict__ P, const double* __restrict__ Q,
                                      double* __restrict__ B) {
-  const size_t idx = blockIdx.x * size_t(blockDim.x) + threadIdx.x;
-  if (idx >= size_t(n) * n) return;
-  const int i = int(idx % n), j = int(idx / n);
-  const size_t ji = j + size_t(i) * n;
-  B[idx] = 0.5 * ((A2[idx] - A3[idx]) - (A2[ji] - A3[ji]));
+  const size_t nn = size_t(n) * n, idx = blockIdx.x * size_t(blockDim.x) + threadIdx.x;
+  if (idx >= nn) return;
+  const int m = blockIdx.y;
+  const size_t ji = idx / n + (idx % n) * size_t(n);
+  const double* p = P + m * nn;
+  if (m < c1) {
+    B[m * nn + idx] = p[idx] - p[ji];
+  } else {
+    const double* q = Q + (m - c1) * nn;
+    B[m * nn + idx] = 0.5 * ((p[idx] - q[idx]) - (p[ji] - q[ji]));
+  }
 }
 
 // Z += sum_m x_m C_m
@@ -138,17 +146,24 @@ int tvap_adjust_constraints(tvap_ctx* c, const double* U0, const double* V0, dou
   const size_t nn = size_t(n) * n;
   cudaStream_t s = c->stream;
   const int njobs = cdim + cdim * (cdim + 1) / 2;
-  // U0, V0, Z, U1, V1, rho, kappa, T1, T2, T3, evolution work, the operators, C20, x, partial sums and results, the jobs
+  // U0, V0, Z, U1, V1, evolution work, the operators, C20, W and P (U^T W) of
+  // every operator, C V and V^T C V of the pair operators, x, partial sums and
+  // results, the jobs
   double* buf = nullptr;
+  const int c1 = cdim - cpair;
   const size_t jobs_doubles = (sizeof(DotJob) * size_t(njobs > 0 ? njobs : 1) + 7) / 8;
-  const size_t tot = 10 * nn + evolve_work(n) + 2 * size_t(cdim) * nn + cdim + size_t(njobs) * (kDotBlocks + 1) + jobs_doubles + 2;
+  const size_t tot = 5 * nn + evolve_work(n) + (4 * size_t(cdim) + 2 * size_t(cpair)) * nn + cdim +
+                     size_t(njobs) * (kDotBlocks + 1) + jobs_doubles + 2;
   int rc;
   if ((rc = ctx_scratch(c, tot, &buf))) return rc;
-  double *dU0 = buf, *dV0 = dU0 + nn, *dZ = dV0 + nn, *dU1 = dZ + nn, *dV1 = dU1 + nn, *rho = dV1 + nn,
-         *kap = rho + nn, *T1 = kap + nn, *T2 = T1 + nn, *T3 = T2 + nn, *work = T3 + nn;
+  double *dU0 = buf, *dV0 = dU0 + nn, *dZ = dV0 + nn, *dU1 = dZ + nn, *dV1 = dU1 + nn, *work = dV1 + nn;
   double* cops = work + evolve_work(n);
   double* c20 = cops + size_t(cdim) * nn;
-  double* dx = c20 + size_t(cdim) * nn;
+  double* W = c20 + size_t(cdim) * nn;
+  double* P = W + size_t(cdim) * nn;
+  double* Wv = P + size_t(cdim) * nn;
+  double* Q = Wv + size_t(cpair) * nn;
+  double* dx = Q + size_t(cpair) * nn;
   double* partial = dx + cdim;
   double* results = partial + size_t(njobs) * kDotBlocks;
   DotJob* djobs = reinterpret_cast<DotJob*>(results + njobs + (njobs & 1));
@@ -159,43 +174,43 @@ int tvap_adjust_constraints(tvap_ctx* c, const double* U0, const double* V0, dou
   // the dot products of one iteration: the expectation values, then the
   // upper triangle of the Gram matrix of the C20
   std::vector<DotJob> jobs;
-  for (int m = 0; m < cdim; ++m) {
-    if (m < cdim - cpair)
-      jobs.push_back({cops + m * nn, rho, 1});  // Tr(C rho) = sum C_ik rho_ki
-    else
-      jobs.push_back({cops + m * nn, kap, 0});  // Tr(C kappa^T) = sum C_ik kappa_ik
-  }
+  for (int m = 0; m < cdim; ++m) jobs.push_back({dV1, W + m * nn});
   for (int i = 0; i < cdim; ++i)
-    for (int j = i; j < cdim; ++j) jobs.push_back({c20 + i * nn, c20 + j * nn, 0});
+    for (int j = i; j < cdim; ++j) jobs.push_back({c20 + i * nn, c20 + j * nn});
   if (njobs > 0) TVAP_CUDA(cudaMemcpyAsync(djobs, jobs.data(), sizeof(DotJob) * njobs, cudaMemcpyHostToDevice, s));
   const View Uv = view_cm(dU1, n, 0), Vv = view_cm(dV1, n, 0);
   const int tb = 256;
   const unsigned nb = unsigned((nn + tb - 1) / tb);
+  // C_q = A_q B_q for q < count, a stride of 0 for a shared operand
+  auto product = [&](int count, View A, View B, double* C) -> int {
+    if (count == 0) return TVAP_OK;
+    GemmArgs g{};
+    g.M = g.N = g.K = n;
+    g.batch = count;
+    g.A = A;
+    g.B = B;
+    g.C = C;
+    g.crs = 1;
+    g.ccs = n;
+    g.cbs = (long long)nn;
+    g.alpha = make_double2(1.0, 0.0);
+    g.beta = make_double2(0.0, 0.0);
+    g.a_real = g.b_real = g.c_real = true;
+    return gemm(g, s);
+  };
   std::vector<double> res(njobs), x(cdim);
   int iter = 0;
   for (iter = 1; iter <= 100; ++iter) {
     if ((rc = evolve_state(c, dU0, dV0, dZ, dU1, dV1, work))) return rc;
     if (cdim == 0) break;
-    if ((rc = real_product(n, n, n, Vv, view_t(Vv), rho, n, 1.0, 0.0, s))) return rc;
-    if ((rc = real_product(n, n, n, Vv, view_t(Uv), kap, n, 1.0, 0.0, s))) return rc;
-    for (int m = 0; m < cdim; ++m) {
-      const View A = view_cm(cops + m * nn, n, 0);
-      if (m < cdim - cpair) {
-        // f20: U^T A V - V^T A^T U
-        if ((rc = real_product(n, n, n, view_t(Uv), A, T1, n, 1.0, 0.0, s))) return rc;
-        if ((rc = real_product(n, n, n, view_cm(T1, n, 0), Vv, T2, n, 1.0, 0.0, s))) return rc;
-        if ((rc = real_product(n, n, n, view_t(Vv), view_t(A), T1, n, 1.0, 0.0, s))) return rc;
-        if ((rc = real_product(n, n, n, view_cm(T1, n, 0), Uv, T3, n, 1.0, 0.0, s))) return rc;
-      } else {
-        // g20: U^T A U - V^T A V
-        if ((rc = real_product(n, n, n, view_t(Uv), A, T1, n, 1.0, 0.0, s))) return rc;
-        if ((rc = real_product(n, n, n, view_cm(T1, n, 0), Uv, T2, n, 1.0, 0.0, s))) return rc;
-        if ((rc = real_product(n, n, n, view_t(Vv), A, T1, n, 1.0, 0.0, s))) return rc;
-        if ((rc = real_product(n, n, n, view_cm(T1, n, 0), Vv, T3, n, 1.0, 0.0, s))) return rc;
-      }
-      part20_finish_kernel<<<nb, tb, 0, tvap::counted(s)>>>(n, T2, T3, c20 + m * nn);
-    }
-    dot_partial_kernel<<<dim3(kDotBlocks, njobs), kDotThreads, 0, tvap::counted(s)>>>(n, djobs, partial);
+    const View ops = view_cm(cops, n, (long long)nn), opsp = view_cm(cops + c1 * nn, n, (long long)nn);
+    if ((rc = product(c1, ops, Vv, W))) return rc;
+    if ((rc = product(cpair, opsp, Uv, W + c1 * nn))) return rc;
+    if ((rc = product(cdim, view_t(Uv), view_cm(W, n, (long long)nn), P))) return rc;
+    if ((rc = product(cpair, opsp, Vv, Wv))) return rc;
+    if ((rc = product(cpair, view_t(Vv), view_cm(Wv, n, (long long)nn), Q))) return rc;
+    part20_finish_kernel<<<dim3(nb, cdim), tb, 0, tvap::counted(s)>>>(n, c1, P, Q, c20);
+    dot_partial_kernel<<<dim3(kDotBlocks, njobs), kDotThreads, 0, tvap::counted(s)>>>(nn, djobs, partial);
     dot_finish_kernel<<<(njobs + 127) / 128, 128, 0, tvap::counted(s)>>>(njobs, partial, results);
     TVAP_CUDA(cudaGetLastError());
     TVAP_CUDA(cudaMemcpyAsync(res.data(), results, sizeof(double) * njobs, cudaMemcpyDeviceToHost, s));
