@@ -2693,7 +2693,9 @@ int angles_overlap(tvap_ctx* c, int G, const double2* d_ephase, int nocc, int ne
 // Thouless chain of angles [0, G) on stream s (needs only U, V and their
 // blocks): U_phi, V_phi, A_phi, U~, V~, the transition densities, the fields,
 // the traces and H20.
-int angles_thouless(tvap_ctx* c, int G, const double2* d_ephase, double factor_delta, cudaStream_t s) {
+// want_h20 = false stops after the traces.
+int angles_thouless(tvap_ctx* c, int G, const double2* d_ephase, double factor_delta, cudaStream_t s,
+                    bool want_h20 = true) {
   Workspace* w = c->ws;
   const int n = c->n;
   const size_t nn = size_t(n) * n;
@@ -2775,11 +2777,11 @@ int angles_thouless(tvap_ctx* c, int G, const double2* d_ephase, double factor_d
   traces_finish_kernel<<<G, 9 * 32, 0, tvap::counted(st)>>>(G, w->tpart, c->H0, w->obs);
   TVAP_CUDA(cudaGetLastError());
   sec_end_on(c, SEC_TRACES, st);
-  sec_begin_on(c, SEC_H20, s);
+  if (want_h20) sec_begin_on(c, SEC_H20, s);
   // H20: T = U~^T (h V~ + fd/2 DeltaLR U~) - fd/2 V~^T DeltaRL V~, H20 = T - T^T,
   // as three products: X = [h | DeltaLR] [V~; fd/2 U~], Y = DeltaRL V~ and
   // T = [U~^T | V~^T] [X; -fd/2 Y] (the first and the last stacked along K)
-  {
+  if (want_h20) {
     TcTimingScope tc_timing(c, SEC_H20_TC);
     const View hv{w->hsp, (long long)G, (long long)n * G, 1};
     const View dl{w->dLR, (long long)G, (long long)n * G, 1};
@@ -2815,7 +2817,7 @@ int angles_thouless(tvap_ctx* c, int G, const double2* d_ephase, double factor_d
     g.C = w->T;
     if ((rc = gemm(g, s))) return rc;
   }
-  sec_end_on(c, SEC_H20, s);
+  if (want_h20) sec_end_on(c, SEC_H20, s);
   if (st != s) {
     TVAP_CUDA(cudaEventRecord(c->ev_join2, st));
     TVAP_CUDA(cudaStreamWaitEvent(s, c->ev_join2, 0));
@@ -2824,9 +2826,9 @@ int angles_thouless(tvap_ctx* c, int G, const double2* d_ephase, double factor_d
 }
 
 // Contribution of angles [0, G) to the gauge sums (accumulate = 0 starts new
-// sums), after both chains.
+// sums), after both chains; want_h20: the matrix sums of the gradient too.
 int angles_sums(tvap_ctx* c, int G, const double2* d_weight, const double* d_mult, bool have_overlap,
-                int accumulate, cudaStream_t s) {
+                int accumulate, cudaStream_t s, bool want_h20 = true) {
   Workspace* w = c->ws;
   const int n = c->n;
   const size_t nn = size_t(n) * n;
@@ -2835,7 +2837,8 @@ int angles_sums(tvap_ctx* c, int G, const double2* d_weight, const double* d_mul
   overlap_finish_kernel<<<nblk(G, tb), tb, 0, tvap::counted(s)>>>(n, G, have_overlap ? 1 : 0, w->canon_i, w->canon_d, w->pf,
                                                     w->detR22, d_weight, d_mult, w->obs, w->coefA, w->coefAE);
   sum_scalars_kernel<<<1, 32, 0, tvap::counted(s)>>>(G, w->obs, d_mult, d_weight, w->pscal, accumulate);
-  sum_matrices_kernel<<<unsigned((nn + 31) / 32), 32 * kSumWarps, sizeof(double2) * 3 * size_t(G), tvap::counted(s)>>>(
+  if (want_h20)
+    sum_matrices_kernel<<<unsigned((nn + 31) / 32), 32 * kSumWarps, sizeof(double2) * 3 * size_t(G), tvap::counted(s)>>>(
       n, G, w->A, w->T, w->coefA, w->coefAE, d_mult, w->pA, w->pH, w->pAH, accumulate);
   TVAP_CUDA(cudaGetLastError());
   sec_end_on(c, SEC_SUMS, s);
@@ -3051,14 +3054,36 @@ namespace {
 
 constexpr int kObsRows = 8;       // rows per CTA of the trace kernels
 constexpr int kObsThreads = 128;  // threads over the angles
+constexpr int kObsCols = 32;      // angles per CTA of the kernels with one row per warp
 
 // part[((ch * nops + k) * 2 + t) * G + b] = sum over the rows i of chunk ch
-// of isospin t of (B_k rho_b)(i, i) = sum_j B_k(i, j) rho_b(j, i)
+// of isospin t of (B_k rho_b)(i, i) = sum_j B_k(i, j) rho_b(j, i).  The
+// operators of print_results are sparse (one to a dozen entries a row, most
+// of them real): each warp lists the non-zero columns of its rows in order,
+// and the angles run over the lists only (26 operators, n = 80, 81 angles:
+// 307 us and 54 M FMAs with every entry).  nz: kObsRows lists of n indices.
 __global__ void __launch_bounds__(kObsThreads)
     obs_trace_kernel(int n, int G, const double2* __restrict__ ops, const double2* __restrict__ rho,
                      double2* __restrict__ part) {
+  extern __shared__ unsigned short nz[];
+  __shared__ int cnt[kObsRows];
   const int k = blockIdx.x, nops = gridDim.x, ch = blockIdx.y, h = n / 2;
   const double2* B = ops + size_t(k) * n * n;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (int r = warp; r < kObsRows; r += kObsThreads / 32) {
+    const int i = ch * kObsRows + r;
+    int m = 0;
+    for (int j0 = 0; i < n && j0 < n; j0 += 32) {
+      const int j = j0 + lane;
+      const double2 v = j < n ? B[i + size_t(j) * n] : make_double2(0.0, 0.0);
+      const bool is = v.x != 0.0 || v.y != 0.0;
+      const unsigned mask = __ballot_sync(0xffffffffu, is);
+      if (is) nz[r * n + m + __popc(mask & ((1u << lane) - 1u))] = static_cast<unsigned short>(j);
+      m += __popc(mask);
+    }
+    if (lane == 0) cnt[r] = m;
+  }
+  __syncthreads();
   const int b = blockIdx.z * blockDim.x + threadIdx.x;
   if (b >= G) return;
   double2 sp = make_double2(0.0, 0.0), sn = make_double2(0.0, 0.0);
@@ -3066,7 +3091,18 @@ __global__ void __launch_bounds__(kObsThreads)
     const int i = ch * kObsRows + r;
     if (i >= n) break;
     double2 acc = make_double2(0.0, 0.0);
-    for (int j = 0; j < n; ++j) cfma(acc, B[i + size_t(j) * n], rho[(size_t(j) + size_t(i) * n) * G + b]);
+    const int m = cnt[r];
+#pragma unroll 4
+    for (int q = 0; q < m; ++q) {
+      const int j = nz[r * n + q];
+      const double2 v = B[i + size_t(j) * n], x = rho[(size_t(j) + size_t(i) * n) * G + b];
+      if (v.y == 0.0) {
+        acc.x = fma(v.x, x.x, acc.x);
+        acc.y = fma(v.x, x.y, acc.y);
+      } else {
+        cfma(acc, v, x);
+      }
+    }
     if (i < h)
       sp = cadd(sp, acc);
     else
@@ -3076,40 +3112,159 @@ __global__ void __launch_bounds__(kObsThreads)
   part[((size_t(ch) * nops + k) * 2 + 1) * G + b] = sn;
 }
 
-// part[(ch * 10 + q) * G + b] for the rows i of chunk ch: q = 0..3 PH pp, pn,
-// np, nn = 0.5 sum gamma(i, j) rho(j, i); q = 4..7 PP = 0.5 sum delta(i, j)
-// kappaRL(i, j) (i, j in the blocks' isospins); q = 8, 9 the <O^2> terms
-// sum_j X(i, j) X(j, i) and sum_j Y1(i, j) Y2(i, j) when X is given
-__global__ void __launch_bounds__(kObsThreads)
-    obs_blocks_kernel(int n, int G, const double2* __restrict__ rho, const double2* __restrict__ kRL,
-                      const double2* __restrict__ gam, const double2* __restrict__ dLR,
-                      const double2* __restrict__ X, const double2* __restrict__ Y1, const double2* __restrict__ Y2,
-                      double2* __restrict__ part) {
-  const int ch = blockIdx.x, h = n / 2;
-  const int b = blockIdx.y * blockDim.x + threadIdx.x;
-  if (b >= G) return;
-  auto at = [G, n, b](const double2* A, int i, int j) { return A[(size_t(i) + size_t(j) * n) * G + b]; };
-  double2 a[10];
-#pragma unroll
-  for (int q = 0; q < 10; ++q) a[q] = make_double2(0.0, 0.0);
-  for (int r = 0; r < kObsRows; ++r) {
-    const int i = ch * kObsRows + r;
-    if (i >= n) break;
-    const int ti = i >= h ? 2 : 0;
-    for (int j = 0; j < n; ++j) {
-      const int q = ti + (j >= h ? 1 : 0);
-      if (gam) {
-        cfma(a[q], at(gam, i, j), at(rho, j, i));
-        cfma(a[4 + q], at(dLR, i, j), at(kRL, i, j));
-      }
-      if (X) {
-        cfma(a[8], at(X, i, j), at(X, j, i));
-        cfma(a[9], at(Y1, i, j), at(Y2, i, j));
-      }
+// Sums a value over the 8 warps of a CTA (one row each) in order; the result
+// is that of warp 0's threads.
+__device__ __forceinline__ double2 sum_rows(double2 v, double2 (*red)[kObsCols]) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  __syncthreads();
+  red[warp][lane] = v;
+  __syncthreads();
+  double2 t = make_double2(0.0, 0.0);
+  if (warp == 0)
+    for (int w = 0; w < kObsRows; ++w) t = cadd(t, red[w][lane]);
+  return t;
+}
+
+// The isospin blocks of the energy decomposition, part[(ch * 8 + q) * G + b]:
+// q = 0..3 PH pp, pn, np, nn = 0.5 sum gamma(i, j) rho(j, i), q = 4..7 PP =
+// 0.5 sum delta(i, j) kappaRL(i, j), i over the 8 rows of chunk ch of its
+// isospin, j over the other's.  One warp per row, lanes over the angles;
+// blockIdx.y = the isospin pair: the pair is fixed for a CTA, so that two
+// accumulators suffice (indexing ten of them by the pair kept them in local
+// memory, on 10 CTAs at n = 80: 670 us).
+__global__ void __launch_bounds__(32 * kObsRows)
+    obs_energy_kernel(int n, int G, const double2* __restrict__ rho, const double2* __restrict__ kRL,
+                      const double2* __restrict__ gam, const double2* __restrict__ dLR, double2* __restrict__ part) {
+  __shared__ double2 red[kObsRows][kObsCols];
+  const int h = n / 2, ch = blockIdx.x, q = blockIdx.y, lane = threadIdx.x & 31;
+  const int il = ch * kObsRows + (threadIdx.x >> 5), i = il + (q >> 1) * h, j0 = (q & 1) * h;
+  const int b = blockIdx.z * kObsCols + lane;
+  double2 ph = make_double2(0.0, 0.0), pp = make_double2(0.0, 0.0);
+  if (il < h && b < G) {
+#pragma unroll 4
+    for (int j = j0; j < j0 + h; ++j) {
+      const size_t ij = (size_t(i) + size_t(j) * n) * G + b, ji = (size_t(j) + size_t(i) * n) * G + b;
+      cfma(ph, gam[ij], rho[ji]);
+      cfma(pp, dLR[ij], kRL[ij]);
     }
   }
-#pragma unroll
-  for (int q = 0; q < 10; ++q) part[(size_t(ch) * 10 + q) * G + b] = (q < 8) ? cscale(a[q], 0.5) : a[q];
+  ph = sum_rows(ph, red);
+  pp = sum_rows(pp, red);
+  if (threadIdx.x < kObsCols && b < G) {
+    part[(size_t(ch) * 8 + q) * G + b] = cscale(ph, 0.5);
+    part[(size_t(ch) * 8 + 4 + q) * G + b] = cscale(pp, 0.5);
+  }
+}
+
+// part[(ch * 2 + q) * G + b] for the rows i of chunk ch: the <O^2> terms
+// q = 0: sum_j X(i, j) X(j, i), q = 1: sum_j Y1(i, j) Y2(i, j)
+__global__ void __launch_bounds__(32 * kObsRows)
+    obs_squares_kernel(int n, int G, const double2* __restrict__ X, const double2* __restrict__ Y1,
+                       const double2* __restrict__ Y2, double2* __restrict__ part) {
+  __shared__ double2 red[kObsRows][kObsCols];
+  const int ch = blockIdx.x, i = ch * kObsRows + (threadIdx.x >> 5);
+  const int b = blockIdx.z * kObsCols + (threadIdx.x & 31);
+  double2 x2 = make_double2(0.0, 0.0), y2 = make_double2(0.0, 0.0);
+  if (i < n && b < G) {
+#pragma unroll 4
+    for (int j = 0; j < n; ++j) {
+      const size_t ij = (size_t(i) + size_t(j) * n) * G + b, ji = (size_t(j) + size_t(i) * n) * G + b;
+      cfma(x2, X[ij], X[ji]);
+      cfma(y2, Y1[ij], Y2[ij]);
+    }
+  }
+  x2 = sum_rows(x2, red);
+  y2 = sum_rows(y2, red);
+  if (threadIdx.x < kObsCols && b < G) {
+    part[(size_t(ch) * 2 + 0) * G + b] = x2;
+    part[(size_t(ch) * 2 + 1) * G + b] = y2;
+  }
+}
+
+// Sparse form of the <O^2> operators: the non-zero columns of each row and
+// the non-zero rows of each column of operator q = blockIdx.y (O_q at
+// ops + 2 q n^2), at most kSparseMax of each, in order; *overflow is raised
+// for an operator with more (the products are formed then).  One warp per
+// row or column.
+constexpr int kSparseMax = 8;
+struct SparseOps {
+  int* count;             // [nsq][2][n]
+  unsigned short* index;  // [nsq][2][n][kSparseMax]
+  double2* value;         // [nsq][2][n][kSparseMax]
+};
+__global__ void __launch_bounds__(128)
+    obs_sparse_kernel(int n, const double2* __restrict__ ops, SparseOps sp, int* __restrict__ overflow) {
+  const int line = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (line >= 2 * n) return;
+  const int q = blockIdx.y, byc = line >= n ? 1 : 0, i = line - byc * n;
+  const double2* O = ops + size_t(2 * q) * n * n;
+  const size_t at = (size_t(q) * 2 + byc) * n + i;
+  int m = 0;
+  for (int j0 = 0; j0 < n; j0 += 32) {
+    const int j = j0 + lane;
+    const double2 v = j < n ? (byc ? O[j + size_t(i) * n] : O[i + size_t(j) * n]) : make_double2(0.0, 0.0);
+    const bool is = v.x != 0.0 || v.y != 0.0;
+    const unsigned mask = __ballot_sync(0xffffffffu, is);
+    const int k = m + __popc(mask & ((1u << lane) - 1u));
+    if (is && k < kSparseMax) {
+      sp.index[at * kSparseMax + k] = static_cast<unsigned short>(j);
+      sp.value[at * kSparseMax + k] = v;
+    }
+    m += __popc(mask);
+  }
+  if (lane == 0) {
+    sp.count[at] = min(m, kSparseMax);
+    if (m > kSparseMax) atomicOr(overflow, 1);
+  }
+}
+
+// The <O^2> terms of obs_squares_kernel straight from the sparse operators
+// (blockIdx.y = operator; X = O rho, Y1 = kappaRL O, Y2 = O kappaLR, an
+// element of each from a handful of entries): part of operator q at
+// part + q * 2 * nch * G.  J_x, J_y, J_z have at most two entries a row, so
+// that this costs the reading of the densities: the three operators at n = 80,
+// 81 angles, take 202 us in one launch, where each took three complex
+// products with their digit planes (300 us) and a 670 us reduction.
+__global__ void __launch_bounds__(32 * kObsRows)
+    obs_sparse_squares_kernel(int n, int G, SparseOps sp, const double2* __restrict__ rho,
+                              const double2* __restrict__ kLR, const double2* __restrict__ kRL,
+                              double2* __restrict__ part) {
+  __shared__ double2 red[kObsRows][kObsCols];
+  const int ch = blockIdx.x, q = blockIdx.y, i = ch * kObsRows + (threadIdx.x >> 5);
+  const int b = blockIdx.z * kObsCols + (threadIdx.x & 31);
+  double2 x2 = make_double2(0.0, 0.0), y2 = make_double2(0.0, 0.0);
+  if (i < n && b < G) {
+    auto el = [G, n, b](const double2* A, int r, int c) { return A[(size_t(r) + size_t(c) * n) * G + b]; };
+    const size_t rows = size_t(q) * 2 * n, cols = rows + n;
+    const int ci = sp.count[rows + i];
+    for (int j = 0; j < n; ++j) {
+      double2 xij = make_double2(0.0, 0.0), xji = xij, y1 = xij, yb = xij;
+      for (int k = 0; k < ci; ++k) {
+        const size_t e = (rows + i) * kSparseMax + k;
+        const double2 v = sp.value[e];
+        cfma(xij, v, el(rho, sp.index[e], j));
+        cfma(yb, v, el(kLR, sp.index[e], j));
+      }
+      const int cj = sp.count[rows + j], dj = sp.count[cols + j];
+      for (int k = 0; k < cj; ++k) {
+        const size_t e = (rows + j) * kSparseMax + k;
+        cfma(xji, sp.value[e], el(rho, sp.index[e], i));
+      }
+      for (int k = 0; k < dj; ++k) {
+        const size_t e = (cols + j) * kSparseMax + k;
+        cfma(y1, el(kRL, i, sp.index[e]), sp.value[e]);
+      }
+      cfma(x2, xij, xji);
+      cfma(y2, y1, yb);
+    }
+  }
+  x2 = sum_rows(x2, red);
+  y2 = sum_rows(y2, red);
+  if (threadIdx.x < kObsCols && b < G) {
+    double2* p = part + size_t(q) * 2 * gridDim.x * G;
+    p[(size_t(ch) * 2 + 0) * G + b] = x2;
+    p[(size_t(ch) * 2 + 1) * G + b] = y2;
+  }
 }
 
 // Q[q * G + b] = sum over the chunks of part[(ch * nq + q) * G + b], in order
@@ -3139,7 +3294,7 @@ __global__ void obs_occ_kernel(int n, int G, int nshell, const int* __restrict__
 }
 
 // <O^2> per angle: tr1^2 + tr2 - tr5 + tr6 (tr1, tr2 = the traces of O and
-// O^2 with rho over both isospins; tr5, tr6 from obs_blocks_kernel)
+// O^2 with rho over both isospins; tr5, tr6 the two terms of the squares)
 __global__ void obs_sq_kernel(int G, const double2* __restrict__ t1p, const double2* __restrict__ t2p,
                               const double2* __restrict__ t56, double2* __restrict__ out) {
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
@@ -3232,115 +3387,73 @@ int project_observables_device(tvap_ctx* c, const tvap_proj_opts& o, int nobo, c
   }
   // the trace operators: obo, H1, then O_k and O2_k of the pairs
   const int ntr = nobo + 1 + 2 * nsq;
-  const int nch = (n + kObsRows - 1) / kObsRows;
+  const int nch = (n + kObsRows - 1) / kObsRows, nchh = (h + kObsRows - 1) / kObsRows;
   // Q: 8 energy blocks, 2 per trace operator, nsq <O^2>, 2 per shell
   const int nq = 8 + 2 * ntr + nsq + 2 * nshell;
-  const size_t part_elems = size_t(nch) * std::max(2 * ntr, 10) * G;
-  double2 *ops = nullptr, *part = nullptr, *Q = nullptr, *sums = nullptr, *obs2 = nullptr, *rsum = nullptr;
-  int *dpar = nullptr, *doff = nullptr;
-  const size_t obs2_elems = 10 * size_t(G);
-  TVAP_CUDA(cudaMallocAsync(reinterpret_cast<void**>(&ops), sizeof(double2) * nn * ntr, s));
-  TVAP_CUDA(cudaMallocAsync(reinterpret_cast<void**>(&part), sizeof(double2) * part_elems, s));
-  TVAP_CUDA(cudaMallocAsync(reinterpret_cast<void**>(&Q), sizeof(double2) * size_t(nq) * G, s));
-  TVAP_CUDA(cudaMallocAsync(reinterpret_cast<void**>(&sums), sizeof(double2) * (nq + 1), s));
-  TVAP_CUDA(cudaMallocAsync(reinterpret_cast<void**>(&obs2), sizeof(double2) * obs2_elems, s));
-  TVAP_CUDA(cudaMallocAsync(reinterpret_cast<void**>(&rsum), sizeof(double2) * nn, s));
-  TVAP_CUDA(cudaMallocAsync(reinterpret_cast<void**>(&dpar), sizeof(int) * n, s));
-  TVAP_CUDA(cudaMallocAsync(reinterpret_cast<void**>(&doff), sizeof(int) * (nshell + 1), s));
-  auto release = [&]() {
-    void* bufs[] = {ops, part, Q, sums, obs2, rsum, dpar, doff};
-    for (void* p : bufs)
-      if (p) cudaFreeAsync(p, s);
-  };
+  // the buffers, from the context's scratch
+  const size_t part_elems = std::max({size_t(nch) * 2 * ntr, size_t(nchh) * 8, size_t(nsq) * 2 * nch}) * G;
+  const size_t sp_lines = size_t(nsq) * 2 * n;
+  const size_t c2_elems = nn * ntr + part_elems + size_t(nq) * G + (nq + 1) + 10 * size_t(G) + nn +
+                          2 * size_t(nsq) * G + sp_lines * kSparseMax;
+  const size_t words = sp_lines * (kSparseMax / 2) + sp_lines + n + (nshell + 1) + 1;  // 32-bit
+  double* buf = nullptr;
+  if ((rc = ctx_scratch(c, 2 * c2_elems + (words + 1) / 2, &buf))) return rc;
+  double2* ops = reinterpret_cast<double2*>(buf);
+  double2 *part = ops + nn * ntr, *Q = part + part_elems, *sums = Q + size_t(nq) * G, *obs2 = sums + nq + 1,
+          *rsum = obs2 + 10 * size_t(G), *sqt = rsum + nn;
+  SparseOps sp{};
+  sp.value = sqt + 2 * size_t(nsq) * G;
+  sp.count = reinterpret_cast<int*>(sp.value + sp_lines * kSparseMax);
+  sp.index = reinterpret_cast<unsigned short*>(sp.count + sp_lines);
+  int* dpar = sp.count + sp_lines + sp_lines * (kSparseMax / 2);
+  int *doff = dpar + n, *overflow = doff + nshell + 1;
+  const size_t nz_shm = sizeof(unsigned short) * kObsRows * size_t(n);
+  if (nz_shm > 48 * 1024) return TVAP_ERR_ARG;  // n > 3072: beyond every other limit of the path
   auto run = [&]() -> int {
     int r;
-    for (int k = 0; k < nobo; ++k)
-      if ((r = upload_matrix(obo + 2 * nn * k, ops + nn * k, sizeof(double2) * nn, s))) return r;
+    if (nobo > 0 && (r = upload_matrix(obo, ops, sizeof(double2) * nn * nobo, s))) return r;
     TVAP_CUDA(cudaMemcpyAsync(ops + nn * nobo, c->d_H1, sizeof(double2) * nn, cudaMemcpyDeviceToDevice, s));
-    for (int k = 0; k < 2 * nsq; ++k)
-      if ((r = upload_matrix(sq + 2 * nn * k, ops + nn * (nobo + 1 + k), sizeof(double2) * nn, s))) return r;
+    const double2* sqops = ops + nn * (nobo + 1);
+    if (nsq > 0 && (r = upload_matrix(sq, ops + nn * (nobo + 1), sizeof(double2) * nn * 2 * nsq, s))) return r;
     std::vector<int> off(nshell + 1, 0);
     for (int k = 0; k < nshell; ++k) off[k + 1] = off[k] + shell_size[k];
     if (off[nshell] > h) return TVAP_ERR_ARG;
     TVAP_CUDA(cudaMemcpyAsync(doff, off.data(), sizeof(int) * (nshell + 1), cudaMemcpyHostToDevice, s));
     if (parity) TVAP_CUDA(cudaMemcpyAsync(dpar, parity, sizeof(int) * n, cudaMemcpyHostToDevice, s));
+    int dense_sq = 0;
+    if (nsq > 0) {
+      TVAP_CUDA(cudaMemsetAsync(overflow, 0, sizeof(int), s));
+      obs_sparse_kernel<<<dim3((2 * n + 3) / 4, nsq), 128, 0, tvap::counted(s)>>>(n, sqops, sp, overflow);
+      TVAP_CUDA(cudaGetLastError());
+      TVAP_CUDA(cudaMemcpyAsync(&dense_sq, overflow, sizeof(int), cudaMemcpyDeviceToHost, s));
+    }
     TVAP_CUDA(cudaStreamSynchronize(s));  // the host vectors go out of scope
-    // the projection itself (densities, fields, overlaps, traces, sums) on
-    // one stream, then the parity-rotated overlaps
+    // the projection itself (densities, fields, overlaps, traces, sums; no
+    // gradient) on the streams of project_device, the parity-rotated overlaps
+    // ahead of the overlaps on the third
     int canon[3] = {0, 0, 0};
+    cudaStream_t s2 = c->stream2, s3 = c->stream3, sm = c->streamM;
+    const int tb = 256;
     sec_mark(c, s);
-    if ((r = prepare_uv_blocks(c, s))) return r;
-    if ((r = prepare_canonical(c, o.seed_occeps, o.seed_allemp, canon, s))) return r;
+    TVAP_CUDA(cudaEventRecord(c->ev_fork, s));
+    TVAP_CUDA(cudaStreamWaitEvent(s2, c->ev_fork, 0));
+    TVAP_CUDA(cudaStreamWaitEvent(sm, c->ev_fork, 0));
+    if ((r = prepare_uv_blocks(c, sm))) return r;
+    if ((r = angles_thouless(c, G, w->ephase, o.factor_delta, sm, false))) return r;
+    TVAP_CUDA(cudaEventRecord(c->ev_main, sm));
+    if ((r = prepare_canonical(c, o.seed_occeps, o.seed_allemp, canon, s2))) return r;
     if (canon[2]) {
       set_last_error("canonical basis: a degenerate subspace larger than 64 or not reducible to 2 x 2 blocks",
                      __FILE__, __LINE__);
       return TVAP_ERR_CANONICAL;
     }
-    if ((r = angles_thouless(c, G, w->ephase, o.factor_delta, s))) return r;
-    if (have_overlap && (r = angles_overlap(c, G, w->ephase, canon[0], canon[1], s))) return r;
-    if ((r = angles_sums(c, G, w->weight, w->mult, have_overlap, 0, s))) return r;
-    nocc_nemp[0] = canon[0];
-    nocc_nemp[1] = canon[1];
-    const int tb = 256;
-    // Q: the energy blocks (and, per pair, the <O^2> terms)
-    const dim3 gblk(nch, (G + kObsThreads - 1) / kObsThreads);
-    obs_blocks_kernel<<<gblk, kObsThreads, 0, tvap::counted(s)>>>(n, G, w->rhoL, w->kRL, w->gam, w->dLR, nullptr,
-                                                                   nullptr, nullptr, part);
-    obs_chunks_kernel<<<nblk(size_t(10) * G, tb), tb, 0, tvap::counted(s)>>>(G, 10, nch, part, obs2);
-    TVAP_CUDA(cudaMemcpyAsync(Q, obs2, sizeof(double2) * 8 * G, cudaMemcpyDeviceToDevice, s));
-    // the traces of the operators
-    const dim3 gtr(ntr, nch, (G + kObsThreads - 1) / kObsThreads);
-    obs_trace_kernel<<<gtr, kObsThreads, 0, tvap::counted(s)>>>(n, G, ops, w->rhoL, part);
-    obs_chunks_kernel<<<nblk(size_t(2 * ntr) * G, tb), tb, 0, tvap::counted(s)>>>(G, 2 * ntr, nch, part,
-                                                                                   Q + size_t(8) * G);
-    TVAP_CUDA(cudaGetLastError());
-    // <O^2>: X = O rho, Y1 = kappaRL O, Y2 = O kappaLR per angle (angle-innermost)
-    for (int k = 0; k < nsq; ++k) {
-      const double2* Op = ops + nn * (nobo + 1 + 2 * k);
-      const View Ov{Op, 1, n, 0};
-      const View rhoV{w->rhoL, (long long)G, (long long)n * G, 1};
-      GemmArgs g{};
-      g.M = g.N = g.K = n;
-      g.batch = G;
-      g.crs = G;
-      g.ccs = (long long)n * G;
-      g.cbs = 1;
-      g.alpha = make_double2(1.0, 0.0);
-      g.beta = make_double2(0.0, 0.0);
-      g.A = Ov;
-      g.B = rhoV;
-      g.C = w->X;
-      if ((r = gemm(g, s))) return r;
-      g.A = View{w->kRL, (long long)G, (long long)n * G, 1};
-      g.B = Ov;
-      g.C = w->Y;
-      if ((r = gemm(g, s))) return r;
-      g.A = Ov;
-      g.B = View{w->kLR, (long long)G, (long long)n * G, 1};
-      g.C = w->T;
-      if ((r = gemm(g, s))) return r;
-      obs_blocks_kernel<<<gblk, kObsThreads, 0, tvap::counted(s)>>>(n, G, w->rhoL, w->kRL, nullptr, nullptr, w->X,
-                                                                     w->Y, w->T, part);
-      obs_chunks_kernel<<<nblk(size_t(10) * G, tb), tb, 0, tvap::counted(s)>>>(G, 10, nch, part, obs2);
-      const double2* tr = Q + size_t(8) * G;
-      obs_sq_kernel<<<nblk(G, tb), tb, 0, tvap::counted(s)>>>(G, tr + size_t(2 * (nobo + 1 + 2 * k)) * G,
-                                                              tr + size_t(2 * (nobo + 2 + 2 * k)) * G,
-                                                              obs2 + size_t(8) * G,
-                                                              Q + size_t(8 + 2 * ntr + k) * G);
-      TVAP_CUDA(cudaGetLastError());
-    }
-    if (nshell > 0)
-      obs_occ_kernel<<<nblk(size_t(nshell) * G, tb), tb, 0, tvap::counted(s)>>>(
-          n, G, nshell, doff, w->rhoL, Q + size_t(8 + 2 * ntr + nsq) * G);
-    // sums with weight x overlap (coefA of angles_sums), and pnp_rho
-    obs_sum_kernel<<<(nq + 3) / 4, 128, 0, tvap::counted(s)>>>(G, nq, Q, w->coefA, sums);
-    obs_rho_kernel<<<nblk(nn, tb), tb, 0, tvap::counted(s)>>>(n, G, w->rhoL, w->coefA, rsum);
-    TVAP_CUDA(cudaGetLastError());
-    // the overlaps with the parity-rotated state: R_n from the blocks
-    // D_t^T Pi D_t (10, 11), then the overlap chain once more
+    TVAP_CUDA(cudaEventRecord(c->ev_canon, s2));
+    TVAP_CUDA(cudaStreamWaitEvent(s3, c->ev_canon, 0));
     double2 pari = make_double2(0.0, 0.0);
     if (parity) {
-      scale_rows_kernel<<<nblk(nn, tb), tb, 0, tvap::counted(s)>>>(n, dpar, w->D, w->tmp);
+      // the overlaps with the parity-rotated state: R_n from the blocks
+      // D_t^T Pi D_t (10, 11)
+      scale_rows_kernel<<<nblk(nn, tb), tb, 0, tvap::counted(s3)>>>(n, dpar, w->D, w->tmp);
       GemmArgs g{};
       g.M = g.N = n;
       g.K = h;
@@ -3354,18 +3467,87 @@ int project_observables_device(tvap_ctx* c, const tvap_proj_opts& o, int nobo, c
       g.alpha = make_double2(1.0, 0.0);
       g.beta = make_double2(0.0, 0.0);
       g.a_real = g.b_real = g.c_real = true;
-      if ((r = gemm(g, s))) return r;
-      if ((r = angles_overlap(c, G, w->ephase, canon[0], canon[1], s, w->blocks + 2 * nn))) return r;
-      // the overlap formula into obs2 (8 G), its coefficients into scratch
-      double2* o2 = obs2;
-      TVAP_CUDA(cudaMemsetAsync(o2, 0, sizeof(double2) * 8 * G, s));
-      overlap_finish_kernel<<<nblk(G, tb), tb, 0, tvap::counted(s)>>>(n, G, 1, w->canon_i, w->canon_d, w->pf,
-                                                                     w->detR22, w->weight, w->mult, o2, part,
-                                                                     part + G);
-      // sum_b weight_b rot_pari_b (the overlaps sit at stride 8 in o2)
-      obs_pari_kernel<<<1, 32, 0, tvap::counted(s)>>>(G, o2, w->weight, sums + nq);
+      if ((r = gemm(g, s3))) return r;
+      if ((r = angles_overlap(c, G, w->ephase, canon[0], canon[1], s3, w->blocks + 2 * nn))) return r;
+      // the overlap formula into obs2 (8 G, the overlaps at stride 8), its
+      // coefficients after it; then sum_b weight_b rot_pari_b
+      TVAP_CUDA(cudaMemsetAsync(obs2, 0, sizeof(double2) * 8 * G, s3));
+      overlap_finish_kernel<<<nblk(G, tb), tb, 0, tvap::counted(s3)>>>(n, G, 1, w->canon_i, w->canon_d, w->pf,
+                                                                      w->detR22, w->weight, w->mult, obs2,
+                                                                      obs2 + 8 * size_t(G), obs2 + 9 * size_t(G));
+      obs_pari_kernel<<<1, 32, 0, tvap::counted(s3)>>>(G, obs2, w->weight, sums + nq);
       TVAP_CUDA(cudaGetLastError());
     }
+    if (have_overlap && (r = angles_overlap(c, G, w->ephase, canon[0], canon[1], s3))) return r;
+    TVAP_CUDA(cudaEventRecord(c->ev_join, s3));
+    TVAP_CUDA(cudaStreamWaitEvent(s, c->ev_main, 0));
+    nocc_nemp[0] = canon[0];
+    nocc_nemp[1] = canon[1];
+    const int gcol = (G + kObsCols - 1) / kObsCols;
+    // Q: the energy blocks
+    obs_energy_kernel<<<dim3(nchh, 4, gcol), 32 * kObsRows, 0, tvap::counted(s)>>>(n, G, w->rhoL, w->kRL, w->gam,
+                                                                                  w->dLR, part);
+    obs_chunks_kernel<<<nblk(size_t(8) * G, tb), tb, 0, tvap::counted(s)>>>(G, 8, nchh, part, Q);
+    // the traces of the operators
+    const dim3 gtr(ntr, nch, (G + kObsThreads - 1) / kObsThreads);
+    obs_trace_kernel<<<gtr, kObsThreads, nz_shm, tvap::counted(s)>>>(n, G, ops, w->rhoL, part);
+    obs_chunks_kernel<<<nblk(size_t(2 * ntr) * G, tb), tb, 0, tvap::counted(s)>>>(G, 2 * ntr, nch, part,
+                                                                                   Q + size_t(8) * G);
+    TVAP_CUDA(cudaGetLastError());
+    // <O^2>
+    if (nsq > 0 && !dense_sq) {
+      obs_sparse_squares_kernel<<<dim3(nch, nsq, gcol), 32 * kObsRows, 0, tvap::counted(s)>>>(
+          n, G, sp, w->rhoL, w->kLR, w->kRL, part);
+      for (int k = 0; k < nsq; ++k)
+        obs_chunks_kernel<<<nblk(size_t(2) * G, tb), tb, 0, tvap::counted(s)>>>(
+            G, 2, nch, part + size_t(k) * 2 * nch * G, sqt + size_t(2 * k) * G);
+      TVAP_CUDA(cudaGetLastError());
+    }
+    for (int k = 0; k < nsq; ++k) {
+      if (dense_sq) {
+        // X = O rho, Y1 = kappaRL O, Y2 = O kappaLR per angle (angle-innermost)
+        const View Ov{sqops + nn * 2 * k, 1, n, 0};
+        const View rhoV{w->rhoL, (long long)G, (long long)n * G, 1};
+        GemmArgs g{};
+        g.M = g.N = g.K = n;
+        g.batch = G;
+        g.crs = G;
+        g.ccs = (long long)n * G;
+        g.cbs = 1;
+        g.alpha = make_double2(1.0, 0.0);
+        g.beta = make_double2(0.0, 0.0);
+        g.A = Ov;
+        g.B = rhoV;
+        g.C = w->X;
+        if ((r = gemm(g, s))) return r;
+        g.A = View{w->kRL, (long long)G, (long long)n * G, 1};
+        g.B = Ov;
+        g.C = w->Y;
+        if ((r = gemm(g, s))) return r;
+        g.A = Ov;
+        g.B = View{w->kLR, (long long)G, (long long)n * G, 1};
+        g.C = w->T;
+        if ((r = gemm(g, s))) return r;
+        obs_squares_kernel<<<dim3(nch, 1, gcol), 32 * kObsRows, 0, tvap::counted(s)>>>(n, G, w->X, w->Y, w->T, part);
+        obs_chunks_kernel<<<nblk(size_t(2) * G, tb), tb, 0, tvap::counted(s)>>>(G, 2, nch, part,
+                                                                               sqt + size_t(2 * k) * G);
+      }
+      const double2* tr = Q + size_t(8) * G;
+      obs_sq_kernel<<<nblk(G, tb), tb, 0, tvap::counted(s)>>>(G, tr + size_t(2 * (nobo + 1 + 2 * k)) * G,
+                                                              tr + size_t(2 * (nobo + 2 + 2 * k)) * G,
+                                                              sqt + size_t(2 * k) * G,
+                                                              Q + size_t(8 + 2 * ntr + k) * G);
+      TVAP_CUDA(cudaGetLastError());
+    }
+    if (nshell > 0)
+      obs_occ_kernel<<<nblk(size_t(nshell) * G, tb), tb, 0, tvap::counted(s)>>>(
+          n, G, nshell, doff, w->rhoL, Q + size_t(8 + 2 * ntr + nsq) * G);
+    // sums with weight x overlap (coefA of angles_sums), and pnp_rho
+    TVAP_CUDA(cudaStreamWaitEvent(s, c->ev_join, 0));
+    if ((r = angles_sums(c, G, w->weight, w->mult, have_overlap, 0, s, false))) return r;
+    obs_sum_kernel<<<(nq + 3) / 4, 128, 0, tvap::counted(s)>>>(G, nq, Q, w->coefA, sums);
+    obs_rho_kernel<<<nblk(nn, tb), tb, 0, tvap::counted(s)>>>(n, G, w->rhoL, w->coefA, rsum);
+    TVAP_CUDA(cudaGetLastError());
     // results
     std::vector<double2> hs(nq + 1);
     TVAP_CUDA(cudaMemcpyAsync(hs.data(), sums, sizeof(double2) * (nq + 1), cudaMemcpyDeviceToHost, s));
@@ -3393,7 +3575,6 @@ int project_observables_device(tvap_ctx* c, const tvap_proj_opts& o, int nobo, c
     return TVAP_OK;
   };
   rc = run();
-  release();
   if (rc == TVAP_OK) TVAP_CUDA(cudaStreamSynchronize(s));
   return rc;
 }
