@@ -404,7 +404,7 @@ def run_ours(args):
     # ozaki_tc_kernel; its largest use is H20: 5 complex products of n x n x n
     # per angle, formed as 3 launches (two of them stacked along K) of real
     # products [[Ar,-Ai],[Ai,Ar]] [Br;Bi] (2n x n x 2n per complex product) of
-    # digit planes, 36 digit pairs, bf16 MMAs with FP32 accumulation in tensor
+    # digit planes, 28 digit pairs, bf16 MMAs with FP32 accumulation in tensor
     # memory.  The h20_tc section times exactly those launches with CUDA
     # events on their stream; per-launch figures are the per-step totals
     # divided by the launch count (a flop-weighted average).
@@ -422,11 +422,11 @@ def run_ours(args):
     fp64_peak = measure_fp64_peak(torch)
     h20_launches = max(1, round(sections["h20_tc"][1] / sec_steps))
     tc_launch_ms = sections["h20_tc"][0] / sec_steps / h20_launches
-    h20_flops = 5 * 2.0 * (2 * n) * n * (2 * n) * 36 * G / h20_launches  # bf16 tensor flops per launch (unpadded)
+    h20_flops = 5 * 2.0 * (2 * n) * n * (2 * n) * 28 * G / h20_launches  # bf16 tensor flops per launch (unpadded)
     h20_tflops = h20_flops / (tc_launch_ms / 1000.0) / 1e12
     roofline = {
         "kernel": "ozaki_tc_kernel (tcgen05): the H20 complex products (5 x n^3 x G per step, 3 launches) as real "
-                  "products of bf16 digit planes, 36 digit pairs, per launch",
+                  "products of bf16 digit planes, 28 digit pairs, per launch",
         "bound": "tensor",
         "achieved": h20_tflops,
         "peak": bf16_peak,

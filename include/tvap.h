@@ -120,7 +120,7 @@ int tvap_kernel_launches(const tvap_ctx* ctx);
 int tvap_set_timing(tvap_ctx* ctx, int on);
 /* Arithmetic of the dense products: 0 = the FP64 pipe (DFMA);
  * 1 = FP64 emulated on the bf16 tensor cores by integer splitting (8
- * balanced 7-bit digits per FP64 value under one power-of-two scale per row
+ * balanced 7-bit or 7 balanced 8-bit digits per FP64 value under one power-of-two scale per row
  * or column, exact FP32 partial sums, integer recombination; error bound at
  * tvap_zgemm) with warp-level mma.sync; 2 (default) = the same splitting
  * with tcgen05 MMAs and tensor-memory accumulators for the batched products
@@ -316,8 +316,8 @@ int tvap_project_observables(tvap_ctx* ctx, const double* U0, const double* V0, 
 
 /* Launch shapes of the projection, chosen by measurement (no counterpart
  * in the reference).  tvap_autotune times `reps` projections of (U0, V0)
- * with opts for each candidate -- B' tile policy of the tcgen05 products (0:
- * the width that pads the output columns less, 1: 64 rows, 2: 48 rows) x the
+ * with opts for each candidate -- column policy of the tcgen05 products (0
+ * and 1: tiles of two halves of 32 columns, 2: of one half) x the
  * groups of angles in the Thouless solve (2 staggered on two streams, or 1)
  * x the cap on the tcgen05 CTAs beside the second group's panels (0: the
  * SMs the panels leave, 1: half the SMs, 2: none; 2 groups only) x the
@@ -388,9 +388,9 @@ int tvap_zskpfa_batched(tvap_ctx* ctx, int batch, int64_t n, const double* A, do
  * is emulated on the tensor cores: every row i of op(A) and
  * column j of op(B) gets one power-of-two scale 2^e (2^e <= its largest
  * entry), each entry is rounded to an integer multiple of 2^(e-53) (error
- * <= 2^-54 of the row's or column's largest entry) and written as 8 balanced
- * base-2^7 digits, and the digit pairs of total weight below the 8th are
- * dropped.  With a_i = max_k max(|Re op(A)_ik|, |Im op(A)_ik|) and b_j the
+ * <= 2^-54 of the row's or column's largest entry) and written as 7 balanced
+ * base-2^8 digits (8 of base 2^7 with mma.sync), and the digit pairs of total
+ * weight below the last one are dropped.  With a_i = max_k max(|Re op(A)_ik|, |Im op(A)_ik|) and b_j the
  * same over column j of op(B):
  *   real:    |C_ij - (op(A) op(B))_ij| <= 2^-49 K a_i b_j
  *   complex: |C_ij - (op(A) op(B))_ij| <= 2^-46 K a_i b_j

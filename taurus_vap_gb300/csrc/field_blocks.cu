@@ -156,7 +156,7 @@ __global__ void __launch_bounds__(oz::kThreads, 1)
 // tcgen05 form (GEMM mode 2): per block, C_b = W_b X_b with W_b in 128-row
 // tiles (planes tiled once per Hamiltonian) and X_b' = [Re X_b; Im X_b]^T
 // (B' rows: the real parts of the ncols_tot columns, then the imaginary
-// parts) sliced per call into 64-row tiles, on the persistent kernel of
+// parts) sliced per call into 32-row tiles, on the persistent kernel of
 // ozaki_tc.cuh with one k-step count per block.
 // ---------------------------------------------------------------------------
 
@@ -211,28 +211,28 @@ __global__ void __launch_bounds__(128)
     for (int kk = 0; kk < 8; ++kk) v[kk] = ent[kk] >= 0 ? X[(long long)ent[kk] * ldc + jj] : make_double2(0.0, 0.0);
 #pragma unroll
     for (int part = 0; part < 2; ++part) {
-      uint32_t w[kDigits][4];
+      uint32_t w[oztc::kDigits][4];
 #pragma unroll
       for (int kk = 0; kk < 8; kk += 2) {
-        int d0[kDigits], d1[kDigits];
-        oz::to_digits(oz::to_fixed(part ? v[kk].y : v[kk].x, e), d0);
-        oz::to_digits(oz::to_fixed(part ? v[kk + 1].y : v[kk + 1].x, e), d1);
+        int d0[oztc::kDigits], d1[oztc::kDigits];
+        oztc::to_digits(oz::to_fixed(part ? v[kk].y : v[kk].x, e), d0);
+        oztc::to_digits(oz::to_fixed(part ? v[kk + 1].y : v[kk + 1].x, e), d1);
 #pragma unroll
-        for (int s = 0; s < kDigits; ++s) w[s][kk >> 1] = oz::bf16x2_of_ints(d0[s], d1[s]);
+        for (int s = 0; s < oztc::kDigits; ++s) w[s][kk >> 1] = oz::bf16x2_of_ints(d0[s], d1[s]);
       }
       const int jr = part * ncols_tot + j;
-      const size_t tb = (size_t(q.kboff) * ntn + size_t(jr / oztc::kN) * q.nks + k0 / 16) * kDigits;
-      const int toff = oztc::tile_offset(jr % oztc::kN, k0 % 16);
+      const size_t tb = (size_t(q.kboff) * ntn + size_t(jr / oztc::kHalf) * q.nks + k0 / 16) * oztc::kDigits;
+      const int toff = oztc::tile_offset(jr % oztc::kHalf, k0 % 16);
 #pragma unroll
-      for (int s = 0; s < kDigits; ++s)
+      for (int s = 0; s < oztc::kDigits; ++s)
         *reinterpret_cast<uint4*>(xt + (tb + s) * oztc::kBTileElems + toff) =
             make_uint4(w[s][0], w[s][1], w[s][2], w[s][3]);
     }
   }
 }
 
-// One persistent CTA per SM over the (block, 128-row tile, 64-column tile)
-// tiles.  DELTA = false: Gamma and h = Gamma + H1; DELTA = true: Delta^LR
+// One persistent CTA per SM over the (block, 128-row tile, 2 x 32 columns)
+// tiles; ntn = the 32-column halves.  DELTA = false: Gamma and h = Gamma + H1; DELTA = true: Delta^LR
 // (columns < ncol) and Delta^RL, each written with its skew image.  Every
 // thread stores one real or imaginary part per column.
 template <bool DELTA>
@@ -245,29 +245,32 @@ __global__ void __launch_bounds__(oztc::kThreads, 1)
                     int* counter, int* flags) {
   extern __shared__ __align__(1024) unsigned char fsm[];
   __shared__ oztc::Ctl ctl;
-  const int ntiles = nbm * ntn;
-  auto tile_ptrs = [&](int tile, const unsigned char*& A, const unsigned char*& B) {
-    const int2 m = bm[tile / ntn];
-    const int nt = tile % ntn;
+  const int nct = (ntn + 1) / 2, ntiles = nbm * nct;
+  auto tile_ptrs = [&](int tile, const unsigned char*& A, const unsigned char*& B0, const unsigned char*& B1) {
+    const int2 m = bm[tile / nct];
+    const int nt = 2 * (tile % nct);
     const FieldTcBlock q = tcb[m.x];
     A = reinterpret_cast<const unsigned char*>(wt) +
-        (size_t(q.woff) + size_t(m.y) * q.nks * kDigits * oztc::kATileElems) * sizeof(__nv_bfloat16);
-    B = reinterpret_cast<const unsigned char*>(xt) + (size_t(q.kboff) * ntn + size_t(nt) * q.nks) * size_t(oztc::kBBytes);
+        (size_t(q.woff) + size_t(m.y) * q.nks * oztc::kDigits * oztc::kATileElems) * sizeof(__nv_bfloat16);
+    B0 = reinterpret_cast<const unsigned char*>(xt) +
+         (size_t(q.kboff) * ntn + size_t(nt) * q.nks) * size_t(oztc::kBBytes);
+    B1 = B0 + size_t(q.nks) * oztc::kBBytes;
   };
-  auto nks_of = [&](int tile) { return tcb[bm[tile / ntn].x].nks; };
+  auto nks_of = [&](int tile) { return tcb[bm[tile / nct].x].nks; };
+  auto halves_of = [=](int tile) { return min(2, ntn - 2 * (tile % nct)); };
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  auto store = [&](int tile, const oztc::Acc& acc) {
-    const int2 m = bm[tile / ntn];
-    const int nt = tile % ntn;
+  auto store = [&](int tile, int half, const oztc::Acc& acc) {
+    const int2 m = bm[tile / nct];
+    const int nt = 2 * (tile % nct) + half;
     const FieldBlockDesc d = blocks[m.x];
     const int i = m.y * oztc::kM + 32 * (warp & 3) + lane;
     if (i >= d.r_pad) return;
     const int rr = d.row_base + i;
     const int p = rowperm[rr];
     if (p < 0) return;
-    const int eai = ea[rr] - 57;
+    const int eai = ea[rr] - oztc::kExpShift;
     const int pt = p / n + (p % n) * n;
-    const int col0 = nt * oztc::kN + 16 * (warp >> 2);
+    const int col0 = nt * oztc::kHalf + 16 * ((warp >> 2) & 1);
     double h1[2] = {0.0, 0.0};
     if (!DELTA) {
       const double2 hv = H1[p];
@@ -294,7 +297,7 @@ __global__ void __launch_bounds__(oztc::kThreads, 1)
       }
     }
   };
-  if (!oztc::run_tiles<oztc::kN>(counter, ntiles, nks_of, fsm, ctl, tile_ptrs, store) && threadIdx.x == 0 && flags)
+  if (!oztc::run_tiles(counter, ntiles, nks_of, halves_of, fsm, ctl, tile_ptrs, store) && threadIdx.x == 0 && flags)
     atomicOr(flags, DEV_TC_TIMEOUT);
 }
 
@@ -401,7 +404,7 @@ int build_one(int n, bool delta, const std::vector<int>& rowptr, const std::vect
     q.kboff = kboff;
     q.pad = 0;
     q.woff = woff;
-    woff += (long long)q.mtiles * q.nks * kDigits * oztc::kATileElems;
+    woff += (long long)q.mtiles * q.nks * oztc::kDigits * oztc::kATileElems;
     kboff += q.nks;
   }
   std::vector<uint16_t> wt(size_t(std::max<long long>(woff, 1)), 0);
@@ -434,13 +437,14 @@ int build_one(int n, bool delta, const std::vector<int>& rowptr, const std::vect
       for (int k = 0; k < d.kb_pad; ++k) {
         int dg[kDigits];
         oz::to_digits(oz::to_fixed(wr[k], emax), dg);
-        for (int s = 0; s < kDigits; ++s) {
-          const uint16_t bits = oz::bf16_bits_of_int(dg[s]);
-          wd[size_t(d.aoff) + (size_t(s) * d.r_pad + i) * d.kb_pad + k] = bits;
-          if (mt < q.mtiles)
-            wt[size_t(q.woff) + ((size_t(mt) * q.nks + k / 16) * kDigits + s) * oztc::kATileElems +
-               oztc::tile_offset(ri, k % 16)] = bits;
-        }
+        for (int s = 0; s < kDigits; ++s)
+          wd[size_t(d.aoff) + (size_t(s) * d.r_pad + i) * d.kb_pad + k] = oz::bf16_bits_of_int(dg[s]);
+        if (mt >= q.mtiles) continue;
+        int dt[oztc::kDigits];
+        oztc::to_digits(oz::to_fixed(wr[k], emax), dt);
+        for (int s = 0; s < oztc::kDigits; ++s)
+          wt[size_t(q.woff) + ((size_t(mt) * q.nks + k / 16) * oztc::kDigits + s) * oztc::kATileElems +
+             oztc::tile_offset(ri, k % 16)] = oz::bf16_bits_of_int(dt[s]);
       }
     }
   }
@@ -470,7 +474,10 @@ int build_one(int n, bool delta, const std::vector<int>& rowptr, const std::vect
     TVAP_CUDA(cudaMemcpy(f->tc_bm, tc_bm.data(), sizeof(int2) * tc_bm.size(), cudaMemcpyHostToDevice));
   if (!tc_chunks.empty())
     TVAP_CUDA(cudaMemcpy(f->tc_chunks, tc_chunks.data(), sizeof(int2) * tc_chunks.size(), cudaMemcpyHostToDevice));
-  f->tc_nbm = int(tc_bm.size());
+  // (a block longer than the accumulators allow: the mma.sync form)
+  bool fits = true;
+  for (int b = 0; b < nb; ++b) fits = fits && tcb[b].nks <= oztc::kMaxKs;
+  f->tc_nbm = fits ? int(tc_bm.size()) : 0;
   f->tc_ksteps = kboff;
   f->tc_nchunks = int(tc_chunks.size());
   f->tc_empty_base = desc[nb].row_base;
@@ -497,12 +504,12 @@ int apply_one_tc(tvap_ctx* c, const FieldDense& f, int ncol, int ldc, const doub
                  double2* out0, double2* out1, cudaStream_t s) {
   const int n = c->n, nent = n * n;
   const int ncols_tot = DELTA ? 2 * ncol : ncol;
-  const int ntn = (2 * ncols_tot + oztc::kN - 1) / oztc::kN;
+  const int ntn = (2 * ncols_tot + oztc::kHalf - 1) / oztc::kHalf;
   const int npad = (ncols_tot + 31) / 32 * 32;
   __nv_bfloat16* xt = nullptr;
   int* eb = nullptr;
   int rc;
-  const size_t xt_elems = size_t(f.tc_ksteps) * ntn * kDigits * oztc::kBTileElems;
+  const size_t xt_elems = size_t(f.tc_ksteps) * ntn * oztc::kDigits * oztc::kBTileElems;
   if ((rc = oz_scratch(s, sizeof(__nv_bfloat16) * xt_elems + sizeof(int) * 64, size_t(npad), &xt, &eb))) return rc;
   // the tile counter sits after the planes (256-byte aligned: the planes are multiples of 2 KB)
   int* counter = reinterpret_cast<int*>(xt + xt_elems);
@@ -513,7 +520,7 @@ int apply_one_tc(tvap_ctx* c, const FieldDense& f, int ncol, int ldc, const doub
       n, ncol, ncols_tot, ntn, ldc, X0, X1, f.colperm, f.blocks, f.tcb, f.tc_chunks, f.tc_nchunks,
       f.rowperm + f.tc_empty_base, f.tc_nempty, eb, xt, c->d_H1, out0, out1);
   if ((rc = smem_opt_in((const void*)field_tc_kernel<DELTA>, oztc::kSmemBytes))) return rc;
-  const int grid = std::min(f.tc_nbm * ntn, device_sms());
+  const int grid = std::min(f.tc_nbm * ((ntn + 1) / 2), device_sms());
   field_tc_kernel<DELTA><<<grid, oztc::kThreads, oztc::kSmemBytes, tvap::counted(s)>>>(
       n, ncol, ncols_tot, ntn, ldc, f.blocks, f.tcb, f.tc_bm, f.tc_nbm, static_cast<const __nv_bfloat16*>(f.wt), xt,
       f.ea, f.rowperm, eb, c->d_H1, out0, out1, counter, g_dev_flags);

@@ -158,27 +158,32 @@ int launch_ozaki_mma(int M, int N, int mpad, int npad, int kpad, const __nv_bflo
 
 // Real operand X' of a product, built from a strided batched source operand X
 // (element (r, k) of batch b at p[r sr + k sk + b bs]; r a row of op(A) or a
-// column of op(B), k the contraction index).  Forms:
+// column of op(B), k the contraction index).  Forms (rows of a complex source
+// come as adjacent pairs, so that the outputs of neighbouring TMEM lanes are
+// neighbours in a complex result):
 //   0  real:                        X'(r, k) = X(r, k)                      (rows x K)
-//   1  complex, planes stacked:     X' = [Re X; Im X]                       (2 rows x K)
-//   2  complex, real representation X' = [[Re X, -Im X], [Im X, Re X]]      (2 rows x 2 kp)
+//   1  complex, parts interleaved:  X'(2r, k) = Re X, X'(2r+1, k) = Im X    (2 rows x K)
+//   2  complex, real representation X'(2r, .) = [Re X, -Im X],
+//                                   X'(2r+1, .) = [Im X, Re X]              (2 rows x 2 kp)
 //   3  complex, planes side by side X' = [Re X, Im X]                       (rows x 2 kp)
-//   4  complex, rows interleaved:   X'(2r, k) = Re X(r, k), X'(2r+1, k) = Im X(r, k)
-//                                                                           (2 rows x K)
-// so that A' B'^T of (2, 3) holds [Re C; Im C] of a complex x complex
-// product, of (1, 0) [Re C; Im C] and of (0, 1) [Re C, Im C]; of (4, 4) the
-// four real products Re/Im A x Re/Im B in 2 x 2 blocks, which the epilogue
+//   4  as 1, one exponent for both parts of a row
+// so that A' B'^T of (2, 3) holds the parts of a complex x complex product as
+// row pairs, of (1, 0) as row pairs and of (0, 1) as column pairs; of (4, 4)
+// the four real products Re/Im A x Re/Im B in 2 x 2 blocks, which the epilogue
 // combines.  In forms 2 and 3 each column block is padded with zeros from K
 // to kp (a multiple of 16).  Forms 2, 3 and 4 give the real and imaginary part
 // of a row one exponent (so that the digits of form 4 are those of forms 2
 // and 3); forms 0 and 1 give each part its own.
-// nstack > 1 stacks the rows of nstack batch entries (X' row b xrows + r).
+// nstack > 1 stacks the rows of nstack batch entries, the batches one after
+// the other or, with bfast, the entries of all batches for each row (a result
+// whose batch index is the innermost one is then stored contiguously).
 struct TcSrc {
   const void* p;
   long long sr, sk, bs;
   int rows, K, form;
   bool conj;
   int xrows, xk, nstack, kp;
+  bool bfast;
   // k >= K1 comes from the second source (k - K1), scaled by scale2
   const void* p2;
   long long sr2, sk2, bs2;
@@ -190,7 +195,7 @@ struct TcSrc {
 // source rows of one slot: the rows are gathered into shared memory
 // (independent loads, consecutive threads on the source's contiguous index),
 // one warp per row takes the exponents, then every thread converts 8
-// consecutive k of one part (real or imaginary) of one row to 8 digits and
+// consecutive k of one part (real or imaginary) of one row to 7 digits and
 // stores one 16-byte core-matrix row per digit at each place of X' that
 // holds them (twice in form 2: the imaginary block negated by its sign bits;
 // once in form 4, whose left operand is half the size of form 2's).
@@ -210,10 +215,19 @@ __global__ void __launch_bounds__(kSliceThreads) slice_tc_kernel(TcSrc x, int ti
   const int sq0 = blockIdx.x * 8;
   const int slot = blockIdx.y;
   const int nsrc = x.nstack * x.rows;
+  const int mult = (form == 1 || form == 2 || form == 4) ? 2 : 1;  // rows of X' per source row
   auto src_row = [&](int row, int& b, int& i) {
     const int sq = sq0 + row;
-    b = x.nstack > 1 ? sq / x.rows : slot;
-    i = x.nstack > 1 ? sq - b * x.rows : sq;
+    if (x.nstack == 1) {
+      b = slot;
+      i = sq;
+    } else if (x.bfast) {
+      i = sq / x.nstack;
+      b = sq - i * x.nstack;
+    } else {
+      b = sq / x.rows;
+      i = sq - b * x.rows;
+    }
   };
   const bool k_fast = (x.sk == 1);
 #pragma unroll 4
@@ -266,62 +280,50 @@ __global__ void __launch_bounds__(kSliceThreads) slice_tc_kernel(TcSrc x, int ti
       e_s[w][0] = er;
       e_s[w][1] = ei;
       if (sq0 + w < nsrc) {
-        int b, i;
-        src_row(w, b, i);
-        const size_t qtop = size_t(x.nstack > 1 ? b * x.xrows : 0) + (form == 4 ? 2 * i : i);
-        ex[size_t(slot) * rows_pad + qtop] = er;
-        if (form == 1 || form == 2) ex[size_t(slot) * rows_pad + qtop + x.rows] = ei;
-        if (form == 4) ex[size_t(slot) * rows_pad + qtop + 1] = ei;
+        int* e = ex + size_t(slot) * rows_pad + size_t(sq0 + w) * mult;
+        e[0] = er;
+        if (mult == 2) e[1] = ei;
       }
     }
   }
   __syncthreads();
-  // work items: (row, chunk of 8 k, part), rows fastest so that a half-warp
-  // writes whole 256-byte core-matrix row groups
+  // work items: (part, row, chunk of 8 k), parts and rows fastest so that
+  // neighbouring threads write the 16-byte pieces of whole core matrices
   const int nchunk = (form == 2 || form == 3) ? x.kp / 8 : nks * 2;
-  const int nparts = cplx ? 2 : 1;
+  const int pbits = cplx ? 1 : 0;
   const int tiles = rows_pad / tile_rows;
   const size_t tile_elems = size_t(tile_rows) * 16;
-  for (int item = t; item < 8 * nchunk * nparts; item += kSliceThreads) {
-    const int row = item & 7;
-    const int c = (item >> 3) % nchunk, part = (item >> 3) / nchunk;
+  for (int item = t; item < (8 * nchunk << pbits); item += kSliceThreads) {
+    const int part = item & pbits, row = (item >> pbits) & 7, c = item >> (pbits + 3);
     if (sq0 + row >= nsrc) continue;
-    int b, i;
-    src_row(row, b, i);
-    const int qtop = (x.nstack > 1 ? b * x.xrows : 0) + (form == 4 ? 2 * i : i);
+    const int qtop = (sq0 + row) * mult;
     const int emax = e_s[row][part];
     const int k0 = 8 * c;
-    uint32_t w[kDigits][4];
+    uint32_t w[oztc::kDigits][4];
 #pragma unroll
     for (int j = 0; j < 8; j += 2) {
-      int d0[kDigits], d1[kDigits];
+      int d0[oztc::kDigits], d1[oztc::kDigits];
       const double2 v0 = (k0 + j < K) ? xs[row * ldk + k0 + j] : make_double2(0.0, 0.0);
       const double2 v1 = (k0 + j + 1 < K) ? xs[row * ldk + k0 + j + 1] : make_double2(0.0, 0.0);
-      oz::to_digits(oz::to_fixed(part ? v0.y : v0.x, emax), d0);
-      oz::to_digits(oz::to_fixed(part ? v1.y : v1.x, emax), d1);
+      oztc::to_digits(oz::to_fixed(part ? v0.y : v0.x, emax), d0);
+      oztc::to_digits(oz::to_fixed(part ? v1.y : v1.x, emax), d1);
 #pragma unroll
-      for (int s = 0; s < kDigits; ++s) w[s][j >> 1] = oz::bf16x2_of_ints(d0[s], d1[s]);
+      for (int s = 0; s < oztc::kDigits; ++s) w[s][j >> 1] = oz::bf16x2_of_ints(d0[s], d1[s]);
     }
     auto put = [&](int q, int kq, uint32_t flip) {
       const size_t tb = (size_t(slot) * tiles + q / tile_rows) * nks + (kq >> 4);
       const int toff = oztc::tile_offset(q % tile_rows, kq);
 #pragma unroll
-      for (int s = 0; s < kDigits; ++s) {
-        __nv_bfloat16* dst = out + (tb * kDigits + s) * tile_elems + toff;
+      for (int s = 0; s < oztc::kDigits; ++s) {
+        __nv_bfloat16* dst = out + (tb * oztc::kDigits + s) * tile_elems + toff;
         *reinterpret_cast<uint4*>(dst) = make_uint4(w[s][0] ^ flip, w[s][1] ^ flip, w[s][2] ^ flip, w[s][3] ^ flip);
       }
     };
     switch (form) {
       case 0: put(qtop, k0, 0u); break;
-      case 1: put(part ? qtop + x.rows : qtop, k0, 0u); break;
       case 2:
-        if (part == 0) {
-          put(qtop, k0, 0u);
-          put(qtop + x.rows, x.kp + k0, 0u);
-        } else {
-          put(qtop + x.rows, k0, 0u);
-          put(qtop, x.kp + k0, 0x80008000u);
-        }
+        put(qtop + part, k0, 0u);
+        put(qtop + 1 - part, x.kp + k0, part ? 0x80008000u : 0u);
         break;
       case 3: put(qtop, part ? x.kp + k0 : k0, 0u); break;
       default: put(qtop + part, k0, 0u); break;
@@ -329,93 +331,92 @@ __global__ void __launch_bounds__(kSliceThreads) slice_tc_kernel(TcSrc x, int ti
   }
 }
 
-// Output mapping of the tensor-memory product: row q of A' (slot z) and row
-// col of B' hold component comp = (r >= a_split) + (col >= b_split) of
-// C(i, j) of batch entry b; alpha and beta are real.  In the paired form
-// (both operands sliced in form 4) rows 2i, 2i + 1 of A' and 2j, 2j + 1 of B'
-// are the real and imaginary parts of row i of op(A) and column j of op(B).
+// Output mapping of the tensor-memory product: row q of A' (slot z) is part q %
+// a_mult of source row q / a_mult, column col of B' part col % b_mult of j =
+// col / b_mult; at most one of the two is a pair, whose members are the real
+// and imaginary parts of C(i, j) of batch entry b; alpha and beta are real.
+// In the paired form (both operands sliced in form 4) both are.
 struct TcOut {
   void* C;
   long long crs, ccs, cbs;
   bool c_real;
   double alpha, beta;
-  int a_rows, a_split, b_rows, b_split, nstack;
+  int a_rows, a_mult, b_rows, b_mult, nstack;  // a_rows: source rows per batch entry, b_rows: columns of B'
+  bool bfast;
 };
 
-// Persistent CTAs over the (128 x 64 tile of A' B'^T, slot) tiles, claimed in
-// order from *counter; tile numbers run over the N tiles fastest, then the M
-// tiles, then the slots, so that the CTAs working at one time share their A
-// and B tiles through L2.  PAIRS: the paired form, whose 2 x 2 blocks
-// P(2i .. 2i+1, 2j .. 2j+1) give Re C(i, j) = P(2i, 2j) - P(2i+1, 2j+1) and
-// Im C(i, j) = P(2i+1, 2j) + P(2i, 2j+1): the two rows of a block are adjacent
-// TMEM lanes (one shuffle per column pair), its two columns adjacent
+// Persistent CTAs over the (128 rows x `halves` x 32 columns of A' B'^T, slot)
+// tiles, claimed in order from *counter; tile numbers run over the columns
+// fastest, then the M tiles, then the slots, so that the CTAs working at one
+// time share their A and B tiles through L2.  PAIRS: the paired form, whose 2
+// x 2 blocks P(2i .. 2i+1, 2j .. 2j+1) give Re C(i, j) = P(2i, 2j) - P(2i+1,
+// 2j+1) and Im C(i, j) = P(2i+1, 2j) + P(2i, 2j+1): the two rows of a block are
+// adjacent TMEM lanes (one shuffle per column pair), its two columns adjacent
 // accumulator columns of one thread.  The four products of a block share one
 // exponent (rows and columns: one per real/imaginary pair), so the
 // combination is exact on the integer accumulators and the result is, bit
 // for bit, that of the real representation [[Re, -Im], [Im, Re]] x [Re, Im].
-template <bool UNIT, int BN, bool PAIRS>
+template <bool UNIT, bool PAIRS>
 __global__ void __launch_bounds__(oztc::kThreads, 1)
     ozaki_tc_kernel(const __nv_bfloat16* __restrict__ As, const int* __restrict__ ea, int a_rows_pad,
                     const __nv_bfloat16* __restrict__ Bs, const int* __restrict__ eb, int b_rows_pad, int b_shared,
-                    int nslots, int nks, TcOut o, int* counter, int* flags) {
+                    int nslots, int nks, int halves, TcOut o, int* counter, int* flags) {
   extern __shared__ __align__(1024) unsigned char tsm[];
   __shared__ oztc::Ctl ctl;
-  const int a_tiles = a_rows_pad / oztc::kM, b_tiles = b_rows_pad / BN;
+  const int a_tiles = a_rows_pad / oztc::kM, b_halves = b_rows_pad / oztc::kHalf;
+  const int b_tiles = (b_halves + halves - 1) / halves;
   const int ntiles = a_tiles * b_tiles * nslots;
-  auto tile_ptrs = [&](int tile, const unsigned char*& A, const unsigned char*& B) {
+  auto tile_ptrs = [&](int tile, const unsigned char*& A, const unsigned char*& B0, const unsigned char*& B1) {
     const int nt = tile % b_tiles, rest = tile / b_tiles;
     const int mt = rest % a_tiles, z = rest / a_tiles;
     const int bz = b_shared ? 0 : z;
     A = reinterpret_cast<const unsigned char*>(As) + (size_t(z) * a_tiles + mt) * nks * size_t(oztc::kABytes);
-    B = reinterpret_cast<const unsigned char*>(Bs) + (size_t(bz) * b_tiles + nt) * nks * size_t(oztc::b_bytes(BN));
+    B0 = reinterpret_cast<const unsigned char*>(Bs) +
+         (size_t(bz) * b_halves + nt * halves) * nks * size_t(oztc::kBBytes);
+    B1 = B0 + size_t(nks) * oztc::kBBytes;
   };
+  auto halves_of = [=](int tile) { return min(halves, b_halves - (tile % b_tiles) * halves); };
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // The stores of a tile overlap the MMAs of the next one: exponents, values
   // and (with beta) the old outputs are fetched with independent loads, all
   // issued before the first store (C is not known not to alias them).
-  auto store = [&](int tile, const oztc::Acc& acc) {
+  auto store = [&](int tile, int half, const oztc::Acc& acc) {
     const int nt = tile % b_tiles, rest = tile / b_tiles;
     const int mt = rest % a_tiles, z = rest / a_tiles;
     const int bz = b_shared ? 0 : z;
     const int q = mt * oztc::kM + 32 * (warp & 3) + lane;
-    if constexpr (BN < 64) {
-      if (16 * (warp >> 2) >= BN) return;  // these warps' columns belong to the next tile
-    }
-    // a row pair lies within the rows of A' or beyond them (a_rows is even):
-    // the paired form returns after its shuffles, which the whole warp takes
-    const bool row_ok = q < o.nstack * o.a_rows;
+    const int col0 = (nt * halves + half) * oztc::kHalf + 16 * ((warp >> 2) & 1);
+    if (col0 >= o.b_rows) return;  // padding (uniform over the warp)
+    // a row pair lies within the rows of A' or beyond them: the paired form
+    // returns after its shuffles, which the whole warp takes
+    const bool row_ok = q < o.nstack * o.a_rows * o.a_mult;
     if (!PAIRS && !row_ok) return;
-    const int b = o.nstack > 1 ? q / o.a_rows : z;
-    int i = o.nstack > 1 ? q - b * o.a_rows : q;
-    int comp_a = 0;
-    if (PAIRS) {
-      comp_a = i & 1;
-      i >>= 1;
-    } else if (i >= o.a_split) {
-      i -= o.a_split;
-      comp_a = 1;
-    }
-    const int eai = (row_ok ? ea[size_t(z) * a_rows_pad + q] : 0) - 57;
-    double* __restrict__ C = static_cast<double*>(o.C);
-    const int cw = o.c_real ? 1 : 2;  // doubles per element
-    const int col0 = nt * BN + 16 * (warp >> 2);
-    const int* __restrict__ ebz = eb + size_t(bz) * b_rows_pad;
-    // element index of column c, or -1 (padding, or the imaginary part of a
-    // real output)
-    auto idx_of = [&](int c) -> long long {
-      const int col = col0 + c;
-      int j = col, comp = comp_a;
-      if (j >= o.b_split) {
-        j -= o.b_split;
-        comp += 1;
+    const int sq = o.a_mult == 2 ? q >> 1 : q, comp_a = o.a_mult == 2 ? q & 1 : 0;
+    int b = z, i = sq;
+    if (o.nstack > 1) {
+      if (o.bfast) {
+        i = sq / o.nstack;
+        b = sq - i * o.nstack;
+      } else {
+        b = sq / o.a_rows;
+        i = sq - b * o.a_rows;
       }
-      if (col >= o.b_rows || (comp > 0 && o.c_real)) return -1;
-      return (i * o.crs + j * o.ccs + b * o.cbs) * cw + comp;
-    };
+    }
+    const int eai = (row_ok ? ea[size_t(z) * a_rows_pad + q] : 0) - oztc::kExpShift;
+    const int cw = o.c_real ? 1 : 2;  // doubles per element
+    const int* __restrict__ ebz = eb + size_t(bz) * b_rows_pad + col0;
+    const int ncol = min(16, o.b_rows - col0);
+    double* __restrict__ C = static_cast<double*>(o.C) + (i * o.crs + b * o.cbs) * cw + comp_a;
+    const long long step = o.ccs * cw;  // from one j to the next
     // UNIT: alpha = +-1 (every product of the path), a sign of the integer
     // conversion; otherwise one product more (a separate instantiation, so
     // that no FP64 multiply is predicated into the common case)
     const bool neg = o.alpha < 0.0;
+    auto number = [&](long long h, long long l, int e) {
+      double x;
+      if (oztc::scaled(h, l, eai + e, UNIT && neg, x)) return UNIT ? x : x * o.alpha;
+      return fma(double(h), 0x1p28, double(l)) * (o.alpha * oz::pow2(eai + e));
+    };
     if constexpr (PAIRS) {
       // even lane (real row): P(2i, 2j) - P(2i+1, 2j+1); odd lane (imaginary
       // row): P(2i+1, 2j) + P(2i, 2j+1).  Both take the partner's odd column.
@@ -428,64 +429,49 @@ __global__ void __launch_bounds__(oztc::kThreads, 1)
         ls[c] = comp_a ? acc.l[2 * c] + tl : acc.l[2 * c] - tl;
       }
       if (!row_ok || (comp_a && o.c_real)) return;
-      const int j0 = col0 >> 1;
+      C += (col0 >> 1) * step;
       double w[8];
-      long long k[8];
 #pragma unroll
-      for (int c = 0; c < 8; ++c) {
-        const bool in = col0 + 2 * c < o.b_rows;
-        const int e = in ? ebz[col0 + 2 * c] : 0;
-        double x;
-        if (oztc::scaled(hs[c], ls[c], eai + e, UNIT && neg, x))
-          w[c] = UNIT ? x : x * o.alpha;
-        else
-          w[c] = fma(double(hs[c]), 0x1p28, double(ls[c])) * (o.alpha * oz::pow2(eai + e));
-        k[c] = in ? (i * o.crs + (j0 + c) * o.ccs + b * o.cbs) * cw + comp_a : -1;
-      }
+      for (int c = 0; c < 8; ++c) w[c] = number(hs[c], ls[c], 2 * c < ncol ? ebz[2 * c] : 0);
       if (o.beta != 0.0) {
         double old[8];
 #pragma unroll
-        for (int c = 0; c < 8; ++c) old[c] = k[c] >= 0 ? C[k[c]] : 0.0;
+        for (int c = 0; c < 8; ++c) old[c] = 2 * c < ncol ? C[c * step] : 0.0;
 #pragma unroll
         for (int c = 0; c < 8; ++c) w[c] = fma(o.beta, old[c], w[c]);
       }
 #pragma unroll
       for (int c = 0; c < 8; ++c)
-        if (k[c] >= 0) C[k[c]] = w[c];
+        if (2 * c < ncol) C[c * step] = w[c];
       return;
     }
-    double v[16];
-#pragma unroll
-    for (int c = 0; c < 16; ++c) {
-      const int e = (col0 + c < o.b_rows) ? ebz[col0 + c] : 0;
-      double x;
-      if (oztc::scaled(acc.h[c], acc.l[c], eai + e, UNIT && neg, x))
-        v[c] = UNIT ? x : x * o.alpha;
-      else
-        v[c] = oztc::value(acc, c) * (o.alpha * oz::pow2(eai + e));
-    }
+    if (comp_a && o.c_real) return;
+    // column pairs (b_mult = 2): j = col / 2, the parts adjacent doubles (of a
+    // real result only the first is kept)
+    const bool pairs = o.b_mult == 2, keep_odd = !pairs || !o.c_real;
+    C += pairs ? (col0 >> 1) * step : col0 * step;
     // two groups of 8: the loads of a group are in flight together
 #pragma unroll
     for (int c0 = 0; c0 < 16; c0 += 8) {
+      double v[8];
+#pragma unroll
+      for (int c = 0; c < 8; ++c) v[c] = number(acc.h[c0 + c], acc.l[c0 + c], c0 + c < ncol ? ebz[c0 + c] : 0);
+      auto at = [&](int c) -> double& { return pairs ? C[((c0 + c) >> 1) * step + (c & 1)] : C[(c0 + c) * step]; };
+      auto in = [&](int c) { return c0 + c < ncol && ((c & 1) == 0 || keep_odd); };
       if (o.beta != 0.0) {
         double old[8];
 #pragma unroll
-        for (int c = 0; c < 8; ++c) {
-          const long long k = idx_of(c0 + c);
-          old[c] = k >= 0 ? C[k] : 0.0;
-        }
+        for (int c = 0; c < 8; ++c) old[c] = in(c) ? at(c) : 0.0;
 #pragma unroll
-        for (int c = 0; c < 8; ++c) v[c0 + c] = fma(o.beta, old[c], v[c0 + c]);
+        for (int c = 0; c < 8; ++c) v[c] = fma(o.beta, old[c], v[c]);
       }
 #pragma unroll
-      for (int c = 0; c < 8; ++c) {
-        const long long k = idx_of(c0 + c);
-        if (k >= 0) C[k] = v[c0 + c];
-      }
+      for (int c = 0; c < 8; ++c)
+        if (in(c)) at(c) = v[c];
     }
   };
   auto nks_of = [nks](int) { return nks; };
-  if (!oztc::run_tiles<BN>(counter, ntiles, nks_of, tsm, ctl, tile_ptrs, store) && threadIdx.x == 0 && flags)
+  if (!oztc::run_tiles(counter, ntiles, nks_of, halves_of, tsm, ctl, tile_ptrs, store) && threadIdx.x == 0 && flags)
     atomicOr(flags, DEV_TC_TIMEOUT);
 }
 
@@ -496,13 +482,13 @@ struct LeftSlice {
   const void* p = nullptr;
   const void* p2 = nullptr;
   long long sr = 0, sk = 0, bs = 0, sr2 = 0, sk2 = 0, bs2 = 0;
-  int rows = 0, K = 0, K1 = 0, form = 0, conj = 0, xrows = 0, xk = 0, kp = 0, nstack = 0, slots = 0, rows_pad = 0,
-      nks = 0;
+  int rows = 0, K = 0, K1 = 0, form = 0, conj = 0, xrows = 0, xk = 0, kp = 0, nstack = 0, bfast = 0, slots = 0,
+      rows_pad = 0, nks = 0;
   double scale2 = 0.0;
   bool operator==(const LeftSlice& o) const {
     return valid && o.valid && p == o.p && p2 == o.p2 && sr == o.sr && sk == o.sk && bs == o.bs && sr2 == o.sr2 &&
            sk2 == o.sk2 && bs2 == o.bs2 && rows == o.rows && K == o.K && K1 == o.K1 && form == o.form &&
-           conj == o.conj && xrows == o.xrows && xk == o.xk && kp == o.kp && nstack == o.nstack && slots == o.slots &&
+           conj == o.conj && xrows == o.xrows && xk == o.xk && kp == o.kp && nstack == o.nstack && bfast == o.bfast && slots == o.slots &&
            rows_pad == o.rows_pad && nks == o.nks && scale2 == o.scale2;
   }
 };
@@ -627,12 +613,12 @@ int gemm_tc(const GemmArgs& g, cudaStream_t s) {
   const int K = g.K + (g.K2 > 0 ? g.K2 : 0), kp = (K + 15) / 16 * 16;
   const int K1 = g.K2 > 0 ? g.K : K;
   const bool scale_left = a_sh;  // after the swap the B side is on the left
-  TcSrc xa{L.p, L.sr, L.sk, L.bs, L.rows, K, 0, L.conj, L.rows, K, 1, K, L.p2, L.sr2, L.sk2, L.bs2, K1,
+  TcSrc xa{L.p, L.sr, L.sk, L.bs, L.rows, K, 0, L.conj, L.rows, K, 1, K, false, L.p2, L.sr2, L.sk2, L.bs2, K1,
            scale_left ? g.s2 : 1.0};
-  TcSrc xb{R.p, R.sr, R.sk, R.bs, R.rows, K, 0, R.conj, R.rows, K, 1, K, R.p2, R.sr2, R.sk2, R.bs2, K1,
+  TcSrc xb{R.p, R.sr, R.sk, R.bs, R.rows, K, 0, R.conj, R.rows, K, 1, K, false, R.p2, R.sr2, R.sk2, R.bs2, K1,
            scale_left ? 1.0 : g.s2};
   TcOut o{};
-  o.a_split = o.b_split = INT_MAX;
+  o.a_mult = o.b_mult = 1;
   const bool stack = g.batch > 1 && (a_sh || b_sh);
   // complex x complex: the paired form (rows interleaved on both sides, the
   // 2 x 2 blocks combined by the epilogue; half the left operand's digit
@@ -642,43 +628,45 @@ int gemm_tc(const GemmArgs& g, cudaStream_t s) {
   const bool pairs = !L.real && !R.real && !stack && g_tc_pairs_min_k > 0 && K >= g_tc_pairs_min_k;
   if (pairs) {
     xa.form = xb.form = 4;
-    xa.xrows = 2 * L.rows;
-    xb.xrows = 2 * R.rows;
+    o.a_mult = o.b_mult = 2;
   } else if (!L.real && !R.real) {
     xa.form = 2;
-    xa.xrows = 2 * L.rows;
     xa.xk = 2 * kp;
     xa.kp = kp;
     xb.form = 3;
     xb.xk = 2 * kp;
     xb.kp = kp;
-    o.a_split = L.rows;
+    o.a_mult = 2;
   } else if (!L.real) {
     xa.form = 1;
-    xa.xrows = 2 * L.rows;
-    o.a_split = L.rows;
+    o.a_mult = 2;
   } else if (!R.real) {
     xb.form = 1;
-    xb.xrows = 2 * R.rows;
-    o.b_split = R.rows;
+    o.b_mult = 2;
   }
+  xa.xrows = o.a_mult * L.rows;
+  xb.xrows = o.b_mult * R.rows;
   xa.nstack = stack ? g.batch : 1;
+  // a result whose batch index is the contiguous one (the angle-innermost
+  // densities): the rows of all batch entries side by side, so that a warp
+  // stores 512 contiguous bytes instead of 32 pieces of 8
+  xa.bfast = stack && g.cbs == 1 && crs != 1;
   const int a_slots = stack ? 1 : g.batch, b_slots = stack ? 1 : g.batch;
   const int a_rows_pad = (xa.nstack * xa.xrows + oztc::kM - 1) / oztc::kM * oztc::kM;
-  // B' tiles of 48 or 64 rows, whichever pads the output columns less (140
-  // columns: 144 instead of 192)
-  const int pad48 = (xb.xrows + 47) / 48 * 48, pad64 = (xb.xrows + 63) / 64 * 64;
-  const int bn = g_tc_bn_policy == 1 ? 64 : g_tc_bn_policy == 2 ? 48 : (pad48 < pad64 ? 48 : 64);
-  const int b_rows_pad = bn == 48 ? pad48 : pad64;
+  const int b_halves = (xb.xrows + oztc::kHalf - 1) / oztc::kHalf, b_rows_pad = b_halves * oztc::kHalf;
+  // CTA tiles of two halves (the A tile read once for 64 columns, one half's
+  // folds beside the other's MMAs); one half each if the tuning says so
+  const int halves = g_tc_bn_policy == 2 ? 1 : 2;
   const int nks = (xa.xk + 15) / 16;
+  if (nks > oztc::kMaxKs) return TVAP_ERR_ARG;
   const size_t asz = size_t(a_slots) * (a_rows_pad / oztc::kM) * nks * (oztc::kABytes / 2);
-  const size_t bsz = size_t(b_slots) * (b_rows_pad / bn) * nks * (oztc::b_bytes(bn) / 2);
+  const size_t bsz = size_t(b_slots) * b_halves * nks * (oztc::kBBytes / 2);
   // products of few tiles (the single small products of the canonical basis
   // and the evolution) are latency-bound: the 32 x 32 mma.sync tiles spread
   // them over more SMs.  The paired form has twice the tiles of half the
   // k-steps; it is counted in tiles of the real representation, so that both
   // forms route the same products here.
-  if (size_t(a_rows_pad / oztc::kM) * (b_rows_pad / bn) * a_slots / (pairs ? 2 : 1) < size_t(kTcMinTiles))
+  if (size_t(a_rows_pad / oztc::kM) * ((b_halves + 1) / 2) * a_slots / (pairs ? 2 : 1) < size_t(kTcMinTiles))
     return TVAP_ERR_ARG;
   int rc;
   OzScratch* sc = nullptr;
@@ -713,6 +701,7 @@ int gemm_tc(const GemmArgs& g, cudaStream_t s) {
   left.xk = xa.xk;
   left.kp = xa.kp;
   left.nstack = xa.nstack;
+  left.bfast = xa.bfast ? 1 : 0;
   left.slots = a_slots;
   left.rows_pad = a_rows_pad;
   left.nks = nks;
@@ -722,8 +711,8 @@ int gemm_tc(const GemmArgs& g, cudaStream_t s) {
         xa, oztc::kM, a_rows_pad, nks, As, ea);
     sc->left = left;
   }
-  slice_tc_kernel<<<dim3((xb.rows + 7) / 8, b_slots), kSliceThreads, slice_shm, tvap::counted(s)>>>(xb, bn, b_rows_pad, nks, Bs,
-                                                                                     eb);
+  slice_tc_kernel<<<dim3((xb.rows + 7) / 8, b_slots), kSliceThreads, slice_shm, tvap::counted(s)>>>(
+      xb, oztc::kHalf, b_rows_pad, nks, Bs, eb);
   o.C = g.C;
   o.crs = crs;
   o.ccs = ccs;
@@ -731,24 +720,22 @@ int gemm_tc(const GemmArgs& g, cudaStream_t s) {
   o.c_real = g.c_real;
   o.alpha = g.alpha.x;
   o.beta = g.beta.x;
-  o.a_rows = xa.xrows;
+  o.a_rows = L.rows;
   o.b_rows = xb.xrows;
   o.nstack = xa.nstack;
+  o.bfast = xa.bfast;
   const int sms = device_sms();
-  const long long ntiles = (long long)(a_rows_pad / oztc::kM) * (b_rows_pad / bn) * a_slots;
+  const long long ntiles = (long long)(a_rows_pad / oztc::kM) * ((b_halves + halves - 1) / halves) * a_slots;
   const int grid = int(std::min<long long>(ntiles, g_tc_grid_cap > 0 ? std::min(sms, g_tc_grid_cap) : sms));
   // the instantiation: alpha = +-1 (a sign in the integer conversion) or
-  // general, the B' tile width and the paired form
-  const bool unit_alpha = g_alpha_unit(o.alpha);
-  auto kern = pairs ? (unit_alpha ? (bn == 48 ? ozaki_tc_kernel<true, 48, true> : ozaki_tc_kernel<true, 64, true>)
-                                  : (bn == 48 ? ozaki_tc_kernel<false, 48, true> : ozaki_tc_kernel<false, 64, true>))
-                    : (unit_alpha ? (bn == 48 ? ozaki_tc_kernel<true, 48, false> : ozaki_tc_kernel<true, 64, false>)
-                                  : (bn == 48 ? ozaki_tc_kernel<false, 48, false> : ozaki_tc_kernel<false, 64, false>));
+  // general, and the paired form
+  auto kern = g_alpha_unit(o.alpha) ? (pairs ? ozaki_tc_kernel<true, true> : ozaki_tc_kernel<true, false>)
+                                    : (pairs ? ozaki_tc_kernel<false, true> : ozaki_tc_kernel<false, false>);
   if ((rc = smem_opt_in((const void*)kern, oztc::kSmemBytes))) return rc;
   TVAP_CUDA(cudaMemsetAsync(sc->counter, 0, sizeof(int), s));
   if (g_tc_timing_ctx) sec_begin_on(g_tc_timing_ctx, g_tc_timing_sec, s);
   kern<<<grid, oztc::kThreads, oztc::kSmemBytes, tvap::counted(s)>>>(As, ea, a_rows_pad, Bs, eb, b_rows_pad, b_slots == 1 ? 1 : 0,
-                                                      a_slots, nks, o, sc->counter, g_dev_flags);
+                                                      a_slots, nks, halves, o, sc->counter, g_dev_flags);
   if (g_tc_timing_ctx) sec_end_on(g_tc_timing_ctx, g_tc_timing_sec, s);
   TVAP_CUDA(cudaGetLastError());
   return TVAP_OK;

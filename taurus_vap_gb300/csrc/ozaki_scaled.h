@@ -1,6 +1,7 @@
 // Exact conversion of the two integer accumulators of the emulated
 // products to a double: (h 2^28 + l) 2^s rounded to nearest (ties to even),
-// negated when neg, from the 128-bit integer with integer instructions only.
+// negated when neg, with integer instructions only: the value's leading 64
+// bits and whether anything follows them.
 // It equals fma(double(h), 2^28, double(l)) * (+-2^s) -- both round once
 // when |h|, |l| < 2^53 -- at a fraction of the cost on a part whose FP64
 // pipe retires two operations per SM and cycle.  Returns false when the
@@ -40,44 +41,35 @@ TVAP_HD double bits_to_double(unsigned long long b) {
 }
 
 TVAP_HD bool scaled(long long h, long long l, int s, bool neg, double& out) {
-  unsigned long long lo = static_cast<unsigned long long>(h) << 28;
-  long long hi = h >> 36;
-  const unsigned long long sum = lo + static_cast<unsigned long long>(l);
-  hi += (l >> 63) + (sum < lo ? 1 : 0);
-  lo = sum;
-  bool sign = neg;
-  if (hi < 0) {
-    sign = !sign;
-    lo = ~lo + 1ull;
+  // hi 2^28 + lo with 0 <= lo < 2^28, then the magnitude
+  constexpr unsigned kMask = (1u << 28) - 1u;
+  long long hi = h + (l >> 28);
+  unsigned lo = unsigned(l) & kMask;
+  const bool minus = hi < 0;
+  if (minus) {
     hi = ~hi + (lo == 0 ? 1 : 0);
+    lo = (0u - lo) & kMask;
   }
+  // its leading 64 bits, the lowest one also set for what is shifted out
   const unsigned long long uh = static_cast<unsigned long long>(hi);
-  if ((uh | lo) == 0) {
+  const int top = uh ? 64 - clz64(uh) : 0;
+  const int sh = top > 36 ? top - 36 : 0;
+  unsigned long long u = (uh << (28 - sh)) | (lo >> sh);
+  u |= (lo & ((1u << sh) - 1u)) ? 1ull : 0ull;
+  if (u == 0) {
     out = neg ? -0.0 : 0.0;
     return true;
   }
-  int msb = uh ? 127 - clz64(uh) : 63 - clz64(lo);
-  unsigned long long mant;
-  if (msb <= 52) {
-    mant = lo << (52 - msb);
-  } else {
-    const int sh = msb - 52;
-    if (sh > 63) return false;
-    unsigned long long top = (lo >> sh) | (uh << (64 - sh));
-    const unsigned long long rem = lo & ((1ull << sh) - 1ull), half = 1ull << (sh - 1);
-    if (rem > half || (rem == half && (top & 1ull))) {
-      ++top;
-      if (top >> 53) {
-        top >>= 1;
-        ++msb;
-      }
-    }
-    mant = top;
-  }
-  const int e = msb + s + 1023;
-  if (e <= 0 || e >= 2047) return false;
-  out = bits_to_double((sign ? 1ull << 63 : 0ull) | (static_cast<unsigned long long>(e) << 52) |
-                       (mant & ((1ull << 52) - 1ull)));
+  const int n = clz64(u);
+  const int e = 63 - n + sh + s + 1023;  // biased exponent before rounding
+  if (e <= 0 || e >= 2046 || sh > 28) return false;
+  // round to 53 bits: half of the last one, less one unless the last bit is
+  // set; a carry out of bit 63 leaves the mantissa 0, the next power of two
+  u <<= n;
+  u += 0x3ffull + ((u >> 11) & 1ull);
+  const unsigned long long m = (u >> 11) & ((1ull << 52) - 1ull);
+  const unsigned long long up = u >> 63 ? 0ull : 1ull;
+  out = bits_to_double((minus != neg ? 1ull << 63 : 0ull) | ((static_cast<unsigned long long>(e) + up) << 52) | m);
   return true;
 }
 

@@ -176,9 +176,8 @@ extern thread_local int g_gemm_mode;
 // upper bound on the CTAs of a tcgen05 product (0: one per SM), set while
 // two streams share the SMs with kernels that need their own
 extern thread_local int g_tc_grid_cap;
-// width of the tcgen05 products' B' tiles: 0 the one that pads the output
-// columns less, 1 always 64 rows, 2 always 48 (set by every entry point from
-// its context's tuning)
+// columns of the tcgen05 products' tiles: 0 and 1 two halves of 32, 2 one half
+// (set by every entry point from its context's tuning)
 extern thread_local int g_tc_bn_policy;
 // the tcgen05 complex x complex products of contraction length >= this take
 // the paired form (real and imaginary rows interleaved on both sides), the
@@ -318,7 +317,7 @@ struct tvap_ctx {
   // test hook (tvap_test_wait_timeout): the next cooperative evolution has
   // its last CTA leave before the first grid barrier; one-shot
   bool test_skip_arrival = false;
-  // launch shapes chosen by tvap_autotune: B' tile policy (g_tc_bn_policy),
+  // launch shapes chosen by tvap_autotune: tile columns (g_tc_bn_policy),
   // groups of angles in the Thouless solve (2 staggered or 1), and the cap
   // on the tcgen05 CTAs while the second group's panels run (0: the SMs the
   // panels leave, 1: half of the SMs, 2: none)
