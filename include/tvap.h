@@ -163,9 +163,10 @@ int tvap_calculate_fields(tvap_ctx* ctx, const double* rhoLR, const double* kapp
                           double* gammaLR, double* hspLR, double* deltaLR, double* deltaRL);
 
 /* calculate_fields for `ncol` (1..256) independent density sets stored one
- * after the other (matrix c at offset c*n*n complex elements).  The call
- * allocates its staging buffers (8 ncol n^2 complex values) and frees them
- * before it returns; cudaFree waits for the whole device. */
+ * after the other (matrix c at offset c*n*n complex elements).  The work
+ * memory (up to 8 ncol n^2 complex values) stays in the context while it is
+ * at most 512 MB; a larger one is allocated by the call and freed before it
+ * returns (cudaFree waits for the whole device). */
 int tvap_calculate_fields_batched(tvap_ctx* ctx, int ncol, const double* rhoLR, const double* kappaLR,
                                   const double* kappaRL, double* gammaLR, double* hspLR, double* deltaLR,
                                   double* deltaRL);

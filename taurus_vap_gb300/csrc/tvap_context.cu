@@ -61,6 +61,9 @@ int device_sms() {
 int upload_matrix(const void* src, void* dst, size_t bytes, cudaStream_t s);
 int download_matrix(const void* src, void* dst, size_t bytes, cudaStream_t s);
 bool is_device_pointer(const void* p);
+bool is_device_pointer_on(const void* p, int device);
+// work memory of tvap_calculate_fields_batched that a context keeps, at most
+constexpr size_t kFieldsKeep = size_t(512) << 20;
 int check_finite(tvap_ctx* c, const double* const* ptrs, const char* const* names, int count, size_t elems);
 int project_device(tvap_ctx* c, const tvap_proj_opts& o, tvap_pnp* out, bool sync = true);
 int ensure_workspace(tvap_ctx* c, int G);
@@ -332,6 +335,7 @@ void tvap_destroy(tvap_ctx* c) {
   cudaFree(c->d_trperm);
   cudaFree(c->d_H1);
   cudaFree(c->d_flags);
+  cudaFree(c->fields_buf);
   cudaFree(c->d_bar);
   for (auto& e : c->ev_open) {
     cudaEventDestroy(e.second.first);
@@ -424,33 +428,77 @@ int tvap_calculate_fields_batched(tvap_ctx* c, int ncol, const double* rho, cons
   const int n = c->n;
   const size_t nn = size_t(n) * n, tot = nn * ncol;
   cudaStream_t s = c->stream;
-  double2* buf = nullptr;  // 7 * tot: staging (column-major) + 3 inner inputs + 4 inner outputs ... reused
-  TVAP_CUDA(cudaMalloc(&buf, sizeof(double2) * tot * 8));
-  double2* stage = buf;
-  double2* in[3] = {buf + tot, buf + 2 * tot, buf + 3 * tot};
-  double2* out[4] = {buf + 4 * tot, buf + 5 * tot, buf + 6 * tot, buf + 7 * tot};
   const double* srcs[3] = {rho, kLR, kRL};
   double* dsts[4] = {gamma, hsp, dLR, dRL};
-  int rc = TVAP_OK;
-  const int tb = 256;
-  const unsigned nb = unsigned((tot + tb - 1) / tb);
-  for (int q = 0; q < 3 && rc == TVAP_OK; ++q) {
-    rc = upload_matrix(srcs[q], stage, sizeof(double2) * tot, s);
-    if (rc == TVAP_OK) to_inner_kernel<<<nb, tb, 0, tvap::counted(s)>>>(nn, ncol, stage, in[q]);
-  }
-  if (rc == TVAP_OK) rc = fields_batched(c, ncol, ncol, in[0], in[1], in[2], out[0], out[1], out[2], out[3], s);
-  for (int q = 0; q < 4 && rc == TVAP_OK; ++q) {
-    from_inner_kernel<<<nb, tb, 0, tvap::counted(s)>>>(nn, ncol, out[q], stage);
-    rc = download_matrix(stage, dsts[q], sizeof(double2) * tot, s);
-    if (rc == TVAP_OK) {
-      cudaError_t e = cudaStreamSynchronize(s);
-      if (e != cudaSuccess) {
-        set_last_error(cudaGetErrorString(e), __FILE__, __LINE__);
-        rc = TVAP_ERR_CUDA;
+  // Device arrays of this GPU are transposed to and from the angle-innermost
+  // layout in place of a copy; others (host memory, another GPU, 8-byte
+  // aligned addresses) pass through a staging buffer.  One column is the same
+  // in both layouts.
+  auto direct = [&](const void* p) {
+    return (reinterpret_cast<uintptr_t>(p) & 15) == 0 && is_device_pointer_on(p, c->device);
+  };
+  bool in_direct[3], out_direct[4];
+  bool stage_any = false;
+  for (int q = 0; q < 3; ++q) stage_any |= !(in_direct[q] = direct(srcs[q]));
+  for (int q = 0; q < 4; ++q) stage_any |= !(out_direct[q] = direct(dsts[q]));
+  // 3 inputs, 4 outputs and the staging buffer; kept in the context up to
+  // kFieldsKeep bytes (an allocation and its release, which waits for the
+  // whole device, cost 400 us a call at n = 140, 113 columns)
+  const size_t need = sizeof(double2) * tot * (7 + (stage_any && ncol > 1 ? 1 : 0));
+  double2* buf = nullptr;
+  if (need <= kFieldsKeep) {
+    if (need > c->fields_bytes) {
+      if (c->fields_buf) {
+        TVAP_CUDA(cudaStreamSynchronize(s));
+        cudaFree(c->fields_buf);
       }
+      c->fields_buf = nullptr;
+      c->fields_bytes = 0;
+      TVAP_CUDA(cudaMalloc(&c->fields_buf, need));
+      c->fields_bytes = need;
+    }
+    buf = static_cast<double2*>(c->fields_buf);
+  } else {
+    TVAP_CUDA(cudaMalloc(&buf, need));
+  }
+  double2* in[3] = {buf, buf + tot, buf + 2 * tot};
+  double2* out[4] = {buf + 3 * tot, buf + 4 * tot, buf + 5 * tot, buf + 6 * tot};
+  double2* stage = buf + 7 * tot;
+  auto run = [&]() -> int {
+    const int tb = 256;
+    const unsigned nb = unsigned((tot + tb - 1) / tb);
+    int rc;
+    for (int q = 0; q < 3; ++q) {
+      if (ncol == 1) {
+        if ((rc = upload_matrix(srcs[q], in[q], sizeof(double2) * tot, s))) return rc;
+        continue;
+      }
+      if (!in_direct[q] && (rc = upload_matrix(srcs[q], stage, sizeof(double2) * tot, s))) return rc;
+      to_inner_kernel<<<nb, tb, 0, tvap::counted(s)>>>(
+          nn, ncol, in_direct[q] ? reinterpret_cast<const double2*>(srcs[q]) : stage, in[q]);
+    }
+    if ((rc = fields_batched(c, ncol, ncol, in[0], in[1], in[2], out[0], out[1], out[2], out[3], s))) return rc;
+    for (int q = 0; q < 4; ++q) {
+      if (ncol == 1) {
+        if ((rc = download_matrix(out[q], dsts[q], sizeof(double2) * tot, s))) return rc;
+        continue;
+      }
+      from_inner_kernel<<<nb, tb, 0, tvap::counted(s)>>>(
+          nn, ncol, out[q], out_direct[q] ? reinterpret_cast<double2*>(dsts[q]) : stage);
+      if (!out_direct[q] && (rc = download_matrix(stage, dsts[q], sizeof(double2) * tot, s))) return rc;
+    }
+    TVAP_CUDA(cudaGetLastError());
+    return TVAP_OK;
+  };
+  int rc = run();
+  if (rc == TVAP_OK) {
+    const cudaError_t e = cudaStreamSynchronize(s);
+    if (e != cudaSuccess) {
+      set_last_error(cudaGetErrorString(e), __FILE__, __LINE__);
+      rc = TVAP_ERR_CUDA;
     }
   }
-  cudaFree(buf);
+  if (need > kFieldsKeep) cudaFree(buf);
   // the status word: a bounded wait of the tensor-core field kernels that gave up
   if (rc == TVAP_OK) rc = check_flags(c);
   return rc;

@@ -311,6 +311,9 @@ struct tvap_ctx {
   // demand and reused: no allocation (and no device-wide cudaFree) per call
   double* scratch = nullptr;
   size_t scratch_count = 0;
+  // work memory of tvap_calculate_fields_batched (bounded: kFieldsKeep)
+  void* fields_buf = nullptr;
+  size_t fields_bytes = 0;
   // canonical bases: [0] FP32 Jacobi + refinement attempts, [1] of them
   // accepted, [2] exact FP64 Jacobi runs, [3] FP32 Jacobi sweeps in total
   long long canon_attempts[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
