@@ -214,11 +214,10 @@ __global__ void __launch_bounds__(128)
       uint32_t w[oztc::kDigits][4];
 #pragma unroll
       for (int kk = 0; kk < 8; kk += 2) {
-        int d0[oztc::kDigits], d1[oztc::kDigits];
-        oztc::to_digits(oz::to_fixed(part ? v[kk].y : v[kk].x, e), d0);
-        oztc::to_digits(oz::to_fixed(part ? v[kk + 1].y : v[kk + 1].x, e), d1);
+        uint32_t d2[oztc::kDigits];
+        oztc::digit_pair(part ? v[kk].y : v[kk].x, part ? v[kk + 1].y : v[kk + 1].x, e, d2);
 #pragma unroll
-        for (int s = 0; s < oztc::kDigits; ++s) w[s][kk >> 1] = oz::bf16x2_of_ints(d0[s], d1[s]);
+        for (int s = 0; s < oztc::kDigits; ++s) w[s][kk >> 1] = d2[s];
       }
       const int jr = part * ncols_tot + j;
       const size_t tb = (size_t(q.kboff) * ntn + size_t(jr / oztc::kHalf) * q.nks + k0 / 16) * oztc::kDigits;

@@ -263,16 +263,18 @@ __global__ void __launch_bounds__(kSliceThreads) slice_tc_kernel(TcSrc x, int ti
   __syncthreads();
   {
     const int w = t >> 5, lane = t & 31;
-    int er = oz::kExpZero, ei = oz::kExpZero;
+    // the largest exponent fields (0: zeros and subnormal numbers only)
+    unsigned mr = 0, mi = 0;
     for (int k = lane; k < K; k += 32) {
       const double2 v = xs[w * ldk + k];
-      if (v.x != 0.0) er = max(er, oz::dexp(v.x));
-      if (v.y != 0.0) ei = max(ei, oz::dexp(v.y));
+      mr = max(mr, unsigned(__double2hiint(v.x)) & 0x7ff00000u);
+      mi = max(mi, unsigned(__double2hiint(v.y)) & 0x7ff00000u);
     }
     for (int off = 16; off > 0; off >>= 1) {
-      er = max(er, __shfl_xor_sync(0xffffffffu, er, off));
-      ei = max(ei, __shfl_xor_sync(0xffffffffu, ei, off));
+      mr = max(mr, __shfl_xor_sync(0xffffffffu, mr, off));
+      mi = max(mi, __shfl_xor_sync(0xffffffffu, mi, off));
     }
+    int er = mr ? int(mr >> 20) - 1023 : oz::kExpZero, ei = mi ? int(mi >> 20) - 1023 : oz::kExpZero;
     if (form >= 2) er = ei = max(er, ei);  // one exponent for the real and imaginary part
     if (er == oz::kExpZero) er = 0;
     if (ei == oz::kExpZero) ei = 0;
@@ -302,13 +304,12 @@ __global__ void __launch_bounds__(kSliceThreads) slice_tc_kernel(TcSrc x, int ti
     uint32_t w[oztc::kDigits][4];
 #pragma unroll
     for (int j = 0; j < 8; j += 2) {
-      int d0[oztc::kDigits], d1[oztc::kDigits];
       const double2 v0 = (k0 + j < K) ? xs[row * ldk + k0 + j] : make_double2(0.0, 0.0);
       const double2 v1 = (k0 + j + 1 < K) ? xs[row * ldk + k0 + j + 1] : make_double2(0.0, 0.0);
-      oztc::to_digits(oz::to_fixed(part ? v0.y : v0.x, emax), d0);
-      oztc::to_digits(oz::to_fixed(part ? v1.y : v1.x, emax), d1);
+      uint32_t d[oztc::kDigits];
+      oztc::digit_pair(part ? v0.y : v0.x, part ? v1.y : v1.x, emax, d);
 #pragma unroll
-      for (int s = 0; s < oztc::kDigits; ++s) w[s][j >> 1] = oz::bf16x2_of_ints(d0[s], d1[s]);
+      for (int s = 0; s < oztc::kDigits; ++s) w[s][j >> 1] = d[s];
     }
     auto put = [&](int q, int kq, uint32_t flip) {
       const size_t tb = (size_t(slot) * tiles + q / tile_rows) * nks + (kq >> 4);
@@ -577,6 +578,13 @@ namespace {
 
 constexpr int kTcMinTiles = 152;
 
+// Contraction length from which complex x complex products take the paired
+// form.  It needs half the left operand's digit planes and pads the doubled
+// columns instead of the columns (n = 140: 288 for 2 x 160), at twice the
+// tiles of half the k-steps: as many folds once the real representation's 2 K
+// exceed one fold interval, twice as many below.
+constexpr int kPairsMinK = oztc::kFoldKs * 16 / 2 + 1;
+
 inline bool g_alpha_unit(double a) { return a == 1.0 || a == -1.0; }
 
 // The tensor-memory path for one product (mode 2).  Returns TVAP_ERR_ARG
@@ -621,11 +629,9 @@ int gemm_tc(const GemmArgs& g, cudaStream_t s) {
   o.a_mult = o.b_mult = 1;
   const bool stack = g.batch > 1 && (a_sh || b_sh);
   // complex x complex: the paired form (rows interleaved on both sides, the
-  // 2 x 2 blocks combined by the epilogue; half the left operand's digit
-  // planes, twice the tiles of half the k-steps, so that it pays where the
-  // contraction is long; batches with a shared operand keep the real
-  // representation) or the real representation
-  const bool pairs = !L.real && !R.real && !stack && g_tc_pairs_min_k > 0 && K >= g_tc_pairs_min_k;
+  // 2 x 2 blocks combined by the epilogue) or the real representation; batches
+  // with a shared operand keep the real representation
+  const bool pairs = !L.real && !R.real && !stack && K >= (g_tc_pairs_min_k > 0 ? g_tc_pairs_min_k : kPairsMinK);
   if (pairs) {
     xa.form = xb.form = 4;
     o.a_mult = o.b_mult = 2;

@@ -98,6 +98,38 @@ __host__ __device__ __forceinline__ void to_digits(long long X, int* d) {
   }
 }
 
+#ifdef __CUDACC__
+// bf16 bit patterns of the digits of two values (a in the low halves of w, b
+// in the high ones) under the scale 2^emax, as to_digits(to_fixed()) gives
+// them.  X + 128 (256^0 + .. + 256^6) is positive and its bytes are the
+// balanced digits plus 128; a byte under the exponent of 2^23 minus 2^23 + 128
+// is the digit as an FP32 number whose upper half is its bf16 pattern: three
+// instructions a digit in place of seven.  The rounded shift has no branches:
+// 2 mantissa >> t, half up, t = emax - exponent >= 0 (at most 63: nothing left).
+__device__ __forceinline__ void digit_pair(double a, double b, int emax, uint32_t* w) {
+  auto biased = [emax](double x) {
+    const uint32_t hi = uint32_t(__double2hiint(x)), eb = (hi >> 20) & 0x7ffu;
+    unsigned long long m = (static_cast<unsigned long long>((hi & 0xfffffu) | 0x100000u) << 32) |
+                           uint32_t(__double2loint(x));
+    const int t = min(emax + 1023 - int(eb), 63);
+    m = ((m << 1) + ((1ull << t) >> 1)) >> t;
+    if (eb == 0) m = 0;  // zero and subnormal numbers
+    constexpr unsigned long long kBias = 0x80808080808080ull;
+    return int(hi) < 0 ? kBias - m : kBias + m;
+  };
+  const unsigned long long A = biased(a), B = biased(b);
+#pragma unroll
+  for (int s = 0; s < kDigits; ++s) {
+    const int byte = kDigits - 1 - s;
+    const uint32_t sel = 0x7540u + uint32_t(byte & 3);
+    const uint32_t wa = byte < 4 ? uint32_t(A) : uint32_t(A >> 32), wb = byte < 4 ? uint32_t(B) : uint32_t(B >> 32);
+    const float fa = __uint_as_float(__byte_perm(wa, 0x4B000000u, sel)) - 8388736.0f;
+    const float fb = __uint_as_float(__byte_perm(wb, 0x4B000000u, sel)) - 8388736.0f;
+    w[s] = __byte_perm(__float_as_uint(fa), __float_as_uint(fb), 0x7632);
+  }
+}
+#endif
+
 // element offset of (row r, k) inside the k-step tile of one digit plane
 __host__ __device__ __forceinline__ int tile_offset(int r, int k) {
   return (r >> 3) * 128 + ((k >> 3) & 1) * 64 + (r & 7) * 8 + (k & 7);

@@ -181,8 +181,8 @@ extern thread_local int g_tc_grid_cap;
 extern thread_local int g_tc_bn_policy;
 // the tcgen05 complex x complex products of contraction length >= this take
 // the paired form (real and imaginary rows interleaved on both sides), the
-// others the real representation [[Re, -Im], [Im, Re]] x [Re, Im]; 0: none
-// (set by every entry point from its context)
+// others the real representation [[Re, -Im], [Im, Re]] x [Re, Im]; 0: from
+// kPairsMinK on (set by every entry point from its context)
 extern thread_local int g_tc_pairs_min_k;
 struct TcGridCap {
   int saved;
@@ -329,7 +329,7 @@ struct tvap_ctx {
   int tune_cap = 0;
   int tune_lookahead = 0;  // look-ahead of the Thouless solve's panels (streamB)
   int tune_pf_blocked = 0;  // the blocked Pfaffian also where the shared-memory one fits
-  int tune_pairs_k = 0;     // complex x complex tcgen05 products in the paired form from K = this on (0: none)
+  int tune_pairs_k = 0;     // complex x complex tcgen05 products in the paired form from K = this on (0: kPairsMinK)
 };
 
 namespace tvap {
