@@ -573,27 +573,26 @@ __global__ void __launch_bounds__(kPfThreads) pfaffian_kernel(int N, double2* Aa
   }
 }
 
-// The same elimination with the packed upper triangle in shared memory
-// (N (N + 1) / 2 entries, column-major): every access stays on the SM, the
-// pivot search is a warp reduction plus one block step, and the already
-// eliminated columns (which no longer enter the Pfaffian) are neither
-// exchanged nor scaled.
-// The same elimination with the packed upper triangle in shared memory.  Per
-// step only the pivot's reciprocal is needed by every thread: one thread
-// forms it (an FP64 division costs ~1000 cycles and an FP64 warp instruction
-// ~16 cycles of the SM's FP64 pipe, so redundant scalar work in every thread
-// costs as much as the rank-2 update), the pivot search compares integer keys,
-// and the pivots are kept in shared memory and folded into log|Pf| and its
-// phase once, at the end, by a fixed-order warp reduction.
+// The same elimination with the packed upper triangle in shared memory (N (N +
+// 1) / 2 entries, column-major).  An FP64 warp instruction holds the FP64 unit
+// of its SM sub-partition for about 64 cycles whatever lanes are active, so
+// the rank-2 update (8 N^3 / 6 of the 8 N^3 / 6 + O(N^2) FMAs) runs over the
+// packed entries as one list, whole warps but for the last: by column pairs,
+// 16 warps and 32 lanes rounded every step up, a third of the issues at N =
+// 140.  Per step only the pivot's reciprocal is needed by every thread: one
+// thread forms it beside the interchange, u = x / pivot is formed once per
+// entry (A(I, J) += u_I y_J - y_I u_J), the eliminated columns are neither
+// exchanged nor negated, the pivot search compares integer keys, and the
+// pivots are kept in shared memory and folded into log|Pf| and its phase once,
+// at the end, by a fixed-order warp reduction.  113 matrices of N = 140: 696
+// us with column pairs (470 us of FP64 issues at one matrix per SM).
 __global__ void __launch_bounds__(kPfThreads) pfaffian_smem_kernel(int N, const double2* __restrict__ Aall,
                                                                    double2* pf, int batch, int* flags) {
   extern __shared__ double2 pf_smem[];
   double2* pk = pf_smem;
-  double2* xcol = pk + size_t(N) * (N + 1) / 2;  // 1-based, N + 1 entries
-  double2* ycol = xcol + N + 1;
+  double2* ucol = pk + size_t(N) * (N + 1) / 2;  // x / pivot and y, 1-based, N + 1 entries
+  double2* ycol = ucol + N + 1;
   double2* pivs = ycol + N + 1;                  // N / 2 pivots, then N / 2 signs in .x of the next slots
-  double2* tt1 = pivs + N;                       // alpha y_J and alpha x_J, 1-based
-  double2* tt2 = tt1 + N + 1;
   __shared__ long long wv[kPfThreads / 32];
   __shared__ int wi[kPfThreads / 32];
   __shared__ int s_kp;
@@ -645,93 +644,66 @@ __global__ void __launch_bounds__(kPfThreads) pfaffian_smem_kernel(int N, const 
       if (lane == 0) s_kp = (v <= 0) ? -1 : i;  // -1: the column is zero
     }
     __syncthreads();
-    int KP = s_kp;
-    const int KK = K - 1;
-    if (KP < 0) {
+    const int KK = K - 1, KP = s_kp < 0 ? KK : s_kp;
+    if (s_kp < 0) {
       zero = true;
-      KP = KK;
+      break;
     }
-    if (KP != KK) {
+    const bool swap = KP != KK;
+    const int nn = K - 2;
+    // the pivot's reciprocal (the last thread) beside the interchange of rows
+    // and columns KP and KK; the entries that change sides of the diagonal are
+    // negated here (row KP) or when the column is read (KK)
+    if (tid == nt - 1) {
+      const double2 piv = a(KP, K);
+      pivs[steps] = piv;
+      pivs[N / 2 + steps] = make_double2(swap ? -1.0 : 1.0, 0.0);
+      s_alpha = crcp_newton(piv);
+    }
+    if (swap) {
       for (int i = 1 + tid; i <= KP - 1; i += nt) {
         const double2 t = a(i, KK);
         a(i, KK) = a(i, KP);
         a(i, KP) = t;
       }
-      for (int t = tid; t < KK - KP - 1; t += nt) {
-        const double2 u = a(KP + 1 + t, KK);
-        a(KP + 1 + t, KK) = a(KP, KP + 1 + t);
-        a(KP, KP + 1 + t) = u;
+      for (int j = KP + 1 + tid; j <= KK - 1; j += nt) {
+        const double2 u = a(j, KK);
+        a(j, KK) = a(KP, j);
+        a(KP, j) = cneg(u);
       }
-      if (tid == 0) {
-        const double2 u = a(KK, K);
-        a(KK, K) = a(KP, K);
-        a(KP, K) = u;
-      }
-      __syncthreads();
-      for (int i = KP + tid; i <= KK - 1; i += nt) a(i, KK) = cneg(a(i, KK));
-      for (int j = KP + 1 + tid; j <= KK - 1; j += nt) a(KP, j) = cneg(a(KP, j));
-      __syncthreads();
-    }
-    if (zero) break;
-    const int nn = K - 2;
-    if (tid == 0) {
-      const double2 piv = a(K - 1, K);
-      pivs[steps] = piv;
-      pivs[N / 2 + steps] = make_double2(KP != KK ? -1.0 : 1.0, 0.0);
-      s_alpha = crcp_newton(piv);
     }
     __syncthreads();
-    // the two columns and their products with alpha, once per step (threads
-    // over the entries: the FP64 pipe is the bottleneck of this kernel)
     {
       const double2 alpha = s_alpha;
       for (int i = 1 + tid; i <= nn; i += nt) {
-        const double2 x = a(i, K), y = a(i, K - 1);
-        xcol[i] = x;
-        ycol[i] = y;
-        tt1[i] = cmul(alpha, y);
-        tt2[i] = cmul(alpha, x);
+        // row KP of column K is what row KK was (the pivot moved there)
+        const double2 x = swap && i == KP ? a(KK, K) : a(i, K);
+        const double2 y = a(i, KK);
+        ucol[i] = cmul(alpha, x);
+        ycol[i] = swap && i >= KP ? cneg(y) : y;
       }
     }
     __syncthreads();
-    // A(I,J) += X(I) (alpha Y(J)) - Y(I) (alpha X(J)), I < J <= nn: a warp
-    // per pair of columns J1 = 2 + p and J2 = nn - p (about nn entries
-    // together), lanes over the pair's entries, two entries in flight
-    for (int p = warp; p < nn / 2; p += nw) {
-      const int J1 = 2 + p, J2 = nn - p;
-      const int L1 = J1 - 1, L = L1 + (J2 > J1 ? J2 - 1 : 0);
-      for (int f0 = lane; f0 < L; f0 += 64) {
-        int I[2], J[2];
-        double2 v[2], x[2], y[2], t1[2], t2[2];
-#pragma unroll
-        for (int u = 0; u < 2; ++u) {
-          const int f = f0 + 32 * u;
-          const bool first = f < L1;
-          I[u] = first ? f + 1 : f - L1 + 1;
-          J[u] = first ? J1 : J2;
-          if (f < L) {
-            v[u] = a(I[u], J[u]);
-            x[u] = xcol[I[u]];
-            y[u] = ycol[I[u]];
-            t1[u] = tt1[J[u]];
-            t2[u] = tt2[J[u]];
-          }
-        }
-#pragma unroll
-        for (int u = 0; u < 2; ++u) {
-          if (f0 + 32 * u >= L) continue;
-          double2 w = v[u];
-          w.x = fma(x[u].x, t1[u].x, w.x);
-          w.x = fma(-x[u].y, t1[u].y, w.x);
-          w.y = fma(x[u].x, t1[u].y, w.y);
-          w.y = fma(x[u].y, t1[u].x, w.y);
-          w.x = fma(-y[u].x, t2[u].x, w.x);
-          w.x = fma(y[u].y, t2[u].y, w.x);
-          w.y = fma(-y[u].x, t2[u].y, w.y);
-          w.y = fma(-y[u].y, t2[u].x, w.y);
-          a(I[u], J[u]) = w;
-        }
-      }
+    // A(I, J) += u(I) y(J) - y(I) u(J), I < J <= nn, over the packed entries
+    const int E = nn * (nn + 1) / 2;
+#pragma unroll 2
+    for (int e = 1 + tid; e < E; e += nt) {
+      int J = int((sqrtf(8.0f * float(e) + 1.0f) + 1.0f) * 0.5f);
+      if (J * (J - 1) / 2 > e) --J;
+      if (J * (J + 1) / 2 <= e) ++J;
+      const int I = e - J * (J - 1) / 2 + 1;
+      if (I == J) continue;
+      const double2 u = ucol[I], y = ycol[I], uj = ucol[J], yj = ycol[J];
+      double2 w = pk[e];
+      w.x = fma(u.x, yj.x, w.x);
+      w.y = fma(u.x, yj.y, w.y);
+      w.x = fma(-u.y, yj.y, w.x);
+      w.y = fma(u.y, yj.x, w.y);
+      w.x = fma(-y.x, uj.x, w.x);
+      w.y = fma(-y.x, uj.y, w.y);
+      w.x = fma(y.y, uj.y, w.x);
+      w.y = fma(-y.y, uj.x, w.y);
+      pk[e] = w;
     }
     __syncthreads();
   }
@@ -917,7 +889,7 @@ __global__ void __launch_bounds__(kPfThreads) pf_panel_kernel(int N, int Kstart,
 // other streams share their SMs)
 int pfaffian_batched(int n, int batch, double2* A, double2* pf, int* flags, cudaStream_t s, bool blocked) {
   if (n > 512 || (n & 1)) return TVAP_ERR_ARG;
-  const size_t shm = sizeof(double2) * (size_t(n) * (n + 1) / 2 + 4 * size_t(n + 1) + size_t(n));
+  const size_t shm = sizeof(double2) * (size_t(n) * (n + 1) / 2 + 2 * size_t(n + 1) + size_t(n));
   if (shm <= jacobi32_smem_limit() && !(blocked && n >= 2)) {
     // the packed upper triangle fits shared memory: the unblocked elimination
     if (int rc = smem_opt_in((const void*)pfaffian_smem_kernel, jacobi32_smem_limit())) return rc;
