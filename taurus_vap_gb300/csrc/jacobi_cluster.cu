@@ -51,7 +51,7 @@ __device__ __forceinline__ int jc_block(int r, int p, int nb) {
 // follows), and every step of the per-pair chain is latency.
 template <int kJcRows>
 __device__ __forceinline__ float jc_rotate(int ma, int mb, int wa, int wb, int n, int lane) {
-  extern __shared__ float jc[];  // the kernel's dynamic shared memory: offsets keep the accesses in LDS/STS
+  extern __shared__ __align__(16) float jc[];  // the kernel's dynamic shared memory: offsets keep the accesses in LDS/STS
   float* Ma = jc + ma;
   float* Mb = jc + mb;
   float* Wa = jc + wa;
@@ -94,7 +94,7 @@ __device__ __forceinline__ float jc_rotate(int ma, int mb, int wa, int wb, int n
     t = __fdividef(0.5f, zeta);
   } else {
     const float q = fmaf(zeta, zeta, 1.f);
-    t = copysignf(__frcp_rn(az + q * rsqrtf(q)), zeta);
+    t = copysignf(__fdividef(1.f, az + q * rsqrtf(q)), zeta);
   }
   const float c = rsqrtf(fmaf(t, t, 1.f)), s = c * t;
 #pragma unroll
@@ -120,7 +120,7 @@ __global__ void __launch_bounds__(kJcThreads) jacobi_cluster_kernel(int n, const
                                                                     const double* __restrict__ W0,
                                                                     double* __restrict__ W64, int* sweeps_out) {
   constexpr int kJcBlocks = 2 * kJcCtas;
-  extern __shared__ float jc[];  // [buf 2][slot 2][mat 2][bw][n]
+  extern __shared__ __align__(16) float jc[];  // [buf 2][slot 2][mat 2][bw][n]
   __shared__ float wmax[kJcThreads / 32];
   __shared__ float cl_max[kJcCtas];
   cg::cluster_group cluster = cg::this_cluster();
@@ -218,9 +218,16 @@ __global__ void __launch_bounds__(kJcThreads) jacobi_cluster_kernel(int n, const
         float* dst = col(nxt, slot, 0, 0);
         // M and W of a slot are contiguous: 2 bw n floats
         const int cnt = 2 * bw * n;
-        for (int idx = tid; idx < cnt; idx += blockDim.x) dst[idx] = src[idx];
+        if ((cnt & 3) == 0) {
+          const float4* src4 = reinterpret_cast<const float4*>(src);
+          float4* dst4 = reinterpret_cast<float4*>(dst);
+#pragma unroll 4
+          for (int idx = tid; idx < cnt / 4; idx += blockDim.x) dst4[idx] = src4[idx];
+        } else {
+          for (int idx = tid; idx < cnt; idx += blockDim.x) dst[idx] = src[idx];
+        }
       }
-      cluster.sync();
+      __syncthreads();
       cur = nxt;
     }
     // cluster-wide largest |cos| of the sweep
@@ -258,6 +265,55 @@ __global__ void __launch_bounds__(kJcThreads) jacobi_cluster_kernel(int n, const
     }
   }
   if (c == 0 && tid == 0 && sweeps_out) *sweeps_out = sweep;
+}
+
+// The same one-sided Jacobi with all columns of M and W in one CTA: a sweep is
+// the circle method over the columns, a warp per pair, a CTA barrier per round.  A cluster barrier costs
+// over a microsecond, and the cluster's sweep has 30 of them whatever n is;
+// here a round is the latency of one pair (about 300 cycles).
+constexpr int kJ1MaxWarps = 32;
+template <int kJcRows>
+__global__ void __launch_bounds__(32 * kJ1MaxWarps)
+    jacobi_cta_kernel(int n, const double* __restrict__ M64, int mt, const double* __restrict__ W0,
+                      double* __restrict__ W64, int* sweeps_out) {
+  extern __shared__ __align__(16) float jc[];  // M, then W (n x n each, columns contiguous)
+  __shared__ float wmax[kJ1MaxWarps];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, warps = blockDim.x >> 5;
+  const int nn = n * n;
+  for (int idx = tid; idx < nn; idx += blockDim.x) {
+    const int j = idx / n, r = idx - j * n;
+    jc[idx] = float(mt ? M64[j + size_t(r) * n] : M64[idx]);
+    jc[nn + idx] = W0 ? float(W0[idx]) : (r == j ? 1.f : 0.f);
+  }
+  __syncthreads();
+  const int ne = (n + 1) & ~1, half = ne / 2;  // the odd column out sits a round out
+  int sweep = 0;
+  while (sweep < kJcMaxSweeps) {
+    float mx = 0.f;
+    for (int round = 0; round < ne - 1; ++round) {
+      for (int k = warp; k < half; k += warps) {
+        int p = round, q = ne - 1;
+        if (k > 0) {
+          p = round + k;
+          if (p >= ne - 1) p -= ne - 1;
+          q = round - k;
+          if (q < 0) q += ne - 1;
+        }
+        if (p < n && q < n)
+          mx = fmaxf(mx, jc_rotate<kJcRows>(p * n, q * n, nn + p * n, nn + q * n, n, lane));
+      }
+      __syncthreads();
+    }
+    ++sweep;
+    if (lane == 0) wmax[warp] = mx;
+    __syncthreads();
+    float gm = 0.f;
+    for (int w = 0; w < warps; ++w) gm = fmaxf(gm, wmax[w]);
+    __syncthreads();  // wmax is rewritten by the next sweep
+    if (gm <= kJcTol) break;
+  }
+  for (int idx = tid; idx < nn; idx += blockDim.x) W64[idx] = double(jc[nn + idx]);
+  if (tid == 0 && sweeps_out) *sweeps_out = sweep;
 }
 
 }  // namespace
@@ -306,13 +362,35 @@ int launch_jacobi_cluster(int n, const double* M, int m_transposed, const double
   return TVAP_OK;
 }
 
+// up to here one CTA is quicker (from random starts: n = 24 109 us against 237,
+// n = 40 231 against 360, n = 60 528 against 486)
+constexpr int kJ1MaxN = 48;
+
+template <int ROWS>
+int launch_jacobi_cta(int n, const double* M, int m_transposed, const double* W0, double* W, int* sweeps_out,
+                      cudaStream_t s) {
+  const int half = (n + 1) / 2, per = (half + kJ1MaxWarps - 1) / kJ1MaxWarps, warps = (half + per - 1) / per;
+  const size_t shm = sizeof(float) * 2 * size_t(n) * n;
+  if (shm > 48 * 1024)
+    if (int rc = smem_opt_in((const void*)jacobi_cta_kernel<ROWS>, shm)) return rc;
+  jacobi_cta_kernel<ROWS><<<1, 32 * warps, shm, tvap::counted(s)>>>(n, M, m_transposed, W0, W, sweeps_out);
+  TVAP_CUDA(cudaGetLastError());
+  return TVAP_OK;
+}
+
 }  // namespace
 
-// FP32 block one-sided Jacobi on a cluster: 8 CTAs (16 column blocks) up to
+// FP32 one-sided Jacobi: one CTA up to n = kJ1MaxN; then the block form on a cluster, 8 CTAs (16 column blocks) up to
 // n = 256, 16 CTAs (32 column blocks, an opt-in cluster size) up to n = 384;
 // TVAP_ERR_ARG when neither fits (the caller then uses another eigensolver).
 int jacobi_cluster(int n, const double* M, int m_transposed, const double* W0, double* W, int* sweeps_out,
                    cudaStream_t s) {
+  if (n <= 32) return launch_jacobi_cta<1>(n, M, m_transposed, W0, W, sweeps_out, s);
+  if (n <= kJ1MaxN) return launch_jacobi_cta<2>(n, M, m_transposed, W0, W, sweeps_out, s);
+  // (rows per lane as n needs them: a rotation is bound by its instructions)
+  if (n <= 96) return launch_jacobi_cluster<8, 3>(n, M, m_transposed, W0, W, sweeps_out, s);
+  if (n <= 128) return launch_jacobi_cluster<8, 4>(n, M, m_transposed, W0, W, sweeps_out, s);
+  if (n <= 160) return launch_jacobi_cluster<8, 5>(n, M, m_transposed, W0, W, sweeps_out, s);
   if (n <= 256) return launch_jacobi_cluster<8, 8>(n, M, m_transposed, W0, W, sweeps_out, s);
   return launch_jacobi_cluster<16, 12>(n, M, m_transposed, W0, W, sweeps_out, s);
 }
