@@ -29,6 +29,8 @@
 //   S = R11 - R12 R22^{-1} R21  (R22: the nocc occupied states),
 // which needs one Pfaffian of size n2 - nocc and no inverse of R_n2.
 
+#include <cooperative_groups.h>
+
 #include <algorithm>
 #include <cmath>
 #include <complex>
@@ -36,6 +38,8 @@
 #include <vector>
 
 #include "tvap_internal.cuh"
+
+namespace cg = cooperative_groups;
 
 namespace tvap {
 
@@ -948,38 +952,57 @@ __global__ void schur_kernel(int n2, int nb, int G, const double2* __restrict__ 
 // a serial Jacobi sweep on one SM.  Near-degenerate clusters are
 // diagonalised exactly afterwards (cluster_finish_kernel).
 // ---------------------------------------------------------------------------
-constexpr int kRlThreads = 1024;
-__global__ void __launch_bounds__(kRlThreads)
+// The reductions over n^2 entries of the refinement (norms, clusters, the final
+// check) run on a cluster of 8 CTAs, partial results gathered in CTA 0's
+// shared memory in a fixed order: an SM retires two FP64 operations a cycle,
+// so that one CTA took 43 us for the three norms at n = 140.  Comparisons of
+// doubles, FP64 operations too, are made on their bits.
+constexpr int kRlCtas = 8;
+constexpr int kRlThreads = 512;
+// a double's bits as an integer of the same order (-0 below +0)
+__device__ __forceinline__ long long order_key(double v) {
+  const long long b = __double_as_longlong(v);
+  return b ^ ((b >> 63) & 0x7fffffffffffffffLL);
+}
+// |v| as an integer of the same order (a NaN is larger than any number)
+__device__ __forceinline__ unsigned long long abs_key(double v) {
+  return static_cast<unsigned long long>(__double_as_longlong(v)) & 0x7fffffffffffffffULL;
+}
+
+__global__ void __cluster_dims__(kRlCtas, 1, 1) __launch_bounds__(kRlThreads)
     refine_lambda_kernel(int n, const double* __restrict__ XtX, const double* __restrict__ S,
                          const double* __restrict__ A, double* __restrict__ lam, double* __restrict__ rscal) {
-  __shared__ double red[3][kRlThreads / 32];
-  const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, warp = tid >> 5;
-  for (int i = tid; i < n; i += nt) lam[i] = S[i + size_t(i) * n] / XtX[i + size_t(i) * n];
+  __shared__ double red[3][kRlThreads / 32], gathered[kRlCtas][3];
+  cg::cluster_group cluster = cg::this_cluster();
+  const int rank = int(cluster.block_rank());
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int g = rank * kRlThreads + tid, ng = kRlCtas * kRlThreads;
+  for (int i = g; i < n; i += ng) lam[i] = S[i + size_t(i) * n] / XtX[i + size_t(i) * n];
   double s_off = 0.0, s_r = 0.0, s_a = 0.0;
-  const size_t nn = size_t(n) * n;
+  const int nn = n * n;
   // four elements in flight per thread
-  for (size_t e0 = tid; e0 < nn; e0 += 4 * size_t(nt)) {
+  for (int e0 = g; e0 < nn; e0 += 4 * ng) {
     double xv[4], sv[4], av[4];
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
-      const size_t e = e0 + size_t(u) * nt;
+      const int e = e0 + u * ng;
       xv[u] = e < nn ? XtX[e] : 0.0;
       sv[u] = e < nn ? S[e] : 0.0;
       av[u] = e < nn ? A[e] : 0.0;
     }
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
-      const size_t e = e0 + size_t(u) * nt;
+      const int e = e0 + u * ng;
       if (e >= nn) continue;
-      const int i = int(e % n), j = int(e / n);
-      const bool d = (i == j);
+      const bool d = e % (n + 1) == 0;
       const double r = (d ? 1.0 : 0.0) - xv[u];
       // the diagonal of S - diag(l) with l = S_ii / XtX_ii, formed here from
       // the same operands as lam
-      const double so = d ? sv[u] - sv[u] / xv[u] : sv[u];
-      s_off += so * so;
-      s_r += r * r;
-      s_a += av[u] * av[u];
+      double so = sv[u];
+      if (d) so = sv[u] - sv[u] / xv[u];
+      s_off = fma(so, so, s_off);
+      s_r = fma(r, r, s_r);
+      s_a = fma(av[u], av[u], s_a);
     }
   }
   for (int o = 16; o > 0; o >>= 1) {
@@ -993,12 +1016,18 @@ __global__ void __launch_bounds__(kRlThreads)
     red[2][warp] = s_a;
   }
   __syncthreads();
-  if (tid == 0) {
+  if (tid < 3) {
+    double t = 0.0;
+    for (int w2 = 0; w2 < kRlThreads / 32; ++w2) t += red[tid][w2];
+    *cluster.map_shared_rank(&gathered[rank][tid], 0) = t;
+  }
+  cluster.sync();
+  if (rank == 0 && tid == 0) {
     double a0 = 0.0, a1 = 0.0, a2 = 0.0;
-    for (int w2 = 0; w2 < nt / 32; ++w2) {
-      a0 += red[0][w2];
-      a1 += red[1][w2];
-      a2 += red[2][w2];
+    for (int q = 0; q < kRlCtas; ++q) {
+      a0 += gathered[q][0];
+      a1 += gathered[q][1];
+      a2 += gathered[q][2];
     }
     const double nS = sqrt(a0), nR = sqrt(a1), nA = sqrt(a2);
     rscal[0] = 2.0 * (nS + nA * nR);  // delta
@@ -1116,36 +1145,44 @@ constexpr double kCfGate = 64.0;    // Newton step where |l_j - l_i| > kCfGate |
 // is not kCfGate times their coupling, |l_j - l_i| <= kCfGate |S_ij| +
 // 1e-13 ||A||, belong to one cluster, and a cluster is the smallest range
 // of the sorted Rayleigh quotients that contains every such pair.  cid[i] =
-// the first sorted position of column i's cluster.  One CTA.
-__global__ void __launch_bounds__(kCfThreads)
+// the first sorted position of column i's cluster.  Every CTA of the cluster
+// sorts (integers), the pairs are split, CTA 0 joins them.
+__global__ void __cluster_dims__(kRlCtas, 1, 1) __launch_bounds__(kCfThreads)
     cluster_assign_kernel(int n, const double* __restrict__ S, const double* __restrict__ lam,
                           const double* __restrict__ rscal, int* __restrict__ cid) {
   __shared__ int pos[kCfMaxN], order[kCfMaxN], reach[kCfMaxN];
+  __shared__ double ls[kCfMaxN];
+  __shared__ long long key[kCfMaxN];
+  cg::cluster_group cluster = cg::this_cluster();
+  const int rank = int(cluster.block_rank());
   const int tid = threadIdx.x, nt = blockDim.x;
   for (int i = tid; i < n; i += nt) {
-    const double v = lam[i];
-    int rank = 0;
-    for (int j = 0; j < n; ++j) {
-      const double u = lam[j];
-      rank += (u < v || (u == v && j < i)) ? 1 : 0;
-    }
-    pos[i] = rank;
-    order[rank] = i;
-    reach[rank] = rank;
+    ls[i] = lam[i];
+    key[i] = order_key(ls[i]);
   }
   __syncthreads();
+  for (int i = tid; i < n; i += nt) {
+    const long long v = key[i];
+    int r = 0;
+    for (int j = 0; j < n; ++j) r += (key[j] < v || (key[j] == v && j < i)) ? 1 : 0;
+    pos[i] = r;
+    order[r] = i;
+    reach[r] = r;
+  }
+  cluster.sync();  // CTA 0's reach is written by all
+  int* reach0 = cluster.map_shared_rank(reach, 0);
   const double floor = 1.0e-13 * rscal[1];
-  for (size_t e = tid; e < size_t(n) * n; e += nt) {
-    const int i = int(e % n), j = int(e / n);
+  for (int e = rank * nt + tid; e < n * n; e += kRlCtas * nt) {
+    const int j = e / n, i = e - j * n;
     if (i >= j) continue;
     const double sb = 0.5 * (S[e] + S[j + size_t(i) * n]);
-    if (fabs(lam[j] - lam[i]) <= kCfGate * fabs(sb) + floor) {
+    if (fabs(ls[j] - ls[i]) <= kCfGate * fabs(sb) + floor) {
       const int pa = pos[i], pb = pos[j];
-      atomicMax(&reach[min(pa, pb)], max(pa, pb));
+      atomicMax(&reach0[min(pa, pb)], max(pa, pb));
     }
   }
-  __syncthreads();
-  if (tid == 0) {
+  cluster.sync();
+  if (rank == 0 && tid == 0) {
     int k = 0;
     while (k < n) {
       int j = reach[k];
@@ -1162,11 +1199,12 @@ __global__ void __launch_bounds__(kCfThreads)
 // beyond the rotation buffer: listed in bigd for the FP64 Jacobi of their
 // block, big_cluster_rotate_kernel); the coupling between clusters and the
 // orthonormality verified; D and the eigenvalues written in that order.
-// One CTA: the diagonal, the order and the clusters in shared memory, one
-// thread per small cluster for its Jacobi, a warp per cluster for the
-// rotation of its columns.  rflag[0] = failure bits, rflag[2] = number of
+// A cluster of CTAs, each with the diagonal, the order and the clusters in
+// shared memory and a thread per small cluster for its Jacobi (the same in
+// all); the check over the entries and the rotation of the columns (a warp per
+// cluster) are split.  CTA 0 writes the rest.  rflag[0] = failure bits, rflag[2] = number of
 // clusters in bigd, rflag[3] = 0 (the big clusters' Jacobi status).
-__global__ void __launch_bounds__(kCfThreads)
+__global__ void __cluster_dims__(kRlCtas, 1, 1) __launch_bounds__(kCfThreads)
     cluster_finish_kernel(int n, const double* __restrict__ S, const double* __restrict__ X,
                           const double* __restrict__ rscal, const int* __restrict__ cidg, double* __restrict__ D,
                           double* __restrict__ evals, int* __restrict__ cperm, int* __restrict__ bigd, int* rflag) {
@@ -1175,7 +1213,10 @@ __global__ void __launch_bounds__(kCfThreads)
   __shared__ int perm[kCfMaxN], cid[kCfMaxN], osh[kCfMaxN], cl_start[kCfMaxN + 1], qoff[kCfMaxN + 1];
   __shared__ double qbuf[kCfQ];
   __shared__ int ncl, fail, nbig;
-  __shared__ double red[kCfThreads / 32];
+  __shared__ long long key[kCfMaxN];
+  __shared__ unsigned long long red[kCfThreads / 32], gathered[kRlCtas];
+  cg::cluster_group cluster = cg::this_cluster();
+  const int rank = int(cluster.block_rank());
   const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, warp = tid >> 5, nwarp = nt >> 5;
   if (tid == 0) {
     fail = 0;
@@ -1183,22 +1224,24 @@ __global__ void __launch_bounds__(kCfThreads)
   }
   for (int i = tid; i < n; i += nt) {
     sd[i] = S[i + size_t(i) * n];
+    key[i] = order_key(sd[i]);
     cid[i] = cidg[i];
   }
   __syncthreads();
   for (int i = tid; i < n; i += nt) {
-    const double v = sd[i];
+    const long long v = key[i];
     const int ci = cid[i];
-    int rank = 0;
+    int r = 0;
     for (int j = 0; j < n; ++j) {
-      const double u = sd[j];
+      const long long u = key[j];
       const int cj = cid[j];
-      rank += (cj < ci || (cj == ci && (u < v || (u == v && j < i)))) ? 1 : 0;
+      r += (cj < ci || (cj == ci && (u < v || (u == v && j < i)))) ? 1 : 0;
     }
-    perm[rank] = i;
+    perm[r] = i;
   }
   __syncthreads();
-  for (int k = tid; k < n; k += nt) cperm[k] = perm[k];
+  if (rank == 0)
+    for (int k = tid; k < n; k += nt) cperm[k] = perm[k];
   const double nA = rscal[1];
   if (tid == 0) {
     int c = 0;
@@ -1217,8 +1260,10 @@ __global__ void __launch_bounds__(kCfThreads)
         off += m * m;
       } else if (nbig < kCfBigSlots) {
         qoff[q] = -1;
-        bigd[2 * nbig] = cl_start[q];
-        bigd[2 * nbig + 1] = m;
+        if (rank == 0) {
+          bigd[2 * nbig] = cl_start[q];
+          bigd[2 * nbig + 1] = m;
+        }
         ++nbig;
       } else {
         qoff[q] = -1;
@@ -1228,20 +1273,25 @@ __global__ void __launch_bounds__(kCfThreads)
   }
   __syncthreads();
   // coupling between different clusters must be negligible
-  double mx = 0.0;
-  for (size_t e = tid; e < size_t(n) * n; e += nt) {
-    const int i = int(e % n), j = int(e / n);
-    if (cid[i] != cid[j]) mx = fmax(mx, fabs(S[e]));
+  unsigned long long mx = 0;
+  for (int e = rank * nt + tid; e < n * n; e += kRlCtas * nt) {
+    const int j = e / n, i = e - j * n;
+    if (cid[i] != cid[j]) mx = max(mx, abs_key(S[e]));
   }
-  for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+  for (int o = 16; o > 0; o >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
   if (lane == 0) red[warp] = mx;
   __syncthreads();
-  // X orthonormal and X^T A X block diagonal over clusters <=> invariant subspaces
   if (tid == 0) {
-    double m2 = 0.0;
-    for (int w2 = 0; w2 < nwarp; ++w2) m2 = fmax(m2, red[w2]);
-    if (m2 > 1.0e-12 * fmax(nA, 1e-300)) fail |= 1;  // clusters still coupled
-    if (rscal[3] > 1.0e-12 * sqrt(double(n))) fail |= 2;  // not orthonormal
+    for (int w2 = 1; w2 < nwarp; ++w2) mx = max(mx, red[w2]);
+    *cluster.map_shared_rank(&gathered[rank], 0) = mx;
+  }
+  cluster.sync();
+  // X orthonormal and X^T A X block diagonal over clusters <=> invariant subspaces
+  if (rank == 0 && tid == 0) {
+    unsigned long long m2 = 0;
+    for (int q = 0; q < kRlCtas; ++q) m2 = max(m2, gathered[q]);
+    if (!(__longlong_as_double(static_cast<long long>(m2)) <= 1.0e-12 * fmax(nA, 1e-300))) fail |= 1;  // still coupled
+    if (!(rscal[3] <= 1.0e-12 * sqrt(double(n)))) fail |= 2;  // not orthonormal
   }
   for (int c = tid; c < ncl; c += nt) {
     const int k0 = cl_start[c], m = cl_start[c + 1] - k0;
@@ -1260,7 +1310,7 @@ __global__ void __launch_bounds__(kCfThreads)
     }
   }
   __syncthreads();
-  for (int c = warp; c < ncl; c += nwarp) {
+  for (int c = rank * nwarp + warp; c < ncl; c += kRlCtas * nwarp) {
     const int k0 = cl_start[c], m = cl_start[c + 1] - k0;
     if (qoff[c] < 0) {
       // left to the FP64 Jacobi of the block (or the attempt fails): the
@@ -1283,8 +1333,7 @@ __global__ void __launch_bounds__(kCfThreads)
       }
     }
   }
-  __syncthreads();
-  if (tid == 0) {
+  if (rank == 0 && tid == 0) {
     rflag[0] = fail;
     rflag[2] = nbig;
     rflag[3] = 0;
@@ -2413,9 +2462,9 @@ int refine_canonical(tvap_ctx* c, double* X, double* Xn, int steps, int* fail, c
   for (int step = 0; step < steps; ++step) {
     const View Xv = view_cm(X, n, 0);
     if ((rc = gram(X))) return rc;
-    refine_lambda_kernel<<<1, kRlThreads, 0, tvap::counted(s)>>>(n, w->Rr, w->Sr, w->rho, w->lam, w->rscal);
+    refine_lambda_kernel<<<kRlCtas, kRlThreads, 0, tvap::counted(s)>>>(n, w->Rr, w->Sr, w->rho, w->lam, w->rscal);
     if (step == 0 && assign)
-      cluster_assign_kernel<<<1, kCfThreads, 0, tvap::counted(s)>>>(n, w->Sr, w->lam, w->rscal, w->cid);
+      cluster_assign_kernel<<<kRlCtas, kCfThreads, 0, tvap::counted(s)>>>(n, w->Sr, w->lam, w->rscal, w->cid);
     refine_update_kernel<<<nblk(nn, 256), 256, 0, tvap::counted(s)>>>(n, w->Rr, w->Sr, w->lam, w->rscal, w->cid,
                                                                       w->Mr, w->Br);
     if (second_order) {
@@ -2426,8 +2475,8 @@ int refine_canonical(tvap_ctx* c, double* X, double* Xn, int steps, int* fail, c
     std::swap(X, Xn);
   }
   if ((rc = gram(X))) return rc;
-  refine_lambda_kernel<<<1, kRlThreads, 0, tvap::counted(s)>>>(n, w->Rr, w->Sr, w->rho, w->lam, w->rscal);
-  cluster_finish_kernel<<<1, kCfThreads, 0, tvap::counted(s)>>>(n, w->Sr, X, w->rscal, w->cid, w->D, w->evals,
+  refine_lambda_kernel<<<kRlCtas, kRlThreads, 0, tvap::counted(s)>>>(n, w->Rr, w->Sr, w->rho, w->lam, w->rscal);
+  cluster_finish_kernel<<<kRlCtas, kCfThreads, 0, tvap::counted(s)>>>(n, w->Sr, X, w->rscal, w->cid, w->D, w->evals,
                                                                  w->cperm, w->bigd, w->rflag);
   TVAP_CUDA(cudaGetLastError());
   int hr[3] = {1, 0, 0};
