@@ -1678,89 +1678,105 @@ __global__ void __launch_bounds__(kFactorThreads)
 }
 
 // Panel of the blocked Gauss-Jordan solve (GEMM modes 1 and 2), one CTA per
-// angle.  The pivot rows are chosen by a single-precision Crout elimination
-// of the panel rows j0 .. n-1 with partial pivoting (first maximum of
-// |re| + |im|, as izamax): warp w holds columns w, w + 8, w + 16, w + 24,
-// lane l rows l, l + 32, ... (SLOTS rows a lane); one barrier per column
-// (before it the pivot column's warp finds and swaps the pivot row and forms
-// its reciprocal; after it the other warps swap the rows, every warp scales
-// its entries of the pivot row and updates its columns).  Only the choice of
-// rows comes from single precision: the block A11 of the chosen rows is then
-// inverted in FP64 from the original values by Gauss-Jordan elimination
-// without further interchanges (its pivots are the partial-pivoting pivots),
-// T = A11^{-1} written to Tinv + b * tstride (nbp x nbp, column-major).  The
-// panel columns of W are rewritten for the elimination product: the block
-// rows j0 .. j0+nbp-1 as zeros, the rows below with their original values in
-// the pivoted order.  The other columns' interchanges are left to
-// panel_swap_kernel.
+// angle.  The pivot rows are chosen by a single-precision elimination of the
+// panel rows j0 .. n-1 with partial pivoting (first maximum of |re| + |im|):
+// warp w holds columns w, w + 8, w + 16, w + 24, lane l rows l, l + 32, ...
+// (SLOTS rows a lane).  Only the choice of rows comes from single precision:
+// the block A11 of the chosen rows is then inverted in FP64 from the original
+// values by Gauss-Jordan elimination without further interchanges (its pivots
+// are the partial-pivoting pivots), a column a warp and a row a lane as
+// before, T = A11^{-1} written to Tinv + b * tstride (nbp x nbp,
+// column-major).  The panel columns of W are rewritten for the elimination
+// product: the block rows j0 .. j0+nbp-1 as zeros, the rows below with their
+// original values in the new order, src[b * n + j0 + r] = the row (from j0)
+// that is row r of it; the other columns follow in panel_perm_kernel.
+//
+// The chain of steps bounds it, then the FP64 pipe (nbp^3 complex updates at
+// two FMAs a clock: 23 us of 28 columns).  So a step is handed on as early as
+// it can be: the warp of column k + 1 brings that column up to step k, forms
+// the multipliers of step k + 1 and posts them (one mbarrier a step), and
+// only then updates its other columns; no warp waits for the slowest.  Rows
+// are never moved (a used row is left out by a zero multiplier).  An
+// inverting step is one complex FMA per entry: the multiplier of the pivot
+// row is its reciprocal, with the old entry taken as zero.  57 angles at
+// n = 140, first panel (140 x 28) 139 -> 52 us, last (28 x 28) 93 -> 45, of
+// which the FP64 inverse takes about 30.
 __device__ __forceinline__ float2 shfl_f2(float2 v, int src) {
   return make_float2(__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src));
 }
-
-// first maximum over the warp, the result in every lane
-__device__ __forceinline__ void warp_argmax_key_all(int& v, int& i) {
-  for (int off = 16; off > 0; off >>= 1) {
-    const int v2 = __shfl_xor_sync(0xffffffffu, v, off);
-    const int i2 = __shfl_xor_sync(0xffffffffu, i, off);
-    if (v2 > v || (v2 == v && i2 < i)) {
-      v = v2;
-      i = i2;
-    }
-  }
+__device__ __forceinline__ double2 shfl_d2(double2 v, int src) {
+  return make_double2(__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src));
 }
 
 template <int SLOTS>
 __device__ __forceinline__ float2 slot_get(const float2 (&a)[SLOTS], int s) {
-  float2 v = a[0];
+  float x = a[0].x, y = a[0].y;
 #pragma unroll
-  for (int k = 1; k < SLOTS; ++k)
-    if (k == s) v = a[k];
-  return v;
-}
-
-template <int SLOTS>
-__device__ __forceinline__ void slot_set(float2 (&a)[SLOTS], int s, float2 v) {
-#pragma unroll
-  for (int k = 0; k < SLOTS; ++k)
-    if (k == s) a[k] = v;
-}
-
-// exchange rows r1 != r2 of a column held as a[slot] in lanes
-template <int SLOTS>
-__device__ __forceinline__ void swap_rows(float2 (&a)[SLOTS], int r1, int r2, int lane) {
-  const float2 v1 = shfl_f2(slot_get(a, r1 >> 5), r1 & 31);
-  const float2 v2 = shfl_f2(slot_get(a, r2 >> 5), r2 & 31);
-  if (lane == (r1 & 31)) slot_set(a, r1 >> 5, v2);
-  if (lane == (r2 & 31)) slot_set(a, r2 >> 5, v1);
+  for (int k = 1; k < SLOTS; ++k) {
+    const float2 v = a[k];
+    x = k == s ? v.x : x;
+    y = k == s ? v.y : y;
+  }
+  return make_float2(x, y);
 }
 
 __device__ __forceinline__ float2 fcmul(float2 a, float2 b) {
   return make_float2(fmaf(a.x, b.x, -a.y * b.y), fmaf(a.x, b.y, a.y * b.x));
 }
 
+// -z by the sign bits (a negation of its own is an FP64 operation)
+__device__ __forceinline__ double2 flip_sign(double2 z) {
+  const long long sign = 1LL << 63;
+  return make_double2(__longlong_as_double(__double_as_longlong(z.x) ^ sign),
+                      __longlong_as_double(__double_as_longlong(z.y) ^ sign));
+}
+
+// a posted step: an mbarrier of one arrival, used for one phase
+__device__ __forceinline__ uint32_t step_addr(const uint64_t* bar) {
+  return static_cast<uint32_t>(__cvta_generic_to_shared(bar));
+}
+__device__ __forceinline__ void step_post(uint64_t* bar) {
+  asm volatile("{\n.reg .b64 st;\nmbarrier.arrive.shared::cta.b64 st, [%0];\n}\n" ::"r"(step_addr(bar)) : "memory");
+}
+// bounded (a step is posted within a few microseconds)
+__device__ __forceinline__ bool step_wait(const uint64_t* bar) {
+  for (int it = 0; it < (1 << 16); ++it) {
+    uint32_t done;
+    asm volatile(
+        "{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], 0;\nselp.u32 %0, 1, 0, p;\n}\n"
+        : "=r"(done)
+        : "r"(step_addr(bar))
+        : "memory");
+    if (done) return true;
+  }
+  return false;
+}
+
 constexpr int kGjMaxSlots = 12;  // panels of up to 384 rows
-constexpr int kGjEntries = (kPanelMax * kPanelMax + kFactorThreads - 1) / kFactorThreads;  // block entries per thread
+// Multipliers of single-precision steps kept: a warp that posts step k + 9 is
+// the warp that posted k + 1, and the seven others have posted steps k + 2
+// .. k + 8, each after its last use of step k; nobody reads step k any more.
+constexpr int kGjRing = 9;
 
 template <int SLOTS>
 __global__ void __launch_bounds__(kFactorThreads)
-    panel_gj_kernel(int n, int j0, int nbp, double2* __restrict__ Wall, int* __restrict__ piv, int* flags,
+    panel_gj_kernel(int n, int j0, int nbp, double2* __restrict__ Wall, int* __restrict__ src, int* flags,
                     double2* __restrict__ Tinv, long long tstride) {
   constexpr int kQ = kPanelMax / 8;
-  constexpr int kP = kPanelMax + 1;
-  static_assert(kFactorThreads == 256 && kPanelMax % 8 == 0, "eight warps hold the panel's columns");
-  __shared__ float2 scol[2][32 * SLOTS];
-  __shared__ float2 s_rp[2];
-  __shared__ int s_piv[2];
-  __shared__ int s_sing;
+  static_assert(kFactorThreads == 256 && kPanelMax == 32, "eight warps hold the columns, a lane a row of the block");
+  __shared__ float2 scol[kGjRing][32 * SLOTS];
+  __shared__ int s_piv[kPanelMax];
   __shared__ int srow[32 * SLOTS];
-  __shared__ double2 A11[kPanelMax * kP];
-  __shared__ double2 smu[kPanelMax], srk[kPanelMax];
-  __shared__ double2 s_rd[2];
+  __shared__ double2 smu[kPanelMax][32];
+  __shared__ uint64_t posted[2][kPanelMax];
+  __shared__ int s_sing, s_late;
   const int b = blockIdx.x;
   double2* W = Wall + size_t(b) * 2 * n * n;
   const int m = n - j0;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  if (tid == 0) s_sing = 0;
+  if (tid == 0) s_sing = s_late = 0;
+  if (tid < 2 * kPanelMax)
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(step_addr(&posted[0][0] + tid)) : "memory");
   for (int r = tid; r < 32 * SLOTS; r += kFactorThreads) srow[r] = r;
   float2 a[kQ][SLOTS];
 #pragma unroll
@@ -1775,101 +1791,120 @@ __global__ void __launch_bounds__(kFactorThreads)
     }
   }
   __syncthreads();
-  for (int jj = 0; jj < nbp; ++jj) {
-    const int buf = jj & 1, wj = jj & 7, qj = jj >> 3;
-    if (warp == wj) {
-      int best = -1, bi = m;
-#pragma unroll
-      for (int q = 0; q < kQ; ++q)
-        if (q == qj) {
-#pragma unroll
-          for (int s = 0; s < SLOTS; ++s) {
-            const int r = lane + 32 * s;
-            if (r >= jj && r < m) {
-              const int v = __float_as_int(fabsf(a[q][s].x) + fabsf(a[q][s].y));
-              if (v > best) {
-                best = v;
-                bi = r;
-              }
-            }
-          }
-        }
-      warp_argmax_key_all(best, bi);
-      const bool zero = best <= 0;
-      const int p = zero ? jj : bi;
-      if (p != jj) {
-#pragma unroll
-        for (int q = 0; q < kQ; ++q) swap_rows(a[q], jj, p, lane);
-      }
-      float2 pv = make_float2(0.f, 0.f);
-#pragma unroll
-      for (int q = 0; q < kQ; ++q)
-        if (q == qj) {
-          pv = shfl_f2(slot_get(a[q], jj >> 5), jj & 31);
-#pragma unroll
-          for (int s = 0; s < SLOTS; ++s) {
-            const int r = lane + 32 * s;
-            if (r > jj && r < m) scol[buf][r] = a[q][s];
-          }
-        }
-      if (lane == 0) {
-        const float d = fmaf(pv.x, pv.x, pv.y * pv.y);
-        const float rd = (zero || !(d > 0.f)) ? 0.f : __frcp_rn(d);
-        s_rp[buf] = make_float2(pv.x * rd, -pv.y * rd);
-        s_piv[buf] = p;
-        piv[size_t(b) * n + j0 + jj] = j0 + p;
-        const int t0 = srow[jj];
-        srow[jj] = srow[p];
-        srow[p] = t0;
-        if (zero) s_sing = 1;
-      }
-    }
-    __syncthreads();
-    if (warp != wj) {
-      const int p = s_piv[buf];
-      if (p != jj) {
-#pragma unroll
-        for (int q = 0; q < kQ; ++q) swap_rows(a[q], jj, p, lane);
-      }
-    }
-    const float2 rp = s_rp[buf];
-    float2 mu[SLOTS];
+  unsigned used = 0;  // slots of this lane whose row is a pivot row
+  // the pivot of column j (held in t, up to date), its multipliers
+  auto post = [&](const float2 (&t)[SLOTS], int j) {
+    int best = -1, bi = 32 * SLOTS;
 #pragma unroll
     for (int s = 0; s < SLOTS; ++s) {
       const int r = lane + 32 * s;
-      mu[s] = (r > jj && r < m) ? scol[buf][r] : make_float2(0.f, 0.f);
+      const int v = __float_as_int(fabsf(t[s].x) + fabsf(t[s].y)) & 0x7fffffff;  // a NaN: large
+      if (r < m && !(used >> s & 1) && v > best) {
+        best = v;
+        bi = r;
+      }
+    }
+    // j < nbp <= m rows are used: some lane has a row left
+    const int top = __reduce_max_sync(0xffffffffu, best);
+    const int p = __reduce_min_sync(0xffffffffu, best == top ? bi : 32 * SLOTS);
+    const float2 pv = shfl_f2(slot_get(t, p >> 5), p & 31);
+    if (lane == (p & 31)) used |= 1u << (p >> 5);
+    const float d = fmaf(pv.x, pv.x, pv.y * pv.y);
+    const float rd = (top <= 0 || !(d > 0.f)) ? 0.f : __frcp_rn(d);
+    const float2 rp = make_float2(pv.x * rd, -pv.y * rd);
+    float2* out = scol[j % kGjRing];
+#pragma unroll
+    for (int s = 0; s < SLOTS; ++s) out[lane + 32 * s] = (used >> s & 1) ? make_float2(0.f, 0.f) : fcmul(t[s], rp);
+    if (lane == 0) {
+      s_piv[j] = p;
+      if (top <= 0) s_sing = 1;
+    }
+    __syncwarp();
+    if (lane == 0) step_post(&posted[0][j]);
+  };
+  bool ok = true;
+  for (int jj = -1; jj + 1 < nbp; ++jj) {  // step -1: column 0 as it is
+    const int jn = jj + 1;
+    int ps = 0, pl = 0;
+    float2 mu[SLOTS];
+#pragma unroll
+    for (int s = 0; s < SLOTS; ++s) mu[s] = make_float2(0.f, 0.f);
+    if (jj >= 0) {
+      if (!(ok = step_wait(&posted[0][jj]))) break;
+      const int p = s_piv[jj];
+      ps = p >> 5;
+      pl = p & 31;
+      if (lane == pl) used |= 1u << ps;
+#pragma unroll
+      for (int s = 0; s < SLOTS; ++s) mu[s] = scol[jj % kGjRing][lane + 32 * s];
+    }
+    auto update = [&](float2 (&t)[SLOTS]) {
+      const float2 u = shfl_f2(slot_get(t, ps), pl);
+#pragma unroll
+      for (int s = 0; s < SLOTS; ++s) {
+        t[s].x = fmaf(-mu[s].x, u.x, fmaf(mu[s].y, u.y, t[s].x));
+        t[s].y = fmaf(-mu[s].x, u.y, fmaf(-mu[s].y, u.x, t[s].y));
+      }
+    };
+    if (warp == (jn & 7)) {
+      float2 t[SLOTS];
+#pragma unroll
+      for (int s = 0; s < SLOTS; ++s) {  // (a copy per column, then a selection: registers, no indexing)
+        float2 x = a[0][s];
+#pragma unroll
+        for (int q = 1; q < kQ; ++q) {
+          const float2 y = a[q][s];
+          x = q == jn >> 3 ? y : x;
+        }
+        t[s] = x;
+      }
+      if (jj >= 0) update(t);
+      post(t, jn);
     }
 #pragma unroll
     for (int q = 0; q < kQ; ++q) {
       const int c = warp + 8 * q;
-      if (c <= jj || c >= nbp) continue;
-      // U' entry of the pivot row, then the column update
-      const float2 u = fcmul(shfl_f2(slot_get(a[q], jj >> 5), jj & 31), rp);
-      if (lane == (jj & 31)) slot_set(a[q], jj >> 5, u);
-#pragma unroll
-      for (int s = 0; s < SLOTS; ++s)
-        if (32 * s + 31 > jj) {
-          a[q][s].x = fmaf(-mu[s].x, u.x, fmaf(mu[s].y, u.y, a[q][s].x));
-          a[q][s].y = fmaf(-mu[s].x, u.y, fmaf(-mu[s].y, u.x, a[q][s].y));
-        }
+      if (jj >= 0 && c > jn && c < nbp) update(a[q]);
     }
   }
-  // the original rows in the pivoted order: the block to shared memory, the
-  // rows below back to the panel (the block rows as zeros).  A column
-  // belongs to one warp, so the permutation in place needs only that warp's
-  // reads before its writes (one column of rows in registers at a time).
-  __syncthreads();  // srow is complete
+  if (!ok) s_late = 1;
+  __syncthreads();
+  if (s_late) {  // uniform
+    if (tid == 0) atomicOr(flags, DEV_WAIT_TIMEOUT);
+    return;
+  }
+  // the new order: the pivot rows first; the other rows among the first nbp
+  // take the places that pivot rows left further down
+  if (warp == 0) {
+    const int p = lane < nbp ? s_piv[lane] : -1;
+    const unsigned stay = __reduce_or_sync(0xffffffffu, (p >= 0 && p < nbp) ? 1u << p : 0u);
+    const unsigned below = __ballot_sync(0xffffffffu, p >= nbp);
+    unsigned displaced = ~stay & (0xffffffffu >> (32 - nbp));
+    if (p >= nbp) {
+      for (int k = __popc(below & ((1u << lane) - 1)); k > 0; --k) displaced &= displaced - 1;
+      srow[p] = __ffs(displaced) - 1;
+    }
+    if (lane < nbp) srow[lane] = p;
+  }
+  __syncthreads();
+  for (int r = tid; r < m; r += kFactorThreads) src[size_t(b) * n + j0 + r] = srow[r];
+  // the original rows in the new order: the block to registers, the rows
+  // below back to the panel (the block rows as zeros).  A column belongs to
+  // one warp, so the permutation in place needs only that warp's reads
+  // before its writes (one column of rows in registers at a time).
+  double2 v[kQ];
 #pragma unroll
   for (int q = 0; q < kQ; ++q) {
     const int c = warp + 8 * q;
+    v[q] = make_double2(0.0, 0.0);
     if (c >= nbp) continue;
     double2 raw[SLOTS];
 #pragma unroll
     for (int s = 0; s < SLOTS; ++s) {
       const int r = lane + 32 * s;
       raw[s] = (r < m) ? W[(j0 + srow[r]) + size_t(j0 + c) * n] : make_double2(0.0, 0.0);
-      if (r < nbp) A11[r + c * kP] = raw[s];
     }
+    if (lane < nbp) v[q] = raw[0];
     __syncwarp();
 #pragma unroll
     for (int s = 0; s < SLOTS; ++s) {
@@ -1877,52 +1912,57 @@ __global__ void __launch_bounds__(kFactorThreads)
       if (r < m) W[(j0 + r) + size_t(j0 + c) * n] = (r < nbp) ? make_double2(0.0, 0.0) : raw[s];
     }
   }
-  __syncthreads();
   if (s_sing && tid == 0) atomicOr(flags, DEV_SINGULAR_UPHI);
-  // Gauss-Jordan inverse of the block in place: step k with the reciprocal
-  // of the pivot (formed by the owner of that entry at the end of the step
-  // before), multipliers and the pivot row staged, then every entry at once
-  if (tid == 0) s_rd[0] = crcp_newton(A11[0]);
-  // entries of the nbp x nbp block, kGjEntries per thread (ei = nbp: none)
-  int ei[kGjEntries], ej[kGjEntries];
-#pragma unroll
-  for (int e = 0; e < kGjEntries; ++e) {
-    const int idx = tid + e * kFactorThreads;
-    const bool in = idx < nbp * nbp;
-    ei[e] = in ? idx % nbp : nbp;
-    ej[e] = in ? idx / nbp : 0;
-  }
-  __syncthreads();
+  // Gauss-Jordan inverse of the block: the negative multipliers of step k and
+  // the reciprocal of its pivot are column k of the result so far
+  auto invert = [&](double2 t, int k) {
+    const double2 rd = crcp_newton(shfl_d2(t, k));
+    double2 mk = cmul(t, flip_sign(rd));
+    if (lane == k) mk = rd;
+    if (lane >= nbp) mk = make_double2(0.0, 0.0);
+    smu[k][lane] = mk;
+    __syncwarp();
+    if (lane == 0) step_post(&posted[1][k]);
+    return mk;
+  };
+  if (warp == 0) v[0] = invert(v[0], 0);
   for (int k = 0; k < nbp; ++k) {
-    const double2 rd = s_rd[k & 1];
-    if (tid < nbp) {
-      smu[tid] = (tid == k) ? make_double2(0.0, 0.0) : cmul(A11[tid + k * kP], rd);
-      srk[tid] = A11[k + tid * kP];
-    }
-    __syncthreads();
-    double2 v[kGjEntries];
+    const int kn = k + 1;
+    if (!(ok = step_wait(&posted[1][k]))) break;
+    const double2 mk = smu[k][lane];
+    auto update = [&](double2 t) {
+      const double2 r = shfl_d2(t, k);
+      if (lane == k) t = make_double2(0.0, 0.0);
+      cfma(t, mk, r);
+      return t;
+    };
+    if (warp == (kn & 7) && kn < nbp) {
+      double2 t = v[0];
 #pragma unroll
-    for (int e = 0; e < kGjEntries; ++e) v[e] = (ei[e] < nbp) ? A11[ei[e] + ej[e] * kP] : make_double2(0.0, 0.0);
-#pragma unroll
-    for (int e = 0; e < kGjEntries; ++e) {
-      const int i = ei[e], j = ej[e];
-      if (i >= nbp) continue;
-      if (i != k && j != k) {
-        cfma(v[e], cneg(smu[i]), srk[j]);
-      } else if (i == k && j != k) {
-        v[e] = cmul(srk[j], rd);
-      } else if (i != k) {
-        v[e] = cneg(smu[i]);
-      } else {
-        v[e] = rd;
+      for (int q = 1; q < kQ; ++q) {
+        const double2 vq = v[q];
+        t = q == kn >> 3 ? vq : t;
       }
-      A11[i + j * kP] = v[e];
-      if (i == k + 1 && j == k + 1) s_rd[(k + 1) & 1] = crcp_newton(v[e]);
+      t = invert(update(t), kn);
+#pragma unroll
+      for (int q = 0; q < kQ; ++q) {
+        v[q].x = q == kn >> 3 ? t.x : v[q].x;
+        v[q].y = q == kn >> 3 ? t.y : v[q].y;
+      }
     }
-    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < kQ; ++q) {
+      const int c = warp + 8 * q;
+      if (c < nbp && c != k && c != kn) v[q] = update(v[q]);
+    }
   }
+  if (!ok && lane == 0) atomicOr(flags, DEV_WAIT_TIMEOUT);
   double2* T = Tinv + size_t(b) * tstride;
-  for (int idx = tid; idx < nbp * nbp; idx += kFactorThreads) T[idx] = A11[(idx % nbp) + (idx / nbp) * kP];
+#pragma unroll
+  for (int q = 0; q < kQ; ++q) {
+    const int c = warp + 8 * q;
+    if (c < nbp && lane < nbp) T[lane + c * nbp] = v[q];
+  }
 }
 
 // Row interchanges of a factored panel applied to columns j1 .. 2n-1 (one
@@ -1944,51 +1984,36 @@ __global__ void __launch_bounds__(kApplyThreads)
   }
 }
 
-// The same interchanges for 32 columns per CTA: the pivot sequence is first
-// composed into a permutation of rows j0 .. n-1 (row r after = row src[r]
-// before; at most 2 nbp rows move), then the moved rows are read with
-// independent loads and written back, instead of one dependent pair of
-// accesses per interchange and column.
+// The row order of a Gauss-Jordan panel applied to columns j1 .. 2n-1, 32
+// columns per CTA: row j0 + r takes row j0 + order[b * n + j0 + r].  At most 2
+// nbp rows move; they are read with independent loads and written back.
 constexpr int kPermCols = 32;
 constexpr int kPermThreads = 256;
-constexpr int kPermMaxRows = 1024;
 __global__ void __launch_bounds__(kPermThreads)
-    panel_perm_kernel(int n, int j0, int nbp, double2* __restrict__ Wall, const int* __restrict__ piv) {
-  __shared__ int src[kPermMaxRows];
-  __shared__ int moved[2 * kPanelMax];
+    panel_perm_kernel(int n, int j0, int nbp, double2* __restrict__ Wall, const int* __restrict__ order) {
+  __shared__ int2 moved[2 * kPanelMax];
   __shared__ int nmoved;
   __shared__ double2 buf[2 * kPanelMax][kPermCols];
   const int b = blockIdx.y, t = threadIdx.x;
   const int m = n - j0, j1 = j0 + nbp;
   double2* W = Wall + size_t(b) * 2 * n * n;
-  for (int r = t; r < m; r += kPermThreads) src[r] = r;
   if (t == 0) nmoved = 0;
   __syncthreads();
-  if (t == 0) {
-    const int* pv = piv + size_t(b) * n + j0;
-    for (int jj = 0; jj < nbp; ++jj) {
-      const int p = pv[jj] - j0;
-      if (p != jj) {
-        const int x = src[jj];
-        src[jj] = src[p];
-        src[p] = x;
-      }
-    }
+  for (int r = t; r < m; r += kPermThreads) {
+    const int q = order[size_t(b) * n + j0 + r];
+    if (q != r) moved[atomicAdd(&nmoved, 1)] = make_int2(r, q);
   }
-  __syncthreads();
-  for (int r = t; r < m; r += kPermThreads)
-    if (src[r] != r) moved[atomicAdd(&nmoved, 1)] = r;
   __syncthreads();
   const int nm = nmoved;
   const int c0 = j1 + blockIdx.x * kPermCols;
   for (int idx = t; idx < nm * kPermCols; idx += kPermThreads) {
-    const int k = idx / kPermCols, cc = idx - k * kPermCols, c = c0 + cc;
-    if (c < 2 * n) buf[k][cc] = W[(j0 + src[moved[k]]) + size_t(c) * n];
+    const int k = idx % nm, cc = idx / nm, c = c0 + cc;
+    if (c < 2 * n) buf[k][cc] = W[(j0 + moved[k].y) + size_t(c) * n];
   }
   __syncthreads();
   for (int idx = t; idx < nm * kPermCols; idx += kPermThreads) {
-    const int k = idx / kPermCols, cc = idx - k * kPermCols, c = c0 + cc;
-    if (c < 2 * n) W[(j0 + moved[k]) + size_t(c) * n] = buf[k][cc];
+    const int k = idx % nm, cc = idx / nm, c = c0 + cc;
+    if (c < 2 * n) W[(j0 + moved[k].x) + size_t(c) * n] = buf[k][cc];
   }
 }
 
@@ -2219,13 +2244,8 @@ int gj_solve_range(tvap_ctx* c, int g0, int gc, int nb, cudaStream_t s, cudaEven
     // interchanges touch its columns
     if (sb && j0 > 0) TVAP_CUDA(cudaStreamWaitEvent(s, ev_bulk, 0));
     if (j1 < 2 * n) {
-      if (n - j0 <= kPermMaxRows) {
-        dim3 gp((2 * n - j1 + kPermCols - 1) / kPermCols, gc);
-        panel_perm_kernel<<<gp, kPermThreads, 0, tvap::counted(s)>>>(n, j0, nbp, W, piv);
-      } else {
-        dim3 ga((2 * n - j1 + kApplyThreads - 1) / kApplyThreads, gc);
-        panel_swap_kernel<<<ga, kApplyThreads, 0, tvap::counted(s)>>>(n, j0, nbp, W, piv);
-      }
+      dim3 gp((2 * n - j1 + kPermCols - 1) / kPermCols, gc);
+      panel_perm_kernel<<<gp, kPermThreads, 0, tvap::counted(s)>>>(n, j0, nbp, W, piv);
     }
     // the block row: R = T [A12 | B1] in place (the operands are split into
     // digit planes before the product is formed)
