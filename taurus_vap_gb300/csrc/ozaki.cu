@@ -191,86 +191,116 @@ struct TcSrc {
   double scale2;
 };
 
-// Digit planes of X' in the tiled layout of ozaki_tc.cuh.  One CTA per 8
-// source rows of one slot: the rows are gathered into shared memory
+// One operand of the slicing launch: its digit planes and exponents, the rows
+// of a tile (a power of two) and the CTAs that it takes.
+struct TcSlice {
+  TcSrc x;
+  int tile_shift, rows_pad, blocks;
+  __nv_bfloat16* out;
+  int* ex;
+};
+
+// Digit planes of the X' of both operands in the tiled layout of
+// ozaki_tc.cuh; the tile counter of the product that follows is zeroed here.
+// One CTA per R = 2^rshift source rows of one slot (the first a.blocks CTAs of
+// a slot take the left operand): the rows are gathered into shared memory
 // (independent loads, consecutive threads on the source's contiguous index),
-// one warp per row takes the exponents, then every thread converts 8
+// 256 / R threads a row take the exponents, then every thread converts 8
 // consecutive k of one part (real or imaginary) of one row to 7 digits and
 // stores one 16-byte core-matrix row per digit at each place of X' that
 // holds them (twice in form 2: the imaginary block negated by its sign bits;
 // once in form 4, whose left operand is half the size of form 2's).
+//
+// Instructions bound it, then the latency of three phases: so the divisions
+// are multiplications or shifts, a row's address is formed once, and a CTA has
+// the rows that give every thread a conversion (slice_rshift).  57 slots of
+// 256 rows of 28 complex k: 13.2 -> 8 us.
 constexpr int kSliceThreads = 256;
-__global__ void __launch_bounds__(kSliceThreads) slice_tc_kernel(TcSrc x, int tile_rows, int rows_pad, int nks,
-                                                                  __nv_bfloat16* __restrict__ out,
-                                                                  int* __restrict__ ex) {
-  // 8 rows of ldk = K | 1 elements (real sources use .x): an odd row stride,
-  // so that the 8 rows read by 8 consecutive threads (one 16-byte element
-  // each) fall in 8 different groups of 4 banks
+constexpr int kSliceMaxRows = 32;
+__global__ void __launch_bounds__(kSliceThreads)
+    slice_tc_kernel(const __grid_constant__ TcSlice a, const __grid_constant__ TcSlice b, int rshift, unsigned kmagic,
+                    int nks, int* counter) {
+  // R rows of ldk = K | 1 elements (real sources use .x): an odd row stride,
+  // so that 8 rows read by neighbouring threads fall in 8 different groups of
+  // 4 banks
   extern __shared__ double2 xs[];
-  __shared__ int e_s[8][2];        // exponent of the real / imaginary part
-  const int t = threadIdx.x;
-  const int K = x.K, form = x.form;
+  __shared__ int e_s[kSliceMaxRows][2];  // exponent of the real / imaginary part
+  __shared__ long long off_s[kSliceMaxRows][2];
+  if (counter && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *counter = 0;
+  const bool left = int(blockIdx.x) < a.blocks;
+  const TcSlice& job = left ? a : b;
+  const TcSrc& x = job.x;
+  const int t = threadIdx.x, R = 1 << rshift;
+  const int K = x.K, K1 = x.K1, form = x.form;
   const int ldk = K | 1;
   const bool cplx = form != 0;
-  const int sq0 = blockIdx.x * 8;
+  const int sq0 = (left ? int(blockIdx.x) : int(blockIdx.x) - a.blocks) << rshift;
   const int slot = blockIdx.y;
-  const int nsrc = x.nstack * x.rows;
+  const int nrows = min(R, x.nstack * x.rows - sq0);
   const int mult = (form == 1 || form == 2 || form == 4) ? 2 : 1;  // rows of X' per source row
-  auto src_row = [&](int row, int& b, int& i) {
-    const int sq = sq0 + row;
-    if (x.nstack == 1) {
-      b = slot;
-      i = sq;
-    } else if (x.bfast) {
-      i = sq / x.nstack;
-      b = sq - i * x.nstack;
-    } else {
-      b = sq / x.rows;
-      i = sq - b * x.rows;
-    }
-  };
-  const bool k_fast = (x.sk == 1);
-#pragma unroll 4
-  for (int idx = t; idx < 8 * K; idx += kSliceThreads) {
-    int row, k;
-    if (k_fast) {
-      row = idx / K;
-      k = idx - row * K;
-    } else {
-      row = idx & 7;
-      k = idx >> 3;
-    }
-    double2 v = make_double2(0.0, 0.0);
-    if (sq0 + row < nsrc) {
-      int b, i;
-      src_row(row, b, i);
-      const bool second = k >= x.K1;
-      const long long off = second ? b * x.bs2 + i * x.sr2 + (k - x.K1) * x.sk2 : b * x.bs + i * x.sr + k * x.sk;
-      const void* P = second ? x.p2 : x.p;
-      if (cplx) {
-        v = static_cast<const double2*>(P)[off];
-        if (x.conj) v.y = -v.y;
+  if (t < nrows) {
+    const int sq = sq0 + t;
+    int bb = slot, i = sq;
+    if (x.nstack > 1) {
+      if (x.bfast) {
+        i = sq / x.nstack;
+        bb = sq - i * x.nstack;
       } else {
-        v.x = static_cast<const double*>(P)[off];
-      }
-      if (second) {
-        v.x *= x.scale2;
-        v.y *= x.scale2;
+        bb = sq / x.rows;
+        i = sq - bb * x.rows;
       }
     }
-    xs[row * ldk + k] = v;
+    off_s[t][0] = bb * x.bs + i * x.sr;
+    off_s[t][1] = bb * x.bs2 + i * x.sr2;
   }
   __syncthreads();
   {
-    const int w = t >> 5, lane = t & 31;
+    const bool k_fast = x.sk == 1, conj = x.conj;
+    const long long sk = x.sk;
+#pragma unroll 4
+    for (int idx = t; idx < K << rshift; idx += kSliceThreads) {
+      int row, k;
+      if (k_fast) {
+        row = K > 1 ? int(__umulhi(unsigned(idx), kmagic)) : idx;  // idx / K (exact: idx K < 2^32)
+        k = idx - row * K;
+      } else {
+        row = idx & (R - 1);
+        k = idx >> rshift;
+      }
+      if (row >= nrows) continue;
+      double2 v = make_double2(0.0, 0.0);
+      if (k < K1) {
+        const long long off = off_s[row][0] + k * sk;
+        if (cplx)
+          v = static_cast<const double2*>(x.p)[off];
+        else
+          v.x = static_cast<const double*>(x.p)[off];
+      } else {
+        const long long off = off_s[row][1] + (k - K1) * x.sk2;
+        if (cplx)
+          v = static_cast<const double2*>(x.p2)[off];
+        else
+          v.x = static_cast<const double*>(x.p2)[off];
+        v.x *= x.scale2;
+        v.y *= x.scale2;
+      }
+      if (conj) v.y = __longlong_as_double(__double_as_longlong(v.y) ^ (1LL << 63));
+      xs[row * ldk + k] = v;
+    }
+  }
+  __syncthreads();
+  {
+    const int tpr = kSliceThreads >> rshift;  // threads of a row: 32, 16 or 8 neighbouring lanes
+    const int row = t / tpr, sub = t & (tpr - 1);
     // the largest exponent fields (0: zeros and subnormal numbers only)
     unsigned mr = 0, mi = 0;
-    for (int k = lane; k < K; k += 32) {
-      const double2 v = xs[w * ldk + k];
-      mr = max(mr, unsigned(__double2hiint(v.x)) & 0x7ff00000u);
-      mi = max(mi, unsigned(__double2hiint(v.y)) & 0x7ff00000u);
-    }
-    for (int off = 16; off > 0; off >>= 1) {
+    if (row < nrows)
+      for (int k = sub; k < K; k += tpr) {
+        const double2 v = xs[row * ldk + k];
+        mr = max(mr, unsigned(__double2hiint(v.x)) & 0x7ff00000u);
+        mi = max(mi, unsigned(__double2hiint(v.y)) & 0x7ff00000u);
+      }
+    for (int off = tpr >> 1; off > 0; off >>= 1) {
       mr = max(mr, __shfl_xor_sync(0xffffffffu, mr, off));
       mi = max(mi, __shfl_xor_sync(0xffffffffu, mi, off));
     }
@@ -278,47 +308,46 @@ __global__ void __launch_bounds__(kSliceThreads) slice_tc_kernel(TcSrc x, int ti
     if (form >= 2) er = ei = max(er, ei);  // one exponent for the real and imaginary part
     if (er == oz::kExpZero) er = 0;
     if (ei == oz::kExpZero) ei = 0;
-    if (lane == 0) {
-      e_s[w][0] = er;
-      e_s[w][1] = ei;
-      if (sq0 + w < nsrc) {
-        int* e = ex + size_t(slot) * rows_pad + size_t(sq0 + w) * mult;
-        e[0] = er;
-        if (mult == 2) e[1] = ei;
-      }
+    if (sub == 0 && row < nrows) {
+      e_s[row][0] = er;
+      e_s[row][1] = ei;
+      int* e = job.ex + size_t(slot) * job.rows_pad + size_t(sq0 + row) * mult;
+      e[0] = er;
+      if (mult == 2) e[1] = ei;
     }
   }
   __syncthreads();
-  // work items: (part, row, chunk of 8 k), parts and rows fastest so that
-  // neighbouring threads write the 16-byte pieces of whole core matrices
+  // work items: (part, 8 rows, 8-row group, chunk of 8 k), parts and rows
+  // fastest so that neighbouring threads write the 16-byte pieces of whole
+  // core matrices
   const int nchunk = (form == 2 || form == 3) ? x.kp / 8 : nks * 2;
   const int pbits = cplx ? 1 : 0;
-  const int tiles = rows_pad / tile_rows;
-  const size_t tile_elems = size_t(tile_rows) * 16;
-  for (int item = t; item < (8 * nchunk << pbits); item += kSliceThreads) {
-    const int part = item & pbits, row = (item >> pbits) & 7, c = item >> (pbits + 3);
-    if (sq0 + row >= nsrc) continue;
+  const int tiles = job.rows_pad >> job.tile_shift;
+  const size_t tile_elems = size_t(16) << job.tile_shift;
+  const double* xd = reinterpret_cast<const double*>(xs);
+  for (int item = t; item < (nchunk << (rshift + pbits)); item += kSliceThreads) {
+    const int part = item & pbits, row = (item >> pbits) & (R - 1), c = item >> (pbits + rshift);
+    if (row >= nrows) continue;
     const int qtop = (sq0 + row) * mult;
     const int emax = e_s[row][part];
     const int k0 = 8 * c;
+    const double* src = xd + 2 * (row * ldk + k0) + part;
     uint32_t w[oztc::kDigits][4];
 #pragma unroll
     for (int j = 0; j < 8; j += 2) {
-      const double2 v0 = (k0 + j < K) ? xs[row * ldk + k0 + j] : make_double2(0.0, 0.0);
-      const double2 v1 = (k0 + j + 1 < K) ? xs[row * ldk + k0 + j + 1] : make_double2(0.0, 0.0);
+      const double v0 = k0 + j < K ? src[2 * j] : 0.0, v1 = k0 + j + 1 < K ? src[2 * j + 2] : 0.0;
       uint32_t d[oztc::kDigits];
-      oztc::digit_pair(part ? v0.y : v0.x, part ? v1.y : v1.x, emax, d);
+      oztc::digit_pair(v0, v1, emax, d);
 #pragma unroll
       for (int s = 0; s < oztc::kDigits; ++s) w[s][j >> 1] = d[s];
     }
     auto put = [&](int q, int kq, uint32_t flip) {
-      const size_t tb = (size_t(slot) * tiles + q / tile_rows) * nks + (kq >> 4);
-      const int toff = oztc::tile_offset(q % tile_rows, kq);
+      const size_t tb = (size_t(slot) * tiles + (q >> job.tile_shift)) * nks + (kq >> 4);
+      __nv_bfloat16* dst = job.out + tb * oztc::kDigits * tile_elems +
+                           oztc::tile_offset(q & ((1 << job.tile_shift) - 1), kq);
 #pragma unroll
-      for (int s = 0; s < oztc::kDigits; ++s) {
-        __nv_bfloat16* dst = out + (tb * oztc::kDigits + s) * tile_elems + toff;
+      for (int s = 0; s < oztc::kDigits; ++s, dst += tile_elems)
         *reinterpret_cast<uint4*>(dst) = make_uint4(w[s][0] ^ flip, w[s][1] ^ flip, w[s][2] ^ flip, w[s][3] ^ flip);
-      }
     };
     switch (form) {
       case 0: put(qtop, k0, 0u); break;
@@ -330,6 +359,13 @@ __global__ void __launch_bounds__(kSliceThreads) slice_tc_kernel(TcSrc x, int ti
       default: put(qtop + part, k0, 0u); break;
     }
   }
+}
+
+// Rows of a slicing CTA: 8, or as many more as it takes to give 256 threads a
+// conversion of 8 k each (with 8 rows of 28 complex k 64 of them had one).
+int slice_rshift(int K, bool cplx) {
+  const int per_row = (K + 7) / 8 * (cplx ? 2 : 1);
+  return per_row * 8 >= kSliceThreads ? 3 : per_row * 16 >= kSliceThreads ? 4 : 5;
 }
 
 // Output mapping of the tensor-memory product: row q of A' (slot z) is part q %
@@ -683,7 +719,9 @@ int gemm_tc(const GemmArgs& g, cudaStream_t s) {
   __nv_bfloat16* Bs = sc->buf + asz;
   int* ea = sc->ex;
   int* eb = sc->ex + size_t(a_slots) * a_rows_pad;
-  const size_t slice_shm = sizeof(double2) * 8 * size_t(K | 1);  // slice_tc_kernel's padded rows
+  // (both sides have K; a CTA's rows are padded to an odd number of elements)
+  const int rshift = slice_rshift(K, !L.real || !R.real);
+  const size_t slice_shm = sizeof(double2) * (size_t(K | 1) << rshift);
   if (slice_shm > 48 * 1024) {
     if (slice_shm > size_t(227) * 1024) return TVAP_ERR_ARG;
     if ((rc = smem_opt_in((const void*)slice_tc_kernel, slice_shm))) return rc;
@@ -712,13 +750,14 @@ int gemm_tc(const GemmArgs& g, cudaStream_t s) {
   left.rows_pad = a_rows_pad;
   left.nks = nks;
   left.scale2 = xa.scale2;
-  if (!(g.reuse_left && sc->left == left)) {
-    slice_tc_kernel<<<dim3((xa.nstack * xa.rows + 7) / 8, a_slots), kSliceThreads, slice_shm, tvap::counted(s)>>>(
-        xa, oztc::kM, a_rows_pad, nks, As, ea);
-    sc->left = left;
-  }
-  slice_tc_kernel<<<dim3((xb.rows + 7) / 8, b_slots), kSliceThreads, slice_shm, tvap::counted(s)>>>(
-      xb, oztc::kHalf, b_rows_pad, nks, Bs, eb);
+  const int srows = 1 << rshift;
+  const bool reuse = g.reuse_left && sc->left == left;
+  const TcSlice ja{xa, 7, a_rows_pad, reuse ? 0 : (xa.nstack * xa.rows + srows - 1) / srows, As, ea};
+  const TcSlice jb{xb, 5, b_rows_pad, (xb.rows + srows - 1) / srows, Bs, eb};
+  static_assert(oztc::kM == 128 && oztc::kHalf == 32, "tile_shift of the two operands");
+  slice_tc_kernel<<<dim3(ja.blocks + jb.blocks, a_slots), kSliceThreads, slice_shm, tvap::counted(s)>>>(
+      ja, jb, rshift, unsigned((1ull << 32) / K + 1), nks, sc->counter);
+  if (!reuse) sc->left = left;
   o.C = g.C;
   o.crs = crs;
   o.ccs = ccs;
@@ -738,7 +777,6 @@ int gemm_tc(const GemmArgs& g, cudaStream_t s) {
   auto kern = g_alpha_unit(o.alpha) ? (pairs ? ozaki_tc_kernel<true, true> : ozaki_tc_kernel<true, false>)
                                     : (pairs ? ozaki_tc_kernel<false, true> : ozaki_tc_kernel<false, false>);
   if ((rc = smem_opt_in((const void*)kern, oztc::kSmemBytes))) return rc;
-  TVAP_CUDA(cudaMemsetAsync(sc->counter, 0, sizeof(int), s));
   if (g_tc_timing_ctx) sec_begin_on(g_tc_timing_ctx, g_tc_timing_sec, s);
   kern<<<grid, oztc::kThreads, oztc::kSmemBytes, tvap::counted(s)>>>(As, ea, a_rows_pad, Bs, eb, b_rows_pad, b_slots == 1 ? 1 : 0,
                                                       a_slots, nks, halves, o, sc->counter, g_dev_flags);
