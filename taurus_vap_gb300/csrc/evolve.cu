@@ -300,9 +300,9 @@ __device__ void evolve_by_blocks(int n, double* S, const double* A, long long a_
 // load latency, a few FP64 issues per sub-partition and a grid barrier,
 // where each of the n pivots of evolve_by_blocks costs a dependent chain of
 // FP64 operations (64 cycles each): n = 140 265 us (two product launches and
-// the blocks) -> 172 us cold, with L^{-1} (a single-CTA inverse) 1.1 ms -> 172
+// the blocks) -> 155 us cold, with L^{-1} (a single-CTA inverse) 1.1 ms -> 155
 // us.  The blocks remain for n > kNewtonMaxN
-// (the FP32 matrix no longer fits shared memory) and, in the same launch,
+// (beyond the registers of the FP32 stage) and, in the same launch,
 // for an S so ill-conditioned that FP32 gives no usable start (or one with
 // non-finite entries, whose status they report).
 // ---------------------------------------------------------------------------
@@ -311,7 +311,6 @@ constexpr int kNewtonSteps = 6;
 // a residual up to which the step from it is the last: (n f)^2 < 1e-15 in
 // the worst case; and one above which FP32 was no use
 constexpr float kNewtonLast = 1e-10f, kNewtonUsable = 0.05f;
-constexpr int kNb32 = 8;  // block of the FP32 stage
 
 struct EvolveArgs {
   int n, newton, skip_cta, l_smem;
@@ -322,124 +321,238 @@ struct EvolveArgs {
   int* flags;
 };
 
-// X = L^{-1} (zeros above the diagonal) in FP32 by one CTA: the in-place
-// elimination of [S | 1] in blocks of 8 columns K (below, at and left of the
-// diagonal block: L_iK = S_iK R^T, R = L_KK^{-1}, X_K = R T_K; then
-// T_ij -= L_iK W_Kj for every row i below, W the L rows right of K, R on K and
-// X_K left of it).
-__device__ void inverse_f32(int n, const double* S, double* X, float* sm) {
-  const int ld = n | 1;
-  float* T = sm;                                        // row-major lower triangle
-  float* Lp = sm + (size_t(n) * ld + 3) / 4 * 4;        // n x 8
-  float* Wp = Lp + size_t(n) * kNb32;                   // n x 8
-  __shared__ float R[kNb32][kNb32 + 1];
-  const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
-  constexpr int kWarps = kCoopThreads / 32;
-  static_assert(kCoopThreads >= kNewtonMaxN, "one thread per row or column of a block step");
-  for (int j = warp; j < n; j += kWarps)
-    for (int i = j + lane; i < n; i += 32) T[i * ld + j] = float(__ldcg(&S[i + size_t(j) * n]));
-  __syncthreads();
-  for (int k0 = 0; k0 < n; k0 += kNb32) {
-    const int nb = min(kNb32, n - k0), k1 = k0 + nb;
-    if (warp == 0) {
-      // lane r holds row r of the diagonal block, then column r of its inverse
-      const int r = lane & (kNb32 - 1);
-      float a[kNb32], rv[kNb32], x[kNb32];
+// The FP32 values of doubles and back by their bits (a conversion is an FP64
+// operation): a start value for Newton steps, truncated, below the FP32 range
+// zero and above it infinite.
+__device__ __forceinline__ float start_f32(double v) {
+  const unsigned hi = unsigned(__double2hiint(v)), lo = unsigned(__double2loint(v));
+  const int e = int((hi >> 20) & 0x7ff) - 1023 + 127;
+  const unsigned m = e <= 0 ? 0u : e >= 255 ? 0x7f800000u : (unsigned(e) << 23) | ((hi & 0xfffffu) << 3) | (lo >> 29);
+  return __uint_as_float((hi & 0x80000000u) | m);
+}
+__device__ __forceinline__ double start_f64(float f) {
+  const unsigned u = __float_as_uint(f), e = (u >> 23) & 0xffu;
+  const unsigned top = e == 0 ? 0u : (e == 255 ? 0x7ffu : e + 896u) << 20;
+  return __hiloint2double(int((u & 0x80000000u) | top | (e == 0 ? 0u : (u & 0x7fffffu) >> 3)), e == 0 ? 0 : int(u << 29));
+}
+
+// X = L^{-1} (zeros above the diagonal) in FP32 by one CTA: S = M^{-1} D
+// M^{-T} by elimination, in place (column k of M takes the place of column k
+// of S at step k: below row k, T_ij -= c_i / d u_j with c column k, u_j = c_j
+// right of k, M_kj left of it, 1 at k), and L^{-1} = D^{-1/2} M.
+//
+// Warp w holds the column pairs w, w + 8, ..; a lane rows lane, lane + 32, ..
+// (from the column's own 32-row block on: 60 registers at n = 140).  The steps
+// are a chain, taken two at a time; a pair of steps is posted (one mbarrier) by
+// the warp of its columns as soon as they are up to date, before the warp's
+// other columns are, so that the chain is a pair's own update and what the
+// pair does to the other columns runs beside it.  n = 140: 78 us with the
+// matrix in shared memory, in blocks of 8 columns with three CTA barriers
+// each, 48 us so (the steps 32, reading S 9, writing X 8).
+constexpr int kF32Ring = 10;     // pairs kept (nine are needed, as in panel_gj_kernel)
+constexpr int kF32MaxSlots = 8;  // 256 rows (kNewtonMaxN = 224)
+
+template <int SLOTS>
+struct F32Inverse {
+  static constexpr int kCols = 4 * SLOTS;  // of a warp: column q = 2 P + e is column 2 (warp + 8 P) + e
+  static constexpr int kLd = 64 * SLOTS + 2;
+  float a[kCols][SLOTS];  // column q in slots q / 4 ..
+  uint64_t* posted;       // one per pair
+  float* ring;            // kF32Ring x kLd: columns k and k + 1 below rows k and k + 1, then 1 / d of both
+  float* rv;              // n (+ 1): d^{-1/2}
+  int n, warp, lane;
+
+  // columns k (even) and k + 1, up to date in t0 and t1 from slot k / 32 = S0 on
+  template <int S0>
+  __device__ __forceinline__ void post(const float (&t0)[SLOTS], float (&t1)[SLOTS], int k) {
+    const float d0 = __shfl_sync(0xffffffffu, t0[S0], k & 31), below = __shfl_sync(0xffffffffu, t0[S0], (k & 31) + 1);
+    const float r0 = __fdividef(1.f, d0), m = below * r0;
+    float* out = ring + (k / 2 % kF32Ring) * kLd;
 #pragma unroll
-      for (int c = 0; c < kNb32; ++c) a[c] = (r < nb && c <= r) ? T[(k0 + r) * ld + k0 + c] : (c == r ? 1.f : 0.f);
+    for (int s = S0; s < SLOTS; ++s) t1[s] = fmaf(-m, t0[s], t1[s]);
+    const float d1 = __shfl_sync(0xffffffffu, t1[S0], (k & 31) + 1);
+    const float r1 = k + 1 < n ? __fdividef(1.f, d1) : 0.f;
 #pragma unroll
-      for (int k = 0; k < kNb32; ++k) {
-        rv[k] = rsqrtf(__shfl_sync(0xffffffffu, a[k], k));
-        a[k] *= rv[k];
-#pragma unroll
-        for (int c = k + 1; c < kNb32; ++c) a[c] -= a[k] * __shfl_sync(0xffffffffu, a[k], c);
-      }
-#pragma unroll
-      for (int i = 0; i < kNb32; ++i) {
-        float s = 0.f;
-#pragma unroll
-        for (int k = 0; k < i; ++k) s += __shfl_sync(0xffffffffu, a[k], i) * x[k];
-        x[i] = i == r ? rv[i] : (i > r ? -s * rv[i] : 0.f);
-      }
-      if (lane < kNb32)
-#pragma unroll
-        for (int i = 0; i < kNb32; ++i) R[i][r] = x[i];
+    for (int s = S0; s < SLOTS; ++s) {
+      out[lane + 32 * s] = s > S0 || lane > (k & 31) ? t0[s] : 0.f;
+      out[32 * SLOTS + lane + 32 * s] = s > S0 || lane > (k & 31) + 1 ? t1[s] : 0.f;
     }
-    __syncthreads();
-    if (t < n) {
-      float in[kNb32], w[kNb32];
-      if (t >= k0 && t < k1) {
-        for (int c = 0; c < kNb32; ++c) {
-          w[c] = R[c][t - k0];
-          if (c < nb && k0 + c >= t) T[(k0 + c) * ld + t] = w[c];
-        }
-      } else {
-        const bool row = t >= k1;  // a row below the block, else a column left of it
-#pragma unroll
-        for (int c = 0; c < kNb32; ++c) in[c] = c < nb ? (row ? T[t * ld + k0 + c] : T[(k0 + c) * ld + t]) : 0.f;
-#pragma unroll
-        for (int c = 0; c < kNb32; ++c) {
-          float s = 0.f;
-#pragma unroll
-          for (int m = 0; m <= c; ++m) s = fmaf(R[c][m], in[m], s);
-          w[c] = s;
-        }
-        for (int c = 0; c < nb; ++c) {
-          if (row)
-            Lp[t * kNb32 + c] = w[c];
-          else
-            T[(k0 + c) * ld + t] = w[c];
-        }
-        if (row)
-          for (int c = nb; c < kNb32; ++c) Lp[t * kNb32 + c] = 0.f;
-      }
-#pragma unroll
-      for (int c = 0; c < kNb32; ++c) Wp[t * kNb32 + c] = w[c];
+    if (lane == 0) {
+      out[64 * SLOTS] = r0;
+      out[64 * SLOTS + 1] = r1;
     }
-    __syncthreads();
-    for (int jc = 0; jc < n; jc += 32) {
-      const int j = jc + lane;
-      float w[kNb32];
-#pragma unroll
-      for (int c = 0; c < kNb32; ++c) w[c] = j < n ? Wp[j * kNb32 + c] : 0.f;
-      const bool fresh = j >= k0 && j < k1;
-      // four rows at a time: their loads are all issued before the stores
-      // (which the compiler cannot tell apart)
-      constexpr int kRows = 4;
-      for (int i0 = max(k1, jc) + warp; i0 < n; i0 += kRows * kWarps) {
-        float4 l0[kRows], l1[kRows];
-        float v[kRows];
-#pragma unroll
-        for (int r = 0; r < kRows; ++r) {
-          const int i = i0 + r * kWarps;
-          const bool in = i < n && j <= i;
-          const float* l = &Lp[min(i, n - 1) * kNb32];
-          l0[r] = *reinterpret_cast<const float4*>(l);
-          l1[r] = *reinterpret_cast<const float4*>(l + 4);
-          v[r] = in && !fresh ? T[i * ld + j] : 0.f;
-        }
-#pragma unroll
-        for (int r = 0; r < kRows; ++r) {
-          v[r] = fmaf(-l0[r].x, w[0], v[r]);
-          v[r] = fmaf(-l0[r].y, w[1], v[r]);
-          v[r] = fmaf(-l0[r].z, w[2], v[r]);
-          v[r] = fmaf(-l0[r].w, w[3], v[r]);
-          v[r] = fmaf(-l1[r].x, w[4], v[r]);
-          v[r] = fmaf(-l1[r].y, w[5], v[r]);
-          v[r] = fmaf(-l1[r].z, w[6], v[r]);
-          v[r] = fmaf(-l1[r].w, w[7], v[r]);
-        }
-#pragma unroll
-        for (int r = 0; r < kRows; ++r) {
-          const int i = i0 + r * kWarps;
-          if (i < n && j <= i) T[i * ld + j] = v[r];
-        }
-      }
+    __syncwarp();
+    if (lane == 0) {
+      step_post(&posted[k / 2]);
+      rv[k] = rsqrtf(d0);
+      rv[k + 1] = rsqrtf(d1);
     }
-    __syncthreads();
   }
-  for (int j = warp; j < n; j += kWarps)
-    for (int i = lane; i < n; i += 32) X[i + size_t(j) * n] = i >= j ? double(T[i * ld + j]) : 0.0;
+  // the next pair (not needed again before its steps): columns 4 SK + 0, 1 or
+  // 2, 3 of its warp, or 4 SK + 4, 5 if it begins the next 32
+  template <int SK>
+  __device__ __forceinline__ void ahead(const float (&mu0)[SLOTS], const float (&mu1)[SLOTS], const float* c, int kn) {
+    float t0[SLOTS], t1[SLOTS];
+    const float u00 = c[kn], u01 = c[32 * SLOTS + kn], u10 = c[kn + 1], u11 = c[32 * SLOTS + kn + 1];
+    if (kn < 32 * SK + 32) {
+      const bool second = kn >= 32 * SK + 16;
+#pragma unroll
+      for (int s = SK; s < SLOTS; ++s) {
+        const float x0 = a[4 * SK][s], y0 = a[4 * SK + 2][s], x1 = a[4 * SK + 1][s], y1 = a[4 * SK + 3][s];
+        t0[s] = fmaf(-mu1[s], u01, fmaf(-mu0[s], u00, second ? y0 : x0));
+        t1[s] = fmaf(-mu1[s], u11, fmaf(-mu0[s], u10, second ? y1 : x1));
+      }
+      post<SK>(t0, t1, kn);
+    } else if constexpr (SK + 1 < SLOTS) {
+#pragma unroll
+      for (int s = SK + 1; s < SLOTS; ++s) {
+        t0[s] = fmaf(-mu1[s], u01, fmaf(-mu0[s], u00, a[4 * SK + 4][s]));
+        t1[s] = fmaf(-mu1[s], u11, fmaf(-mu0[s], u10, a[4 * SK + 5][s]));
+      }
+      post<SK + 1>(t0, t1, kn);
+    }
+  }
+  // the factors of every column first, without branches, so that their
+  // latencies overlap (0: the pair itself, which follows, and the next one,
+  // which is done).  m: the multiplier of row k + 1 in step k
+  template <int Q, int SK>
+  __device__ __forceinline__ void factors(float (&u0)[kCols], float (&u1)[kCols], const float* c, int k, float m) {
+    if constexpr (Q < kCols) {
+      const int j = 2 * (warp + 8 * (Q / 2)) + Q % 2;
+      if constexpr (Q < 4 * SK + 4) {
+        u0[Q] = __shfl_sync(0xffffffffu, a[Q][SK], k & 31);
+        u1[Q] = fmaf(-m, u0[Q], __shfl_sync(0xffffffffu, a[Q][SK], (k & 31) + 1));
+      }
+      if constexpr (Q >= 4 * SK) {
+        const float right0 = c[j], right1 = c[32 * SLOTS + j];
+        const bool done = Q < 4 * SK + 6 && j < k + 4;
+        if constexpr (Q < 4 * SK + 4) {
+          u0[Q] = j < k ? u0[Q] : done ? 0.f : right0;
+          u1[Q] = j < k ? u1[Q] : done ? 0.f : right1;
+        } else {
+          u0[Q] = done ? 0.f : right0;
+          u1[Q] = done ? 0.f : right1;
+        }
+      }
+      factors<Q + 1, SK>(u0, u1, c, k, m);
+    }
+  }
+  template <int Q, int SK>
+  __device__ __forceinline__ void columns(const float (&mu0)[SLOTS], const float (&mu1)[SLOTS],
+                                          const float (&u0)[kCols], const float (&u1)[kCols]) {
+    if constexpr (Q < kCols) {
+      constexpr int s0 = Q / 4 > SK ? Q / 4 : SK;
+#pragma unroll
+      for (int s = s0; s < SLOTS; ++s) a[Q][s] = fmaf(-mu1[s], u1[Q], fmaf(-mu0[s], u0[Q], a[Q][s]));
+      columns<Q + 1, SK>(mu0, mu1, u0, u1);
+    }
+  }
+  // columns k and k + 1 of M, in columns Q and Q + 1
+  template <int Q, int SK>
+  __device__ __forceinline__ void start(const float (&mu0)[SLOTS], const float (&mu1)[SLOTS], int k, float m) {
+    if (k >> 4 == Q / 2) {
+#pragma unroll
+      for (int s = SK; s < SLOTS; ++s) {
+        a[Q][s] = s == SK && lane == (k & 31) ? 1.f : fmaf(mu1[s], m, -mu0[s]);
+        a[Q + 1][s] = s == SK && lane == (k & 31) + 1 ? 1.f : -mu1[s];
+      }
+    }
+  }
+  template <int SK>
+  __device__ __forceinline__ bool steps() {
+    if constexpr (SK < SLOTS) {
+      for (int k = 32 * SK; k < min(32 * SK + 32, n); k += 2) {
+        if (!step_wait(&posted[k / 2])) return false;
+        const float* c = ring + (k / 2 % kF32Ring) * kLd;
+        const float r0 = c[64 * SLOTS], r1 = c[64 * SLOTS + 1];
+        const float m = c[k + 1] * r0;
+        float mu0[SLOTS], mu1[SLOTS];
+#pragma unroll
+        for (int s = SK; s < SLOTS; ++s) {
+          mu0[s] = c[lane + 32 * s] * r0;
+          mu1[s] = c[32 * SLOTS + lane + 32 * s] * r1;
+        }
+        if (k + 2 < n && warp == ((k / 2 + 1) & 7)) ahead<SK>(mu0, mu1, c, k + 2);
+        float u0[kCols], u1[kCols];
+        factors<0, SK>(u0, u1, c, k, m);
+        columns<0, SK>(mu0, mu1, u0, u1);
+        if (warp == ((k / 2) & 7)) {
+          start<4 * SK, SK>(mu0, mu1, k, m);
+          start<4 * SK + 2, SK>(mu0, mu1, k, m);
+        }
+      }
+      return steps<SK + 1>();
+    }
+    return true;
+  }
+  // between the registers and the matrix in shared memory (column-major, n rows)
+  template <int Q, bool LOAD>
+  __device__ __forceinline__ void transfer(float* T) {
+    if constexpr (Q < kCols) {
+      const int j = 2 * (warp + 8 * (Q / 2)) + Q % 2;
+#pragma unroll
+      for (int s = Q / 4; s < SLOTS; ++s) {
+        const int i = lane + 32 * s;
+        const bool in = i < n && j < n;
+        if (LOAD)
+          a[Q][s] = in ? T[i + j * n] : 0.f;
+        else if (in)
+          T[i + j * n] = a[Q][s];
+      }
+      transfer<Q + 1, LOAD>(T);
+    }
+  }
+};
+
+template <int SLOTS>
+__device__ void inverse_f32(int n, const double* S, double* X, double* sm, int* flags) {
+  static_assert(kCoopThreads == 256, "eight warps hold the columns");
+  __shared__ int s_late;
+  F32Inverse<SLOTS> f;
+  f.n = n;
+  f.warp = threadIdx.x >> 5;
+  f.lane = threadIdx.x & 31;
+  f.posted = reinterpret_cast<uint64_t*>(sm);
+  f.ring = reinterpret_cast<float*>(f.posted + (n + 1) / 2);
+  f.rv = f.ring + kF32Ring * f.kLd;
+  float* T = f.rv + n + 1;
+  if (threadIdx.x == 0) s_late = 0;
+  if (int(threadIdx.x) < (n + 1) / 2) step_init(&f.posted[threadIdx.x]);
+  // (through shared memory: the conversions are a short loop, not an instance
+  // for every register -- a call finds its instructions far away)
+  constexpr int kLoads = 4;
+#pragma unroll 1
+  for (int j = f.warp; j < n; j += 8 * kLoads) {
+    double v[kLoads][SLOTS];
+#pragma unroll
+    for (int q = 0; q < kLoads; ++q)
+#pragma unroll
+      for (int s = 0; s < SLOTS; ++s)
+        v[q][s] = __ldcg(&S[min(f.lane + 32 * s, n - 1) + min(j + 8 * q, n - 1) * n]);
+#pragma unroll
+    for (int q = 0; q < kLoads; ++q)
+#pragma unroll
+      for (int s = 0; s < SLOTS; ++s)
+        if (f.lane + 32 * s < n && j + 8 * q < n) T[f.lane + 32 * s + (j + 8 * q) * n] = start_f32(v[q][s]);
+  }
+  __syncthreads();
+  f.template transfer<0, true>(T);
+  if (f.warp == 0) f.template post<0>(f.a[0], f.a[1], 0);
+  if (!f.template steps<0>()) s_late = 1;
+  __syncthreads();
+  if (s_late && threadIdx.x == 0) atomicOr(flags, DEV_WAIT_TIMEOUT);
+  f.template transfer<0, false>(T);
+  __syncthreads();
+#pragma unroll 1
+  for (int j = f.warp; j < n; j += 8)
+#pragma unroll
+    for (int s = 0; s < SLOTS; ++s) {
+      const int i = f.lane + 32 * s;
+      if (i < n) X[i + size_t(j) * n] = i >= j ? start_f64(T[i + j * n] * f.rv[i]) : 0.0;
+    }
+  // the barriers' shared memory is used for other data next
+  __syncthreads();
+  if (int(threadIdx.x) < (n + 1) / 2) step_inval(&f.posted[threadIdx.x]);
 }
 
 // One 8 x 4 tile of a product: sum over k in [klo, khi) of A(i0 + i, k)
@@ -553,7 +666,7 @@ __global__ void __launch_bounds__(kCoopThreads, 1) thouless_evolve_kernel(Evolve
   const int per = tm * tn;
   if (cta == 0) {
     __syncthreads();
-    inverse_f32(n, p.S, p.X0, reinterpret_cast<float*>(evolve_smem));
+    if constexpr (SLOTS <= kF32MaxSlots) inverse_f32<SLOTS>(n, p.S, p.X0, evolve_smem, p.flags);
   }
   if (cta > 0 || G == 1)
     tile_products(
@@ -671,13 +784,14 @@ int thouless_evolve(int n, const double* Z, const double* U0, const double* V0, 
   p.Linv = Linv;
   p.bar = bar;
   p.flags = flags;
-  // shared memory: the FP32 matrix and its panels, the tiles' operands, the
+  // shared memory: the FP32 stage's steps, the tiles' operands, the
   // blocks' panel rows; without Newton steps L for the blocks' solves when it
   // fits (else the panel rows, L read from L2)
   const size_t panel = sizeof(double) * (nn / n * kCoopNb + n);
   size_t shm = panel;
   if (p.newton) {
-    shm = std::max(shm, sizeof(float) * (size_t(n) * (n | 1) + 4 + 2 * size_t(n) * kNb32));
+    static_assert(kNewtonMaxN <= 32 * kF32MaxSlots, "the FP32 stage holds the matrix");
+    shm = std::max(shm, sizeof(double) * n + sizeof(float) * (kF32Ring * (64 * kF32MaxSlots + 2) + n + 1 + nn));
     shm = std::max(shm, sizeof(double) * kBatch * (size_t(n) * kTileElems + kCoopThreads));
   } else {
     const size_t full = sizeof(double) * (nn + n);

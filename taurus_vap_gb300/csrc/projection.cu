@@ -1731,27 +1731,6 @@ __device__ __forceinline__ double2 flip_sign(double2 z) {
                       __longlong_as_double(__double_as_longlong(z.y) ^ sign));
 }
 
-// a posted step: an mbarrier of one arrival, used for one phase
-__device__ __forceinline__ uint32_t step_addr(const uint64_t* bar) {
-  return static_cast<uint32_t>(__cvta_generic_to_shared(bar));
-}
-__device__ __forceinline__ void step_post(uint64_t* bar) {
-  asm volatile("{\n.reg .b64 st;\nmbarrier.arrive.shared::cta.b64 st, [%0];\n}\n" ::"r"(step_addr(bar)) : "memory");
-}
-// bounded (a step is posted within a few microseconds)
-__device__ __forceinline__ bool step_wait(const uint64_t* bar) {
-  for (int it = 0; it < (1 << 16); ++it) {
-    uint32_t done;
-    asm volatile(
-        "{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], 0;\nselp.u32 %0, 1, 0, p;\n}\n"
-        : "=r"(done)
-        : "r"(step_addr(bar))
-        : "memory");
-    if (done) return true;
-  }
-  return false;
-}
-
 constexpr int kGjMaxSlots = 12;  // panels of up to 384 rows
 // Multipliers of single-precision steps kept: a warp that posts step k + 9 is
 // the warp that posted k + 1, and the seven others have posted steps k + 2
@@ -1776,7 +1755,7 @@ __global__ void __launch_bounds__(kFactorThreads)
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   if (tid == 0) s_sing = s_late = 0;
   if (tid < 2 * kPanelMax)
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(step_addr(&posted[0][0] + tid)) : "memory");
+    step_init(&posted[0][0] + tid);
   for (int r = tid; r < 32 * SLOTS; r += kFactorThreads) srow[r] = r;
   float2 a[kQ][SLOTS];
 #pragma unroll

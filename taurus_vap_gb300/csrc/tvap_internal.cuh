@@ -78,6 +78,34 @@ __device__ __forceinline__ double2 crcp_newton(double2 z) {
   y = fma(y, e, y);
   return make_double2(z.x * y, -z.y * y);
 }
+// A step of an elimination handed from the warp that forms it to the others: an
+// mbarrier of one arrival, used for one phase.
+__device__ __forceinline__ uint32_t step_addr(const uint64_t* bar) {
+  return static_cast<uint32_t>(__cvta_generic_to_shared(bar));
+}
+__device__ __forceinline__ void step_init(uint64_t* bar) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(step_addr(bar)) : "memory");
+}
+// (before the shared memory of a barrier is used for other data)
+__device__ __forceinline__ void step_inval(uint64_t* bar) {
+  asm volatile("mbarrier.inval.shared::cta.b64 [%0];\n" ::"r"(step_addr(bar)) : "memory");
+}
+__device__ __forceinline__ void step_post(uint64_t* bar) {
+  asm volatile("{\n.reg .b64 st;\nmbarrier.arrive.shared::cta.b64 st, [%0];\n}\n" ::"r"(step_addr(bar)) : "memory");
+}
+// bounded (a step is posted within a few microseconds)
+__device__ __forceinline__ bool step_wait(const uint64_t* bar) {
+  for (int it = 0; it < (1 << 20); ++it) {
+    uint32_t done;
+    asm volatile(
+        "{\n.reg .pred p;\nmbarrier.test_wait.parity.shared::cta.b64 p, [%1], 0;\nselp.u32 %0, 1, 0, p;\n}\n"
+        : "=r"(done)
+        : "r"(step_addr(bar))
+        : "memory");
+    if (done) return true;
+  }
+  return false;
+}
 #endif
 __host__ __device__ __forceinline__ double cabs1(double2 a) { return fabs(a.x) + fabs(a.y); }
 
