@@ -35,6 +35,7 @@
 #include <cmath>
 #include <complex>
 #include <cstring>
+#include <functional>
 #include <vector>
 
 #include "tvap_internal.cuh"
@@ -299,7 +300,11 @@ __device__ bool pair_subspace(int n, int k0, int d, double* kapc, double* D, dou
 // diagonalisation, module_wavefunctions.f90:818-945, and the v/u extraction
 // of project_wavefunction, module_projection.f90:219-234).  One CTA.
 __global__ void canon_kernel(int n, const double* __restrict__ rhoc, double* __restrict__ kapc, double* D,
-                             double* sch, double eps, int allemp, int* canon_i, double* canon_d) {
+                             double* sch, double eps, int allemp, int* canon_i, double* canon_d,
+                             const int* __restrict__ gate) {
+  // queued before the verdict on D is known (gate: cluster_finish_kernel's
+  // flags): nothing is done, and D stays as it is, unless D is final
+  if (gate && (gate[0] != 0 || gate[2] != 0)) return;
   __shared__ int submax[1024];
   __shared__ double rd[256];
   __shared__ int ri[3][256];
@@ -2440,12 +2445,12 @@ int blocked_thouless_solve(tvap_ctx* c, int G, cudaStream_t s) {
 namespace {
 
 // Refinement steps from the approximate eigenvectors in X (Xn scratch), the
-// exact treatment of near-degenerate clusters and the final check; *fail is
-// the check's verdict (read back on the host) and *Xout the buffer holding
-// the refined columns.  assign: fix the clusters at the first step (else
-// keep those of the previous call); second_order: add F^2/2 to each step.
-int refine_canonical(tvap_ctx* c, double* X, double* Xn, int steps, int* fail, cudaStream_t s, bool assign,
-                     bool second_order, double** Xout) {
+// exact treatment of near-degenerate clusters and the final check, queued on
+// s; *Xout is the buffer that will hold the refined columns.  assign: fix the
+// clusters at the first step (else keep those of the previous call);
+// second_order: add F^2/2 to each step.
+int refine_launch(tvap_ctx* c, double* X, double* Xn, int steps, cudaStream_t s, bool assign, bool second_order,
+                  double** Xout) {
   Workspace* w = c->ws;
   const int n = c->n;
   const size_t nn = size_t(n) * n;
@@ -2478,11 +2483,23 @@ int refine_canonical(tvap_ctx* c, double* X, double* Xn, int steps, int* fail, c
   cluster_finish_kernel<<<kRlCtas, kCfThreads, 0, tvap::counted(s)>>>(n, w->Sr, X, w->rscal, w->cid, w->D, w->evals,
                                                                  w->cperm, w->bigd, w->rflag);
   TVAP_CUDA(cudaGetLastError());
-  int hr[3] = {1, 0, 0};
-  int bd[2 * kCfBigSlots];
-  TVAP_CUDA(cudaMemcpyAsync(hr, w->rflag, sizeof(hr), cudaMemcpyDeviceToHost, s));
-  TVAP_CUDA(cudaMemcpyAsync(bd, w->bigd, sizeof(bd), cudaMemcpyDeviceToHost, s));
-  TVAP_CUDA(cudaStreamSynchronize(s));
+  *Xout = X;
+  return TVAP_OK;
+}
+
+// What the final check left on the host: w->rflag (verdict, clusters, large
+// clusters) and w->bigd.
+struct RefineFlags {
+  int hr[3], bd[2 * kCfBigSlots];
+};
+
+// The verdict *fail of the refinement that left its columns in X, with its
+// large clusters diagonalised.
+int refine_result(tvap_ctx* c, const RefineFlags& f, double* X, int* fail, cudaStream_t s) {
+  Workspace* w = c->ws;
+  const int n = c->n;
+  const int *hr = f.hr, *bd = f.bd;
+  int rc;
   *fail = hr[0];
   c->canon_attempts[3] += hr[1];
   if (hr[0] == 0 && hr[2] > 0) {
@@ -2513,8 +2530,50 @@ int refine_canonical(tvap_ctx* c, double* X, double* Xn, int steps, int* fail, c
   }
   for (int b = 0; b < 3; ++b)
     if (*fail & (1 << b)) ++c->canon_attempts[4 + b];
-  *Xout = X;
   return TVAP_OK;
+}
+
+int refine_canonical(tvap_ctx* c, double* X, double* Xn, int steps, int* fail, cudaStream_t s, bool assign,
+                     bool second_order, double** Xout) {
+  int rc;
+  if ((rc = refine_launch(c, X, Xn, steps, s, assign, second_order, Xout))) return rc;
+  RefineFlags f;
+  TVAP_CUDA(cudaMemcpyAsync(f.hr, c->ws->rflag, sizeof(f.hr), cudaMemcpyDeviceToHost, s));
+  TVAP_CUDA(cudaMemcpyAsync(f.bd, c->ws->bigd, sizeof(f.bd), cudaMemcpyDeviceToHost, s));
+  TVAP_CUDA(cudaStreamSynchronize(s));
+  return refine_result(c, f, *Xout, fail, s);
+}
+
+// The FP32 start of the refinement, into w->Xr: one-sided Jacobi on M = V^T D
+// (M^T M = D^T rho D) over a cluster of 8 CTAs; the two-sided single-CTA
+// kernel on D^T rho D when n is too large for it.  *none: neither runs here.
+int canonical_start(tvap_ctx* c, bool warm, bool* none, cudaStream_t s) {
+  Workspace* w = c->ws;
+  const int n = c->n;
+  int rc;
+  *none = false;
+  const View Dp = view_cm(w->D, n, 0);
+  if (warm) {
+    if ((rc = real_gemm(n, n, n, view_t(view_cm(w->V, n, 0)), Dp, w->Br, n, 1.0, 0.0, s))) return rc;
+    rc = jacobi_cluster(n, w->Br, 0, w->D, w->Xr, w->rflag + 1, s);
+  } else {
+    rc = jacobi_cluster(n, w->V, 1, nullptr, w->Xr, w->rflag + 1, s);
+  }
+  if (rc != TVAP_ERR_ARG) return rc;
+  if (jacobi32_smem_bytes(n) > jacobi32_smem_limit()) {
+    *none = true;
+    return TVAP_OK;
+  }
+  if (!warm) return jacobi32_smem(n, w->rho, nullptr, w->Xr, w->rflag + 1, s);
+  if ((rc = real_gemm(n, n, n, view_cm(w->rho, n, 0), Dp, w->Br, n, 1.0, 0.0, s))) return rc;
+  if ((rc = real_gemm(n, n, n, view_t(Dp), view_cm(w->Br, n, 0), w->Sr, n, 1.0, 0.0, s))) return rc;
+  return jacobi32_smem(n, w->Sr, w->D, w->Xr, w->rflag + 1, s);
+}
+
+// the FP32 stage: the cluster Jacobi (n <= 384), else the single-CTA one
+// when its matrices fit shared memory
+bool canonical_fp32(int n) {
+  return (n <= 384 || jacobi32_smem_bytes(n) <= jacobi32_smem_limit()) && n <= kCfMaxN;
 }
 
 }  // namespace
@@ -2527,60 +2586,38 @@ int refine_canonical(tvap_ctx* c, double* X, double* Xn, int steps, int* fail, c
 // shared-memory stage.  (Refining the previous basis directly, without the
 // Jacobi stage, does not converge when the state moves by a full gradient
 // step: couplings exceed the gaps between canonical pairs.)
-int eigen_canonical(tvap_ctx* c, cudaStream_t s) {
+// first: what the first attempt, queued by prepare_canonical_begin, left
+// (null: it is not queued), and Xf its refined columns.
+int eigen_canonical(tvap_ctx* c, const RefineFlags* first, double* Xf, cudaStream_t s) {
   Workspace* w = c->ws;
   const int n = c->n;
   const size_t nn = size_t(n) * n;
   int rc, fail = 1;
-  // the FP32 stage: the cluster Jacobi (n <= 384), else the single-CTA one
-  // when its matrices fit shared memory
-  if ((n <= 384 || jacobi32_smem_bytes(n) <= jacobi32_smem_limit()) && n <= kCfMaxN) {
-    double* X = w->Xr;
-    double* Xn = w->Xn;
-    const View Rho = view_cm(w->rho, n, 0);
+  if (canonical_fp32(n)) {
     // a second attempt starts from the basis the first one refined (left in
     // w->D): the FP32 Jacobi then works on a nearly diagonal matrix whose
     // small entries keep their relative precision, which resolves the pairs
     // whose gaps were too small for the Newton steps
-    const View Vn = view_cm(w->V, n, 0);
     for (int attempt = 0; attempt < 2 && fail; ++attempt) {
-      const bool warm = w->have_basis || attempt > 0;
-      // one-sided Jacobi on M = V^T D (M^T M = D^T rho D) over a cluster of
-      // 8 CTAs; the two-sided single-CTA kernel on D^T rho D when n is too
-      // large for it
-      if (warm) {
-        const View Dp = view_cm(w->D, n, 0);
-        if ((rc = real_gemm(n, n, n, view_t(Vn), Dp, w->Br, n, 1.0, 0.0, s))) return rc;
-        rc = jacobi_cluster(n, w->Br, 0, w->D, X, w->rflag + 1, s);
+      if (attempt == 0 && first) {
+        if ((rc = refine_result(c, *first, Xf, &fail, s))) return rc;
       } else {
-        rc = jacobi_cluster(n, w->V, 1, nullptr, X, w->rflag + 1, s);
-      }
-      if (rc == TVAP_ERR_ARG) {
-        if (jacobi32_smem_bytes(n) > jacobi32_smem_limit()) {
+        bool none = false;
+        if ((rc = canonical_start(c, w->have_basis || attempt > 0, &none, s))) return rc;
+        if (none) {
           fail = 1;  // neither FP32 stage runs here: the exact FP64 Jacobi below
           break;
         }
-        if (warm) {
-          const View Dp = view_cm(w->D, n, 0);
-          if ((rc = real_gemm(n, n, n, Rho, Dp, w->Br, n, 1.0, 0.0, s))) return rc;
-          if ((rc = real_gemm(n, n, n, view_t(Dp), view_cm(w->Br, n, 0), w->Sr, n, 1.0, 0.0, s))) return rc;
-          if ((rc = jacobi32_smem(n, w->Sr, w->D, X, w->rflag + 1, s))) return rc;
-        } else {
-          if ((rc = jacobi32_smem(n, w->rho, nullptr, X, w->rflag + 1, s))) return rc;
-        }
-      } else if (rc) {
-        return rc;
+        ++c->canon_attempts[0];
+        if ((rc = refine_canonical(c, w->Xr, w->Xn, 3, &fail, s, true, false, &Xf))) return rc;
       }
-      ++c->canon_attempts[0];
-      double* Xf = X;
-      if ((rc = refine_canonical(c, X, Xn, 3, &fail, s, true, false, &Xf))) return rc;
       if (fail && !(fail & 4)) {
         // not yet orthonormal or decoupled (nearly closed shells: an FP32
         // start with ||I - X^T X|| ~ 1e-4 and clusters of levels it could not
         // separate): two second-order steps more from the refined basis,
         // with the same clusters, before anything is recomputed
         ++c->canon_attempts[8];
-        if ((rc = refine_canonical(c, Xf, Xf == X ? Xn : X, 2, &fail, s, false, true, &Xf))) return rc;
+        if ((rc = refine_canonical(c, Xf, Xf == w->Xr ? w->Xn : w->Xr, 2, &fail, s, false, true, &Xf))) return rc;
       }
     }
     if (!fail) {
@@ -2626,48 +2663,97 @@ int prepare_uv_blocks(tvap_ctx* c, cudaStream_t s) {
   return TVAP_OK;
 }
 
-// Canonical basis (construct_canonical_basis) and its blocks (8, 9) on stream
-// s; host_canon receives nocc, nemp and the bad-block flag (s is
-// synchronised).
-int prepare_canonical(tvap_ctx* c, double occeps, double allemp_d, int* host_canon, cudaStream_t s) {
+// What follows from the basis w->D: rhoc = D^T rho D, kappac = D^T kappa D,
+// the occupations and pairs, and the blocks D_t^T D_t.  gate: as canon_kernel.
+int canonical_products(tvap_ctx* c, double occeps, double allemp_d, const int* gate, cudaStream_t s) {
   Workspace* w = c->ws;
   const int n = c->n, h = n / 2;
   const size_t nn = size_t(n) * n;
   int rc;
-  const View Vn = view_cm(w->V, n, 0), Un = view_cm(w->U, n, 0);
-  sec_begin_on(c, SEC_CANONICAL, s);
-  // rho = V V^T, kappa = V U^T (construct_canonical_basis :826, :862)
-  if ((rc = real_gemm(n, n, n, Vn, view_t(Vn), w->rho, n, 1.0, 0.0, s))) return rc;
-  if ((rc = real_gemm(n, n, n, Vn, view_t(Un), w->kap, n, 1.0, 0.0, s))) return rc;
-  if ((rc = eigen_canonical(c, s))) return rc;
   const View Dn = view_cm(w->D, n, 0);
-  // rhoc = D^T rho D, kappac = D^T kappa D
   if ((rc = real_gemm(n, n, n, view_t(Dn), view_cm(w->rho, n, 0), w->tmp, n, 1.0, 0.0, s))) return rc;
   if ((rc = real_gemm(n, n, n, view_cm(w->tmp, n, 0), Dn, w->rhoc, n, 1.0, 0.0, s))) return rc;
   if ((rc = real_gemm(n, n, n, view_t(Dn), view_cm(w->kap, n, 0), w->tmp, n, 1.0, 0.0, s))) return rc;
   if ((rc = real_gemm(n, n, n, view_cm(w->tmp, n, 0), Dn, w->kapc, n, 1.0, 0.0, s))) return rc;
   const double eps = (occeps < 2.2250738585072014e-308) ? 1.0e-8 : occeps;
   canon_kernel<<<1, 256, 0, tvap::counted(s)>>>(n, w->rhoc, w->kapc, w->D, w->schq, eps, int(allemp_d), w->canon_i,
-                                                w->canon_d);
+                                                w->canon_d, gate);
   TVAP_CUDA(cudaGetLastError());
-  {
-    // D_t^T D_t over the rows of isospin t, batch t = p, n
-    GemmArgs g{};
-    g.M = g.N = n;
-    g.K = h;
-    g.batch = 2;
-    g.A = View{w->D, n, 1, h};
-    g.B = View{w->D, 1, n, h};
-    g.C = w->blocks + 8 * nn;
-    g.crs = 1;
-    g.ccs = n;
-    g.cbs = (long long)nn;
-    g.alpha = make_double2(1.0, 0.0);
-    g.beta = make_double2(0.0, 0.0);
-    g.a_real = g.b_real = g.c_real = true;
-    if ((rc = gemm(g, s))) return rc;
-  }
+  // D_t^T D_t over the rows of isospin t, batch t = p, n
+  GemmArgs g{};
+  g.M = g.N = n;
+  g.K = h;
+  g.batch = 2;
+  g.A = View{w->D, n, 1, h};
+  g.B = View{w->D, 1, n, h};
+  g.C = w->blocks + 8 * nn;
+  g.crs = 1;
+  g.ccs = n;
+  g.cbs = (long long)nn;
+  g.alpha = make_double2(1.0, 0.0);
+  g.beta = make_double2(0.0, 0.0);
+  g.a_real = g.b_real = g.c_real = true;
+  return gemm(g, s);
+}
+
+// The canonical basis between its two halves (the host copies lie in the
+// context's pinned buffer).
+struct CanonicalQueue {
+  bool queued = false;
+  double* Xf = nullptr;
+};
+struct CanonicalHost {
+  RefineFlags f;
+  int canon[3];
+};
+static_assert(sizeof(CanonicalHost) <= kPinnedCanonical, "the pinned buffer's second part");
+
+// Canonical basis (construct_canonical_basis) and its blocks (8, 9) on stream
+// s.  The first half only queues: the first attempt at the basis and, before
+// its verdict is known, what follows from it -- a wait on the host between
+// them left the stream idle for 20 us, and a caller with other chains queues
+// them while this one runs.  The second half waits, and repeats what the
+// verdict asks for; host_canon receives nocc, nemp and the bad-block flag.
+int prepare_canonical_begin(tvap_ctx* c, double occeps, double allemp_d, CanonicalQueue* q, cudaStream_t s) {
+  Workspace* w = c->ws;
+  const int n = c->n;
+  int rc;
+  const View Vn = view_cm(w->V, n, 0), Un = view_cm(w->U, n, 0);
+  sec_begin_on(c, SEC_CANONICAL, s);
+  // rho = V V^T, kappa = V U^T (construct_canonical_basis :826, :862)
+  if ((rc = real_gemm(n, n, n, Vn, view_t(Vn), w->rho, n, 1.0, 0.0, s))) return rc;
+  if ((rc = real_gemm(n, n, n, Vn, view_t(Un), w->kap, n, 1.0, 0.0, s))) return rc;
+  if (!canonical_fp32(n)) return TVAP_OK;
+  bool none = false;
+  if ((rc = canonical_start(c, w->have_basis, &none, s))) return rc;
+  if (none) return TVAP_OK;
+  ++c->canon_attempts[0];
+  if ((rc = refine_launch(c, w->Xr, w->Xn, 3, s, true, false, &q->Xf))) return rc;
+  if ((rc = canonical_products(c, occeps, allemp_d, w->rflag, s))) return rc;
   sec_end_on(c, SEC_CANONICAL, s);
+  auto* host = reinterpret_cast<CanonicalHost*>(static_cast<unsigned char*>(c->h_pin) + kPinnedBytes);
+  TVAP_CUDA(cudaMemcpyAsync(host->f.hr, w->rflag, sizeof(host->f.hr), cudaMemcpyDeviceToHost, s));
+  TVAP_CUDA(cudaMemcpyAsync(host->f.bd, w->bigd, sizeof(host->f.bd), cudaMemcpyDeviceToHost, s));
+  TVAP_CUDA(cudaMemcpyAsync(host->canon, w->canon_i, sizeof(host->canon), cudaMemcpyDeviceToHost, s));
+  q->queued = true;
+  return TVAP_OK;
+}
+
+int prepare_canonical_end(tvap_ctx* c, double occeps, double allemp_d, const CanonicalQueue& q, int* host_canon,
+                          cudaStream_t s) {
+  Workspace* w = c->ws;
+  int rc;
+  const auto* host = reinterpret_cast<const CanonicalHost*>(static_cast<unsigned char*>(c->h_pin) + kPinnedBytes);
+  RefineFlags f{};
+  if (q.queued) {
+    TVAP_CUDA(cudaStreamSynchronize(s));
+    f = host->f;
+    std::memcpy(host_canon, host->canon, sizeof(host->canon));
+  }
+  if ((rc = eigen_canonical(c, q.queued ? &f : nullptr, q.Xf, s))) return rc;
+  if (q.queued && f.hr[0] == 0 && f.hr[2] == 0) return TVAP_OK;
+  if ((rc = canonical_products(c, occeps, allemp_d, nullptr, s))) return rc;
+  if (!q.queued) sec_end_on(c, SEC_CANONICAL, s);
   TVAP_CUDA(cudaMemcpyAsync(host_canon, w->canon_i, sizeof(int) * 3, cudaMemcpyDeviceToHost, s));
   TVAP_CUDA(cudaStreamSynchronize(s));
   return TVAP_OK;
@@ -2741,9 +2827,10 @@ int angles_overlap(tvap_ctx* c, int G, const double2* d_ephase, int nocc, int ne
 // Thouless chain of angles [0, G) on stream s (needs only U, V and their
 // blocks): U_phi, V_phi, A_phi, U~, V~, the transition densities, the fields,
 // the traces and H20.
-// want_h20 = false stops after the traces.
+// want_h20 = false stops after the traces.  meanwhile (may be empty) queues
+// other streams' work once the solve, the longest single part, is queued.
 int angles_thouless(tvap_ctx* c, int G, const double2* d_ephase, double factor_delta, cudaStream_t s,
-                    bool want_h20 = true) {
+                    bool want_h20 = true, const std::function<int()>& meanwhile = {}) {
   Workspace* w = c->ws;
   const int n = c->n;
   const size_t nn = size_t(n) * n;
@@ -2755,6 +2842,7 @@ int angles_thouless(tvap_ctx* c, int G, const double2* d_ephase, double factor_d
   // A_phi = conj(V_phi U_phi^{-1}): solve U_phi^T Y = V_phi^T, A = conj(Y^T)
   if ((rc = blocked_thouless_solve(c, G, s))) return rc;
   sec_end_on(c, SEC_SOLVE, s);
+  if (meanwhile && (rc = meanwhile())) return rc;
   sec_begin_on(c, SEC_UV, s);
   // U~ = U + V A, V~ = V + U A
   broadcast_real_kernel<<<nblk(nn * G, tb), tb, 0, tvap::counted(s)>>>(nn, G, w->U, w->Ut);
@@ -3023,18 +3111,25 @@ int project_device(tvap_ctx* c, const tvap_proj_opts& o, tvap_pnp* out, bool syn
   if (o.mode == 0) {
     // The Thouless chain needs only U and V: it is queued first, on streamM
     // (priority between those of the second and third streams); the
-    // canonical basis (with its host-side checks) follows on the second
-    // stream and the overlap chain on the third, concurrently; the sums join
-    // all three on the caller's stream.
+    // canonical basis (with its host-side checks) on the second stream --
+    // queued behind the solve, which gives the device enough to do until the
+    // rest of the Thouless chain is queued -- and the overlap chain on the
+    // third, concurrently; the sums join all three on the caller's stream.
+    // (Queued behind the whole Thouless chain, the basis began 97 us (n = 24)
+    // to 227 us (n = 140) after it, of 644 and 3835 us for the projection.)
+    CanonicalQueue cq;
     cudaStream_t sm = c->streamM;
     sec_mark(c, s);
     TVAP_CUDA(cudaEventRecord(c->ev_fork, s));
     TVAP_CUDA(cudaStreamWaitEvent(s2, c->ev_fork, 0));
     TVAP_CUDA(cudaStreamWaitEvent(sm, c->ev_fork, 0));
     if ((rc = prepare_uv_blocks(c, sm))) return rc;
-    if ((rc = angles_thouless(c, G, w->ephase, o.factor_delta, sm))) return rc;
+    if ((rc = angles_thouless(c, G, w->ephase, o.factor_delta, sm, true, [&]() {
+           return prepare_canonical_begin(c, o.seed_occeps, o.seed_allemp, &cq, s2);
+         })))
+      return rc;
     TVAP_CUDA(cudaEventRecord(c->ev_main, sm));
-    if ((rc = prepare_canonical(c, o.seed_occeps, o.seed_allemp, canon, s2))) return rc;
+    if ((rc = prepare_canonical_end(c, o.seed_occeps, o.seed_allemp, cq, canon, s2))) return rc;
     if (canon[2] && have_overlap) return canon_error();
     // the overlap chain (wide kernels) at the lowest priority
     cudaStream_t s3 = c->stream3;
@@ -3049,7 +3144,9 @@ int project_device(tvap_ctx* c, const tvap_proj_opts& o, tvap_pnp* out, bool syn
     // plain form: one angle per launch sequence
     sec_mark(c, s);
     if ((rc = prepare_uv_blocks(c, s))) return rc;
-    if ((rc = prepare_canonical(c, o.seed_occeps, o.seed_allemp, canon, s))) return rc;
+    CanonicalQueue cq;
+    if ((rc = prepare_canonical_begin(c, o.seed_occeps, o.seed_allemp, &cq, s))) return rc;
+    if ((rc = prepare_canonical_end(c, o.seed_occeps, o.seed_allemp, cq, canon, s))) return rc;
     if (canon[2] && have_overlap) return canon_error();
     for (int b = 0; b < G; ++b)
       if ((rc = project_angles(c, 1, w->ephase + 2 * b, w->weight + b, w->mult + b, have_overlap, canon[0],
@@ -3487,9 +3584,13 @@ int project_observables_device(tvap_ctx* c, const tvap_proj_opts& o, int nobo, c
     TVAP_CUDA(cudaStreamWaitEvent(s2, c->ev_fork, 0));
     TVAP_CUDA(cudaStreamWaitEvent(sm, c->ev_fork, 0));
     if ((r = prepare_uv_blocks(c, sm))) return r;
-    if ((r = angles_thouless(c, G, w->ephase, o.factor_delta, sm, false))) return r;
+    CanonicalQueue cq;
+    if ((r = angles_thouless(c, G, w->ephase, o.factor_delta, sm, false, [&]() {
+           return prepare_canonical_begin(c, o.seed_occeps, o.seed_allemp, &cq, s2);
+         })))
+      return r;
     TVAP_CUDA(cudaEventRecord(c->ev_main, sm));
-    if ((r = prepare_canonical(c, o.seed_occeps, o.seed_allemp, canon, s2))) return r;
+    if ((r = prepare_canonical_end(c, o.seed_occeps, o.seed_allemp, cq, canon, s2))) return r;
     if (canon[2]) {
       set_last_error("canonical basis: a degenerate subspace larger than 64 or not reducible to 2 x 2 blocks",
                      __FILE__, __LINE__);

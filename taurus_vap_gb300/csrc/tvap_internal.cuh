@@ -291,6 +291,7 @@ struct Workspace;
 // context
 // ---------------------------------------------------------------------------
 constexpr size_t kPinnedBytes = 256;
+constexpr size_t kPinnedCanonical = 256;  // behind them: the canonical basis's flags
 
 struct tvap_ctx {
   int n = 0;
@@ -321,7 +322,7 @@ struct tvap_ctx {
   // factored; ev_la[h][0] = the block row is ready, [1] = the bulk is done
   cudaStream_t streamB[2] = {nullptr, nullptr};
   cudaEvent_t ev_la[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};
-  void* h_pin = nullptr;  // pinned host buffer (kPinnedBytes) for the status word and small results
+  void* h_pin = nullptr;  // pinned host buffer (kPinnedBytes + kPinnedCanonical) for the status word and small results
   tvap::Workspace* ws = nullptr;
   int* d_flags = nullptr;  // device status word
   unsigned* d_bar = nullptr;  // grid-barrier state of the cooperative evolution (kEvolveBarWords words)
