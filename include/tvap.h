@@ -319,9 +319,10 @@ int tvap_project_observables(tvap_ctx* ctx, const double* U0, const double* V0, 
  * in the reference).  tvap_autotune times `reps` projections of (U0, V0)
  * with opts for each candidate -- column policy of the tcgen05 products (0
  * and 1: tiles of two halves of 32 columns, 2: of one half) x the
- * groups of angles in the Thouless solve (2 staggered on two streams, or 1)
- * x the cap on the tcgen05 CTAs beside the second group's panels (0: the
- * SMs the panels leave, 1: half the SMs, 2: none; 2 groups only) x the
+ * groups of angles in the Thouless solve (2: staggered on two streams where
+ * there are more angles than SMs, or 1) x the cap on the tcgen05 CTAs
+ * beside the second group's panels (0: the SMs the panels leave, 1: half the
+ * SMs, 2: none; 2 groups only) x the
  * look-ahead of the solve's panels (the bulk of each elimination product on
  * a stream of its own while the next panel is factored: on, off) x the form
  * of the overlap's Pfaffian (the shared-memory elimination where it fits, or

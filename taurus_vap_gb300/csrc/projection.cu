@@ -2338,17 +2338,21 @@ int blocked_thouless_solve(tvap_ctx* c, int G, cudaStream_t s) {
   // the block row becomes T [A12 | B1] and one product eliminates the panel
   // columns from all other rows; no back substitution follows.
   if (use_inv && (n + 31) / 32 <= kGjMaxSlots && nb <= kPanelMax) {
-    // Two halves of the angles on two streams, the second started after the
-    // first half's first panel: a panel factorisation takes the same time
-    // for any number of angles (one CTA each, latency-bound), so one half's
-    // factorisation runs beside the other half's products.  The products
-    // leave SMs for it (their CTAs are capped at the SMs the other half's
-    // panels do not hold: a panel CTA and a product CTA do not fit one SM).
-    const bool split = c->streamM2 && G >= 32 && c->tune_groups != 1;
+    // More angles than SMs: two halves of them on two streams, the second
+    // started after the first half's first panel, so that one half's panel
+    // factorisations (one CTA and SM an angle) run beside the other half's
+    // products.  The products leave SMs for them (their CTAs are capped at
+    // the SMs the other half's panels do not hold: a panel CTA and a product
+    // CTA do not fit one SM).  While the panels of all angles run at once,
+    // twice the launches of half the size cost more than the overlap gives.
+    // Iterations in one and in two halves: n = 24, 113 angles 0.640 / 0.665
+    // ms; n = 80, 39 angles 1.54 / 1.60; n = 140, 41 angles 2.96 / 3.03, 113
+    // 4.11 / 4.13, 221 6.51 / 6.47.
+    const int sms = device_sms();
+    const bool split = c->streamM2 && G > sms && c->tune_groups != 1;
     const bool la = c->tune_lookahead != 0;
     if (!split)
       return gj_solve_range(c, 0, G, nb, s, nullptr, la ? c->streamB[0] : nullptr, c->ev_la[0][0], c->ev_la[0][1]);
-    const int sms = device_sms();
     const int G1 = (G + 1) / 2, G2 = G - G1;
     TcGridCap cap(c->tune_cap == 2 ? 0 : c->tune_cap == 1 ? sms / 2 : std::max(sms - G1, sms / 2));
     if ((rc = gj_solve_range(c, 0, G1, nb, s, c->ev_stagger, la ? c->streamB[0] : nullptr, c->ev_la[0][0],

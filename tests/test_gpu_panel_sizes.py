@@ -33,3 +33,19 @@ def test_solve_panels(n):
     assert abs(e0 - e2) < 1e-9 * max(1.0, abs(e0))
     assert abs(p0.c("over") - p2.c("over")) < 1e-10 * abs(p0.c("over")) + 1e-14
     assert np.linalg.norm(h2 - h0) < 1e-9 * np.linalg.norm(h0)
+
+
+@pytest.mark.parametrize("grid", [17, 19])
+def test_two_groups_of_angles(grid):
+    # 145 and 181 folded angles: one group (at most one an SM), and two
+    mdl = M.sd_model(seed=2)
+    U, V = M.random_bogoliubov(mdl.basis, 4, 4, seed=3)
+    ctx = Context(mdl.basis, mdl.ham)
+    res = []
+    for mode in (0, 2):
+        ctx.set_gemm_mode(mode)
+        res.append(ctx.project(U, V, grid, grid, 2 * np.pi, 4, 4))
+    (p0, h0), (p2, h2) = res
+    e0, e2 = ((p.c("ener") / p.c("over")).real for p in (p0, p2))
+    assert abs(e0 - e2) < 1e-9 * max(1.0, abs(e0))
+    assert np.linalg.norm(h2 - h0) < 1e-9 * np.linalg.norm(h0)
