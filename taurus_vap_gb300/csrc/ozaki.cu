@@ -612,7 +612,7 @@ void oz_release(cudaStream_t s) {
 
 namespace {
 
-constexpr int kTcMinTiles = 152;
+constexpr int kTcMinTiles = 8;
 
 // Contraction length from which complex x complex products take the paired
 // form.  It needs half the left operand's digit planes and pads the doubled
@@ -703,11 +703,14 @@ int gemm_tc(const GemmArgs& g, cudaStream_t s) {
   if (nks > oztc::kMaxKs) return TVAP_ERR_ARG;
   const size_t asz = size_t(a_slots) * (a_rows_pad / oztc::kM) * nks * (oztc::kABytes / 2);
   const size_t bsz = size_t(b_slots) * b_halves * nks * (oztc::kBBytes / 2);
-  // products of few tiles (the single small products of the canonical basis
-  // and the evolution) are latency-bound: the 32 x 32 mma.sync tiles spread
-  // them over more SMs.  The paired form has twice the tiles of half the
-  // k-steps; it is counted in tiles of the real representation, so that both
-  // forms route the same products here.
+  // The tile route wins long before it has a tile for every SM (slicing and
+  // product, 32 x 32 mma.sync tiles / this route, us): 1024 x 640 x 140 real 53
+  // / 29, 512 x 384 x 336 real 60 / 38, 512 x 256 x 140 complex 42 / 23, 16 tiles
+  // of 512 x 256 x 140 real 28 / 29, 8 of 256 x 128 x 140 complex 43 / 23;
+  // products of fewer tiles that are not small ones (small_gemm_kernel) are
+  // thin ones.  The paired form has twice the tiles of half the k-steps; it is
+  // counted in tiles of the real representation, so that both forms route the
+  // same products here.
   if (size_t(a_rows_pad / oztc::kM) * ((b_halves + 1) / 2) * a_slots / (pairs ? 2 : 1) < size_t(kTcMinTiles))
     return TVAP_ERR_ARG;
   int rc;
