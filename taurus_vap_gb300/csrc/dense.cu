@@ -478,102 +478,7 @@ namespace {
 
 constexpr int kPfThreads = 512;
 
-__global__ void __launch_bounds__(kPfThreads) pfaffian_kernel(int N, double2* Aall, double2* pf, int batch,
-                                                              int* flags) {
-  __shared__ double sv[kPfThreads];
-  __shared__ int si[kPfThreads];
-  __shared__ double2 xcol[512], ycol[512];
-  const int b = blockIdx.x;
-  double2* A = Aall + size_t(b) * N * N;
-  auto a = [A, N](int i, int j) -> double2& { return A[size_t(i - 1) + size_t(j - 1) * N]; };
-  const int tid = threadIdx.x, nt = blockDim.x;
-  double logmag = 0.0;
-  double2 phase = make_double2(1.0, 0.0);
-  bool zero = false;
-  for (int K = N; K >= 2; K -= 2) {
-    double best = -1.0;
-    int bi = N + 1;
-    for (int i = 1 + tid; i <= K - 1; i += nt) {
-      const double v = cabs1(a(i, K));
-      if (v > best) {
-        best = v;
-        bi = i;
-      }
-    }
-    int KP;
-    double pv;
-    block_argmax(best, bi, sv, si, KP, pv);
-    if (KP > K - 1) KP = 1;  // every |a(i, K)| is NaN: IZAMAX returns the first index
-    const int KK = K - 1;
-    if (pv == 0.0) {
-      zero = true;
-      KP = KK;
-    }
-    if (KP != KK) {
-      for (int i = 1 + tid; i <= KP - 1; i += nt) {
-        const double2 t = a(i, KK);
-        a(i, KK) = a(i, KP);
-        a(i, KP) = t;
-      }
-      for (int t = tid; t < KK - KP - 1; t += nt) {
-        const double2 u = a(KP + 1 + t, KK);
-        a(KP + 1 + t, KK) = a(KP, KP + 1 + t);
-        a(KP, KP + 1 + t) = u;
-      }
-      for (int j = K + tid; j <= N; j += nt) {
-        const double2 u = a(KK, j);
-        a(KK, j) = a(KP, j);
-        a(KP, j) = u;
-      }
-      __syncthreads();
-      for (int i = KP + tid; i <= KK - 1; i += nt) a(i, KK) = cneg(a(i, KK));
-      for (int j = KP + 1 + tid; j <= KK - 1; j += nt) a(KP, j) = cneg(a(KP, j));
-      __syncthreads();
-    }
-    const double2 piv = a(K - 1, K);
-    if (!zero) {
-      const double m = hypot(piv.x, piv.y);
-      logmag += log(m);
-      phase = cmul(phase, make_double2(piv.x / m, piv.y / m));
-      if (KP != KK) phase = cneg(phase);
-      const double2 alpha = crcp(piv);
-      const int nn = K - 2;
-      for (int i = 1 + tid; i <= nn; i += nt) {
-        xcol[i] = a(i, K);
-        ycol[i] = a(i, K - 1);
-      }
-      __syncthreads();
-      // A(I,J) += X(I) * (alpha Y(J)) - Y(I) * (alpha X(J)),  I < J <= nn
-      // (ZSKR2 skips a column J whose X(J) and Y(J) are both zero);
-      // one warp per column J, lanes over I (coalesced, no index division)
-      {
-        const int warp = tid >> 5, lane = tid & 31, nw = nt >> 5;
-        for (int J = 2 + warp; J <= nn; J += nw) {
-          const double2 xj = xcol[J], yj = ycol[J];
-          if (xj.x == 0.0 && xj.y == 0.0 && yj.x == 0.0 && yj.y == 0.0) continue;
-          const double2 t1 = cmul(alpha, yj), t2 = cmul(alpha, xj);
-          double2* colJ = A + size_t(J - 1) * N;
-          for (int I = 1 + lane; I <= J - 1; I += 32) {
-            double2 v = colJ[I - 1];
-            cfma(v, xcol[I], t1);
-            cfma(v, cneg(ycol[I]), t2);
-            colJ[I - 1] = v;
-          }
-        }
-      }
-      __syncthreads();
-      for (int i = 1 + tid; i <= nn; i += nt) a(i, K) = cmul(alpha, a(i, K));
-      __syncthreads();
-    }
-  }
-  if (tid == 0) {
-    pf[b] = make_double2(zero ? -INFINITY : logmag, 0.0);
-    pf[batch + b] = zero ? make_double2(0.0, 0.0) : phase;
-    if (zero) atomicOr(flags, DEV_PFAFF_ZERO);
-  }
-}
-
-// The same elimination with the packed upper triangle in shared memory (N (N +
+// The elimination with the packed upper triangle in shared memory (N (N +
 // 1) / 2 entries, column-major).  An FP64 warp instruction holds the FP64 unit
 // of its SM sub-partition for about 64 cycles whatever lanes are active, so
 // the rank-2 update (8 N^3 / 6 of the 8 N^3 / 6 + O(N^2) FMAs) runs over the

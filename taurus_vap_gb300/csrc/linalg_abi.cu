@@ -180,7 +180,7 @@ int tvap_zskpfa_batched(tvap_ctx* c, int batch, int64_t n, const double* A, doub
     return TVAP_OK;
   }
   LaunchTally tally(c);
-  g_gemm_mode = c->gemm_mode;  // the blocked form (n > 164) updates with the context's products
+  g_gemm_mode = c->gemm_mode;  // the blocked form (n > 166) updates with the context's products
   g_tc_bn_policy = c->tune_bn;
   g_tc_pairs_min_k = c->tune_pairs_k;
   g_dev_flags = c->d_flags;

@@ -12,7 +12,6 @@
 #include <cuda_bf16.h>
 
 #include <algorithm>
-#include <climits>
 #include <mutex>
 #include <utility>
 
@@ -213,8 +212,8 @@ struct TcSlice {
 //
 // Instructions bound it, then the latency of three phases: so the divisions
 // are multiplications or shifts, a row's address is formed once, and a CTA has
-// the rows that give every thread a conversion (slice_rshift).  57 slots of
-// 256 rows of 28 complex k: 13.2 -> 8 us.
+// the rows that give every thread a conversion (slice_rshift).  57 slots of 28
+// and 252 rows of 28 complex k: 20 us in two launches -> 10.5 us in one.
 constexpr int kSliceThreads = 256;
 constexpr int kSliceMaxRows = 32;
 __global__ void __launch_bounds__(kSliceThreads)

@@ -350,7 +350,8 @@ struct tvap_ctx {
   // its last CTA leave before the first grid barrier; one-shot
   bool test_skip_arrival = false;
   // launch shapes chosen by tvap_autotune: tile columns (g_tc_bn_policy),
-  // groups of angles in the Thouless solve (2 staggered or 1), and the cap
+  // groups of angles in the Thouless solve (2: staggered where there are more
+  // angles than SMs, or 1), and the cap
   // on the tcgen05 CTAs while the second group's panels run (0: the SMs the
   // panels leave, 1: half of the SMs, 2: none)
   int tune_bn = 0;
