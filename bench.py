@@ -172,8 +172,8 @@ def host_iteration(ctx, state):
 
 # DRAM bytes (read + write) per H20 ozaki_tc_kernel launch at n = 140,
 # G = 113: the mean of ncu's dram__bytes_read.sum + dram__bytes_write.sum over
-# the three launches of one projection (593.2, 299.4 and 590.5 MB)
-H20_TRAFFIC_PER_LAUNCH = 494.4e6
+# the three launches of one projection (333.4, 172.4 and 333.3 MB)
+H20_TRAFFIC_PER_LAUNCH = 279.7e6
 
 
 FP64_PEAK_N = 4096
