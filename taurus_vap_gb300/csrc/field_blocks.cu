@@ -44,27 +44,42 @@ __device__ __forceinline__ int col_exp(const int* eb_enc, int j) {
 }
 
 // maximum exponent of every column j of the input (j < ncol: X0 column j;
-// j >= ncol: X1 column j - ncol), over all n^2 entries
-__global__ void colexp_kernel(int nent, int ncol, int ncols_tot, int ldc, const double2* __restrict__ X0,
-                              const double2* __restrict__ X1, int* __restrict__ eb_enc) {
-  __shared__ int red[8][32];
+// j >= ncol: X1 column j - ncol), over all n^2 entries.  HBM bounds it: eight
+// rows in flight a thread, a few waves of CTAs (colexp_grid), the exponent
+// fields compared as integers (a comparison of doubles is an FP64 operation).
+// 113 columns: n = 140 27 -> 9 us, n = 336 140 -> 34 us.
+constexpr int kColexpRows = 8;
+__global__ void __launch_bounds__(256) colexp_kernel(int nent, int ncol, int ncols_tot, int ldc,
+                                                     const double2* __restrict__ X0,
+                                                     const double2* __restrict__ X1, int* __restrict__ eb_enc) {
+  __shared__ unsigned red[8][32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int j = blockIdx.x * 32 + lane;
-  int e = oz::kExpZero;
+  unsigned m = 0;  // 0: zeros and subnormal numbers only
   if (j < ncols_tot) {
     const double2* X = j < ncol ? X0 + j : X1 + (j - ncol);
-    for (int p = blockIdx.y * 8 + warp; p < nent; p += gridDim.y * 8) {
-      const double2 v = X[(long long)p * ldc];
-      if (v.x != 0.0) e = max(e, oz::dexp(v.x));
-      if (v.y != 0.0) e = max(e, oz::dexp(v.y));
+    const int stride = gridDim.y * 8;
+    for (int p0 = blockIdx.y * 8 + warp; p0 < nent; p0 += kColexpRows * stride) {
+      double2 v[kColexpRows];
+#pragma unroll
+      for (int u = 0; u < kColexpRows; ++u) v[u] = X[(long long)min(p0 + u * stride, nent - 1) * ldc];
+#pragma unroll
+      for (int u = 0; u < kColexpRows; ++u)
+        m = max(m, max(unsigned(__double2hiint(v[u].x)) & 0x7ff00000u, unsigned(__double2hiint(v[u].y)) & 0x7ff00000u));
     }
   }
-  red[warp][lane] = e;
+  red[warp][lane] = m;
   __syncthreads();
   if (warp == 0) {
-    for (int w = 1; w < 8; ++w) e = max(e, red[w][lane]);
-    if (j < ncols_tot && e != oz::kExpZero) atomicMax(&eb_enc[j], e + kExpBias);
+    for (int w = 1; w < 8; ++w) m = max(m, red[w][lane]);
+    if (j < ncols_tot && m) atomicMax(&eb_enc[j], int(m >> 20) - 1023 + kExpBias);
   }
+}
+
+// its grid: about eight CTAs an SM, each with at least one round of rows
+dim3 colexp_grid(int npad, int nent) {
+  const int cols = npad / 32, rounds = (nent + 8 * kColexpRows - 1) / (8 * kColexpRows);
+  return dim3(cols, std::max(1, std::min(rounds, 8 * device_sms() / cols)));
 }
 
 // digit planes of the permuted density columns: a CTA converts a tile of 32
@@ -514,7 +529,7 @@ int apply_one_tc(tvap_ctx* c, const FieldDense& f, int ncol, int ldc, const doub
   int* counter = reinterpret_cast<int*>(xt + xt_elems);
   TVAP_CUDA(cudaMemsetAsync(eb, 0, sizeof(int) * npad, s));
   TVAP_CUDA(cudaMemsetAsync(counter, 0, sizeof(int), s));
-  colexp_kernel<<<dim3(npad / 32, 64), 256, 0, tvap::counted(s)>>>(nent, ncol, ncols_tot, ldc, X0, X1, eb);
+  colexp_kernel<<<colexp_grid(npad, nent), 256, 0, tvap::counted(s)>>>(nent, ncol, ncols_tot, ldc, X0, X1, eb);
   slice_fields_tc_kernel<DELTA><<<(f.tc_nchunks + f.tc_nempty + 3) / 4, 128, 0, tvap::counted(s)>>>(
       n, ncol, ncols_tot, ntn, ldc, X0, X1, f.colperm, f.blocks, f.tcb, f.tc_chunks, f.tc_nchunks,
       f.rowperm + f.tc_empty_base, f.tc_nempty, eb, xt, c->d_H1, out0, out1);
@@ -540,7 +555,7 @@ int apply_one(tvap_ctx* c, const FieldDense& f, int ncol, int ldc, const double2
   if ((rc = oz_scratch(s, sizeof(__nv_bfloat16) * size_t(kDigits) * 2 * npad * f.ktot, size_t(npad), &bd, &eb)))
     return rc;
   TVAP_CUDA(cudaMemsetAsync(eb, 0, sizeof(int) * npad, s));
-  colexp_kernel<<<dim3(npad / 32, 64), 256, 0, tvap::counted(s)>>>(nent, ncol, ncols_tot, ldc, X0, X1, eb);
+  colexp_kernel<<<colexp_grid(npad, nent), 256, 0, tvap::counted(s)>>>(nent, ncol, ncols_tot, ldc, X0, X1, eb);
   slice_cols_kernel<<<dim3(f.ktot / kTile, npad / kTile), 256, 0, tvap::counted(s)>>>(f.ktot, npad, ncol, ncols_tot, ldc, X0, X1,
                                                                        f.colperm, eb, bd);
   const size_t shm = oz::Shape<1, 2>::kSmemBytes;
