@@ -56,7 +56,7 @@ struct Workspace {
   int* canon_i = nullptr;
   double* canon_d = nullptr;
   // per angle complex n x n (batch G)
-  double2 *Uphi = nullptr, *Vphi = nullptr, *W = nullptr, *A = nullptr, *Ut = nullptr, *Vt = nullptr,
+  double2 *W = nullptr, *A = nullptr, *Ut = nullptr, *Vt = nullptr,
           *X = nullptr, *Y = nullptr, *T = nullptr, *Rn = nullptr, *K = nullptr, *SZ = nullptr;
   // angle-innermost (n*n*G)
   double2 *rhoL = nullptr, *kLR = nullptr, *kRL = nullptr, *gam = nullptr, *hsp = nullptr, *dLR = nullptr,
@@ -119,7 +119,7 @@ size_t tinv_stride(int n) { return size_t((n + kPanelMax - 1) / kPanelMax) * 2 *
 
 void ws_free(Workspace* w) {
   void* ptrs[] = {w->VU,  w->rho,    w->kap,   w->jac,    w->D,     w->evals,  w->jwork, w->rhoc,
-                  w->kapc, w->tmp,  w->blocks, w->canon_i, w->canon_d, w->Uphi, w->Vphi,   w->W,     w->A,
+                  w->kapc, w->tmp,  w->blocks, w->canon_i, w->canon_d, w->W,     w->A,
                   w->Ut,  w->Vt,    w->X,      w->Y,     w->T,      w->Rn,    w->K,      w->SZ,    w->rhoL,
                   w->kLR, w->kRL,   w->gam,    w->hsp,   w->dLR,    w->dRL,   w->ephase, w->weight, w->mult,
                   w->obs, w->pf,    w->detR22, w->coefA, w->coefAE, w->pA,    w->pH,     w->pAH,   w->pscal,
@@ -149,7 +149,7 @@ int ws_ensure(tvap_ctx* c, int G) {
   if ((rc = dalloc(&w->p, (cnt), t)) != TVAP_OK) return rc;
   A_(VU, 2 * nn) A_(rho, nn) A_(kap, nn) A_(jac, nn) A_(D, nn) A_(evals, n) A_(jwork, 2 * n + 2)
   A_(rhoc, nn) A_(kapc, nn) A_(tmp, nn + n) A_(blocks, 12 * nn) A_(canon_i, 8) A_(canon_d, 8 + n)
-  A_(Uphi, nG) A_(Vphi, nG) A_(W, 2 * nG) A_(A, nG) A_(Ut, nG) A_(Vt, nG) A_(X, nG) A_(Y, nG) A_(T, nG)
+  A_(W, 2 * nG) A_(A, nG) A_(Ut, nG) A_(Vt, nG) A_(X, nG) A_(Y, nG) A_(T, nG)
   A_(Rn, nG) A_(K, nG) A_(SZ, nG) A_(rhoL, nG) A_(kLR, nG) A_(kRL, nG) A_(gam, nG) A_(hsp, nG) A_(dLR, nG)
   A_(dRL, nG) A_(ephase, 2 * G) A_(weight, G) A_(mult, G) A_(obs, 8 * G) A_(pf, 2 * G) A_(detR22, 2 * G)
   A_(coefA, G) A_(coefAE, G) A_(pA, nn) A_(pH, nn) A_(pAH, nn) A_(pscal, 8) A_(H20v, nn)
@@ -441,32 +441,34 @@ __global__ void canon_kernel(int n, const double* __restrict__ rhoc, double* __r
   }
 }
 
-// per angle: U_phi, V_phi from the angle-independent blocks of U and V
-__global__ void build_uv_kernel(int n, int G, const double* __restrict__ blk, const double2* __restrict__ eph,
-                                double2* __restrict__ Uphi, double2* __restrict__ Vphi) {
-  const size_t nn = size_t(n) * n;
-  const size_t idx = blockIdx.x * size_t(blockDim.x) + threadIdx.x;
-  if (idx >= nn * G) return;
-  const int b = int(idx / nn);
-  const size_t e = idx % nn;
-  const double2 pp = eph[2 * b], pn = eph[2 * b + 1];  // e^{i phi_p}, e^{i phi_n}
+// The augmented systems W = [U_phi^T | V_phi^T] (n x 2n, one per angle) from
+// the angle-independent blocks of U and V.  A thread forms one entry of both
+// halves for kSysAngles angles: the eight sums of blocks, half of an entry's
+// FP64 operations (which bound it), once for all of them.
+// U_phi and V_phi are never stored.  113 angles of n = 140: 98 us in two kernels -> 44 us.
+constexpr int kSysAngles = 8;
+__global__ void __launch_bounds__(256)
+    build_system_kernel(int n, int G, const double* __restrict__ blk, const double2* __restrict__ eph,
+                        double2* __restrict__ Wall) {
+  const int nn = n * n;
+  const int e = blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= nn) return;
+  const int r = e % n, c = e / n;  // W(r, c) = U_phi(c, r), W(r, n + c) = V_phi(c, r)
   // blocks: the Gram matrices C_t = W_t^T W_t of W_t = [V_t | U_t] (rows of
   // isospin t; 2n x 2n at blk + 4 n^2 t), then D_p^T D_p, D_n^T D_n
-  const int i = int(e % n), j = int(e / n);
-  const size_t n2 = 2 * size_t(n);
+  const int i = c, j = r, n2 = 2 * n;
   const double* Cp = blk;
-  const double* Cn = blk + 4 * nn;
-  const size_t vv = i + j * n2, vu = i + (n + j) * n2, uv = (n + i) + j * n2, uu = (n + i) + (n + j) * n2;
-  const double vvp = Cp[vv], vvn = Cn[vv], uup = Cp[uu], uun = Cn[uu];
-  const double vup = Cp[vu], vun = Cn[vu], uvp = Cp[uv], uvn = Cn[uv];
-  double2 up;
-  up.x = (vvp + uup) * pp.x + (vvn + uun) * pn.x;
-  up.y = (uup - vvp) * pp.y + (uun - vvn) * pn.y;
-  double2 vp;
-  vp.x = (vup + uvp) * pp.x + (vun + uvn) * pn.x;
-  vp.y = (vup - uvp) * pp.y + (vun - uvn) * pn.y;
-  Uphi[idx] = up;
-  Vphi[idx] = vp;
+  const double* Cn = blk + 4 * size_t(nn);
+  const int vv = i + j * n2, vu = i + (n + j) * n2, uv = (n + i) + j * n2, uu = (n + i) + (n + j) * n2;
+  const double upx = Cp[vv] + Cp[uu], upy = Cp[uu] - Cp[vv], unx = Cn[vv] + Cn[uu], uny = Cn[uu] - Cn[vv];
+  const double vpx = Cp[vu] + Cp[uv], vpy = Cp[vu] - Cp[uv], vnx = Cn[vu] + Cn[uv], vny = Cn[vu] - Cn[uv];
+  const int b1 = min(G, (int(blockIdx.y) + 1) * kSysAngles);
+  for (int b = blockIdx.y * kSysAngles; b < b1; ++b) {
+    const double2 pp = eph[2 * b], pn = eph[2 * b + 1];  // e^{i phi_p}, e^{i phi_n}
+    double2* W = Wall + size_t(b) * 2 * nn;
+    W[e] = make_double2(upx * pp.x + unx * pn.x, upy * pp.y + uny * pn.y);
+    W[nn + e] = make_double2(vpx * pp.x + vnx * pn.x, vpy * pp.y + vny * pn.y);
+  }
 }
 
 // per angle: the trailing n2 x n2 block (n2 = n - nemp) of R_n = D^T R D
@@ -1411,20 +1413,6 @@ __device__ __forceinline__ void warp_argmax(double& v, int& i) {
 }
 
 __global__ void __launch_bounds__(kPanelThreads)
-    build_augmented_kernel(int n, const double2* __restrict__ Uphi, const double2* __restrict__ Vphi,
-                           double2* __restrict__ Wall) {
-  const int b = blockIdx.y;
-  const size_t nn = size_t(n) * n;
-  double2* W = Wall + b * 2 * nn;
-  const double2* U = Uphi + b * nn;
-  const double2* V = Vphi + b * nn;
-  // W(r, c) = U(c, r);  W(r, n + c) = V(c, r)
-  for (int c = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); c < 2 * n; c += gridDim.x * (blockDim.x >> 5))
-    for (int r = threadIdx.x & 31; r < n; r += 32)
-      W[r + size_t(c) * n] = (c < n) ? U[c + size_t(r) * n] : V[(c - n) + size_t(r) * n];
-}
-
-__global__ void __launch_bounds__(kPanelThreads)
     panel_kernel(int n, int j0, int nbp, double2* __restrict__ Wall, int* flags) {
   __shared__ double wv[kPanelThreads / 32];
   __shared__ int wi[kPanelThreads / 32];
@@ -2179,7 +2167,7 @@ int real_gemm(int M, int N, int K, View A, View B, double* C, int ldc, double al
 
 // Gauss-Jordan solve of angles [g0, g0 + gc) on stream s (panels of nb
 // columns); ev_first, when given, is recorded after the first panel's
-// factorisation.  build_augmented_kernel has filled W.
+// factorisation.  build_system_kernel has filled W.
 // sb (may be null): a stream for the look-ahead -- the elimination product
 // of panel k splits into the next panel's columns (on s, so that panel k+1 is
 // factored right after them) and the rest (on sb, beside that factorisation;
@@ -2308,10 +2296,6 @@ int blocked_thouless_solve(tvap_ctx* c, int G, cudaStream_t s) {
   int rc;
   if (smem_path && panel_bytes > 48 * 1024) {
     if (int r = smem_opt_in((const void*)panel_factor_kernel, jacobi32_smem_limit())) return r;
-  }
-  {
-    dim3 grid(std::max(1, (2 * n + 15) / 16), G);
-    build_augmented_kernel<<<grid, kPanelThreads, 0, tvap::counted(s)>>>(n, w->Uphi, w->Vphi, w->W);
   }
   // product with an inverted diagonal block, in place on a block row:
   // rows r0 .. r0+nbp-1 of columns c0 .. 2n-1 <- T (nbp x nbp) times them
@@ -2841,7 +2825,8 @@ int angles_thouless(tvap_ctx* c, int G, const double2* d_ephase, double factor_d
   const int tb = 256;
   int rc;
   sec_begin_on(c, SEC_SOLVE, s);
-  build_uv_kernel<<<nblk(nn * G, tb), tb, 0, tvap::counted(s)>>>(n, G, w->blocks, d_ephase, w->Uphi, w->Vphi);
+  build_system_kernel<<<dim3(nblk(nn, 256), (G + kSysAngles - 1) / kSysAngles), 256, 0, tvap::counted(s)>>>(
+      n, G, w->blocks, d_ephase, w->W);
   TVAP_CUDA(cudaGetLastError());
   // A_phi = conj(V_phi U_phi^{-1}): solve U_phi^T Y = V_phi^T, A = conj(Y^T)
   if ((rc = blocked_thouless_solve(c, G, s))) return rc;
