@@ -964,6 +964,9 @@ __global__ void schur_kernel(int n2, int nb, int G, const double2* __restrict__ 
 // shared memory in a fixed order: an SM retires two FP64 operations a cycle,
 // so that one CTA took 43 us for the three norms at n = 140.  Comparisons of
 // doubles, FP64 operations too, are made on their bits.
+// (Another CTA's shared memory exists only once that CTA has started, which a
+// cluster barrier shows: each arrives at one on entry and waits for it just
+// before its first remote store, the time of its own reduction between them.)
 constexpr int kRlCtas = 8;
 constexpr int kRlThreads = 512;
 // a double's bits as an integer of the same order (-0 below +0)
@@ -982,6 +985,7 @@ __global__ void __cluster_dims__(kRlCtas, 1, 1) __launch_bounds__(kRlThreads)
   __shared__ double red[3][kRlThreads / 32], gathered[kRlCtas][3];
   cg::cluster_group cluster = cg::this_cluster();
   const int rank = int(cluster.block_rank());
+  cluster.barrier_arrive();  // this CTA has started; waited for before CTA 0's shared memory is written
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int g = rank * kRlThreads + tid, ng = kRlCtas * kRlThreads;
   for (int i = g; i < n; i += ng) lam[i] = S[i + size_t(i) * n] / XtX[i + size_t(i) * n];
@@ -1023,6 +1027,7 @@ __global__ void __cluster_dims__(kRlCtas, 1, 1) __launch_bounds__(kRlThreads)
     red[2][warp] = s_a;
   }
   __syncthreads();
+  cluster.barrier_wait();
   if (tid < 3) {
     double t = 0.0;
     for (int w2 = 0; w2 < kRlThreads / 32; ++w2) t += red[tid][w2];
@@ -1224,6 +1229,7 @@ __global__ void __cluster_dims__(kRlCtas, 1, 1) __launch_bounds__(kCfThreads)
   __shared__ unsigned long long red[kCfThreads / 32], gathered[kRlCtas];
   cg::cluster_group cluster = cg::this_cluster();
   const int rank = int(cluster.block_rank());
+  cluster.barrier_arrive();  // (as in refine_lambda_kernel)
   const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, warp = tid >> 5, nwarp = nt >> 5;
   if (tid == 0) {
     fail = 0;
@@ -1288,6 +1294,7 @@ __global__ void __cluster_dims__(kRlCtas, 1, 1) __launch_bounds__(kCfThreads)
   for (int o = 16; o > 0; o >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
   if (lane == 0) red[warp] = mx;
   __syncthreads();
+  cluster.barrier_wait();
   if (tid == 0) {
     for (int w2 = 1; w2 < nwarp; ++w2) mx = max(mx, red[w2]);
     *cluster.map_shared_rank(&gathered[rank], 0) = mx;
