@@ -137,7 +137,7 @@ __global__ void __launch_bounds__((TM / 2) * (TN / 2)) gemm_kernel(GemmArgs g) {
 #pragma unroll
     for (int c = 0; c < 2; ++c) {
       const int i = i0 + ty + r * HM, j = j0 + tx + c * HN;
-      if (i < g.M && j < g.N) {
+      if (i < g.M && j < g.N && g.writes_row(i)) {
         const long long idx = i * g.crs + j * g.ccs + b * g.cbs;
         if constexpr (sizeof(TC) == sizeof(double)) {
           store_out(g, idx, acc[r][c], alpha);
@@ -208,7 +208,7 @@ __global__ void __launch_bounds__((TM / 2) * (TN / 2)) gemm3m_kernel(GemmArgs g)
 #pragma unroll
     for (int c = 0; c < 2; ++c) {
       const int i = i0 + ty + r * HM, j = j0 + tx + c * HN;
-      if (i < g.M && j < g.N) {
+      if (i < g.M && j < g.N && g.writes_row(i)) {
         const long long idx = i * g.crs + j * g.ccs + b * g.cbs;
         const double2 acc = make_double2(t1[r][c] - t2[r][c], t3[r][c] - t1[r][c] - t2[r][c]);
         store_out(g, idx, acc, alpha);
@@ -303,7 +303,7 @@ __global__ void __launch_bounds__(kSmallThreads) small_gemm_kernel(GemmArgs g, u
   if constexpr (M3) acc = make_double2(t1 - t2, t3 - t1 - t2);
   if (part == 1) half[out] = acc;
   __syncthreads();
-  if (part == 1 || i0 + i >= g.M || j0 + j >= g.N) return;
+  if (part == 1 || i0 + i >= g.M || j0 + j >= g.N || !g.writes_row(i0 + i)) return;
   double2 alpha = g.alpha;
   if (g.alpha_vec) alpha = cmul(alpha, g.alpha_vec[b]);
   const long long idx = (i0 + i) * g.crs + (j0 + j) * g.ccs + b * g.cbs;

@@ -38,6 +38,7 @@
 #include <functional>
 #include <vector>
 
+#include "gj_elimination.h"
 #include "tvap_internal.cuh"
 
 namespace cg = cooperative_groups;
@@ -2244,36 +2245,18 @@ int gj_solve_range(tvap_ctx* c, int g0, int gc, int nb, cudaStream_t s, cudaEven
       g.beta = make_double2(0.0, 0.0);
       if ((rc = gemm_ozaki(g, s))) return rc;
     }
-    // all other rows: W[:, j1:] -= W[:, j0:j1] R (the block rows' panel
-    // entries are zero, so they keep R)
-    GemmArgs g{};
-    g.M = n;
-    g.N = 2 * n - j1;
-    g.K = nbp;
-    g.batch = gc;
-    g.A = View{W + size_t(j0) * n, 1, n, bsW};
-    g.B = View{W + j0 + size_t(j1) * n, 1, n, bsW};
-    g.C = W + size_t(j1) * n;
-    g.crs = 1;
-    g.ccs = n;
-    g.cbs = bsW;
-    g.alpha = make_double2(-1.0, 0.0);
-    g.beta = make_double2(1.0, 0.0);
-    g.three_m = true;
+    // all other rows: W[:, j1:] -= W[:, j0:j1] R
     const int j2 = j1 + std::min(nb, n - j1);  // the next panel's columns end
+    int c1 = 2 * n;
     if (sb && j1 < n) {
       // look-ahead: columns j2 .. 2n-1 on sb, then j1 .. j2-1 on s
       TVAP_CUDA(cudaEventRecord(ev_ready, s));
       TVAP_CUDA(cudaStreamWaitEvent(sb, ev_ready, 0));
-      GemmArgs gb = g;
-      gb.N = 2 * n - j2;
-      gb.B = View{W + j0 + size_t(j2) * n, 1, n, bsW};
-      gb.C = W + size_t(j2) * n;
-      if ((rc = gemm(gb, sb))) return rc;
+      if ((rc = gemm(gj_elimination(n, j0, nbp, j2, 2 * n, gc, W), sb))) return rc;
       TVAP_CUDA(cudaEventRecord(ev_bulk, sb));
-      g.N = j2 - j1;
+      c1 = j2;
     }
-    if ((rc = gemm(g, s))) return rc;
+    if ((rc = gemm(gj_elimination(n, j0, nbp, j1, c1, gc, W), s))) return rc;
   }
   const size_t tot = nn * gc;
   thouless_out_kernel<<<nblk(tot, 256), 256, 0, tvap::counted(s)>>>(n, gc, W, w->A + size_t(g0) * nn);

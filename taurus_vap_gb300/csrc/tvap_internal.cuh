@@ -187,6 +187,13 @@ struct GemmArgs {
   // is the previous tcgen05 product's on this stream, unchanged since: its
   // digit planes are reused (checked against the recorded operand)
   bool reuse_left;
+  // rows keep0 .. keep0 + keep_rows - 1 of C stay as they are (their rows of
+  // op(A) are zeros and beta is 1).  C may overlap an operand there and only
+  // there: the kernels on the FP64 pipe, which read the operands while other
+  // CTAs store, do not touch these rows; the emulated forms split the operands
+  // into digit planes first (and may store the same values again).
+  int keep0, keep_rows;
+  __host__ __device__ bool writes_row(int i) const { return unsigned(i - keep0) >= unsigned(keep_rows); }
 };
 int gemm(const GemmArgs& g, cudaStream_t s);
 // the two terms of a product with K2 > 0 as two products
