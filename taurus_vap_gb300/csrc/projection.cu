@@ -3044,9 +3044,9 @@ int sync_with_flags(tvap_ctx* c, void* dst, const void* src, size_t bytes) {
 
 int check_flags(tvap_ctx* c) { return sync_with_flags(c, nullptr, nullptr, 0); }
 
-// Full projection of state (w->U, w->V) already on the device.  Leaves the
-// sums in w->pscal/pA/pH/pAH and the gradient in w->H20v.
-int project_device(tvap_ctx* c, const tvap_proj_opts& o, tvap_pnp* out, bool sync) {
+namespace {
+
+int project_chains(tvap_ctx* c, const tvap_proj_opts& o, tvap_pnp* out, bool sync) {
   const int n = c->n;
   const size_t nn = size_t(n) * n;
   cudaStream_t s = c->stream, s2 = c->stream2;
@@ -3157,6 +3157,14 @@ int project_device(tvap_ctx* c, const tvap_proj_opts& o, tvap_pnp* out, bool syn
     return rc;
   }
   return check_flags(c);
+}
+
+}  // namespace
+
+// Full projection of state (w->U, w->V) already on the device.  Leaves the
+// sums in w->pscal/pA/pH/pAH and the gradient in w->H20v.
+int project_device(tvap_ctx* c, const tvap_proj_opts& o, tvap_pnp* out, bool sync) {
+  return settle(c, project_chains(c, o, out, sync));
 }
 
 // ---------------------------------------------------------------------------
@@ -3702,7 +3710,7 @@ int project_observables_device(tvap_ctx* c, const tvap_proj_opts& o, int nobo, c
     for (int k = 0; k < 2 * nshell; ++k) occ_out[k] = hs[8 + 2 * ntr + nsq + k];
     return TVAP_OK;
   };
-  rc = run();
+  rc = settle(c, run());
   if (rc == TVAP_OK) TVAP_CUDA(cudaStreamSynchronize(s));
   return rc;
 }

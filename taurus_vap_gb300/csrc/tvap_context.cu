@@ -79,6 +79,19 @@ double* ws_U(tvap_ctx* c);
 double* ws_V(tvap_ctx* c);
 double* ws_H20v(tvap_ctx* c);
 
+void sync_streams(tvap_ctx* c) {
+  for (cudaStream_t st : {c->stream, c->stream2, c->stream3, c->streamM, c->streamM2, c->streamB[0], c->streamB[1]})
+    if (st) cudaStreamSynchronize(st);
+}
+
+int settle(tvap_ctx* c, int rc) {
+  if (rc == TVAP_OK) return rc;
+  sync_streams(c);
+  cudaMemsetAsync(c->d_flags, 0, sizeof(int), c->stream);
+  cudaGetLastError();  // (the call's error has its code and text)
+  return rc;
+}
+
 static cudaEvent_t take_event(tvap_ctx* c) {
   if (!c->ev_pool.empty()) {
     cudaEvent_t e = c->ev_pool.back();
@@ -317,13 +330,7 @@ int tvap_init(tvap_ctx** ctx, int64_t n, const int32_t* sp_2mj, const int32_t* s
 
 void tvap_destroy(tvap_ctx* c) {
   if (!c) return;
-  if (c->stream) cudaStreamSynchronize(c->stream);
-  if (c->stream2) cudaStreamSynchronize(c->stream2);
-  if (c->stream3) cudaStreamSynchronize(c->stream3);
-  if (c->streamM) cudaStreamSynchronize(c->streamM);
-  if (c->streamM2) cudaStreamSynchronize(c->streamM2);
-  for (auto sb : c->streamB)
-    if (sb) cudaStreamSynchronize(sb);
+  sync_streams(c);
   cudaFree(c->scratch);
   destroy_workspace(c);
   free_field_csr(c->csr);
@@ -490,7 +497,7 @@ int tvap_calculate_fields_batched(tvap_ctx* c, int ncol, const double* rho, cons
     TVAP_CUDA(cudaGetLastError());
     return TVAP_OK;
   };
-  int rc = run();
+  int rc = settle(c, run());
   if (rc == TVAP_OK) {
     const cudaError_t e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) {

@@ -383,6 +383,13 @@ enum Section : int {
   SEC_CANONICAL = 0, SEC_BLOCKS, SEC_SOLVE, SEC_UV, SEC_DENSITIES, SEC_FIELDS_GAMMA, SEC_FIELDS_DELTA, SEC_TRACES,
   SEC_H20, SEC_OVERLAP, SEC_PFAFFIAN, SEC_SUMS, SEC_GRADIENT, SEC_EVOLVE, SEC_H20_TC, SEC_COUNT
 };
+// Waits for every stream of the context.
+void sync_streams(tvap_ctx* c);
+// The result of a call that forks chains onto the context's streams: on an
+// error (returned from between the fork and the join) the chains are waited for
+// and the status word is cleared, so that nothing of the call writes the
+// workspace, the caller's arrays or a status bit beside the next one.
+int settle(tvap_ctx* c, int rc);
 // brackets a section with events when timing is on (no-ops otherwise)
 void sec_begin(tvap_ctx* c, int sec);
 void sec_end(tvap_ctx* c, int sec);
