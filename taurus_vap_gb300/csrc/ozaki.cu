@@ -613,12 +613,7 @@ namespace {
 
 constexpr int kTcMinTiles = 8;
 
-// Contraction length from which complex x complex products take the paired
-// form.  It needs half the left operand's digit planes and pads the doubled
-// columns instead of the columns (n = 140: 288 for 2 x 160), at twice the
-// tiles of half the k-steps: as many folds once the real representation's 2 K
-// exceed one fold interval, twice as many below.
-constexpr int kPairsMinK = oztc::kFoldKs * 16 / 2 + 1;
+static_assert(kPairsMinK == oztc::kFoldKs * 16 / 2 + 1, "the paired form from half a fold interval on");
 
 inline bool g_alpha_unit(double a) { return a == 1.0 || a == -1.0; }
 
@@ -666,7 +661,7 @@ int gemm_tc(const GemmArgs& g, cudaStream_t s) {
   // complex x complex: the paired form (rows interleaved on both sides, the
   // 2 x 2 blocks combined by the epilogue) or the real representation; batches
   // with a shared operand keep the real representation
-  const bool pairs = !L.real && !R.real && !stack && K >= (g_tc_pairs_min_k > 0 ? g_tc_pairs_min_k : kPairsMinK);
+  const bool pairs = !L.real && !R.real && !stack && complex_pairs(K, g_tc_pairs_min_k);
   if (pairs) {
     xa.form = xb.form = 4;
     o.a_mult = o.b_mult = 2;

@@ -216,9 +216,16 @@ extern thread_local int g_tc_grid_cap;
 extern thread_local int g_tc_bn_policy;
 // the tcgen05 complex x complex products of contraction length >= this take
 // the paired form (real and imaginary rows interleaved on both sides), the
-// others the real representation [[Re, -Im], [Im, Re]] x [Re, Im]; 0: from
-// kPairsMinK on (set by every entry point from its context)
+// others the real representation [[Re, -Im], [Im, Re]] x [Re, Im]; 0: none
+// (set by every entry point from its context)
 extern thread_local int g_tc_pairs_min_k;
+inline bool complex_pairs(int K, int min_k) { return min_k > 0 && K >= min_k; }
+// Its value in a new context.  The paired form needs half the left operand's
+// digit planes and pads the doubled columns instead of the columns (n = 140:
+// 288 for 2 x 160), at twice the tiles of half the k-steps: as many folds once
+// the real representation's 2 K exceed one fold interval (160), twice as many
+// below.
+constexpr int kPairsMinK = 81;
 struct TcGridCap {
   int saved;
   explicit TcGridCap(int cap) : saved(g_tc_grid_cap) { g_tc_grid_cap = cap; }
@@ -366,7 +373,8 @@ struct tvap_ctx {
   int tune_cap = 0;
   int tune_lookahead = 0;  // look-ahead of the Thouless solve's panels (streamB)
   int tune_pf_blocked = 0;  // the blocked Pfaffian also where the shared-memory one fits
-  int tune_pairs_k = 0;     // complex x complex tcgen05 products in the paired form from K = this on (0: kPairsMinK)
+  // complex x complex tcgen05 products in the paired form from K = this on (0: none)
+  int tune_pairs_k = tvap::kPairsMinK;
 };
 
 namespace tvap {

@@ -370,8 +370,9 @@ class Context:
                                            int(lib().tvap_get_option(self.h, self.OPT_PFAFFIAN_BLOCKED)))
 
     def set_option(self, option, value):
-        """tvap_set_option (OPT_SOLVE_LOOKAHEAD, OPT_PFAFFIAN_BLOCKED,
-        OPT_COMPLEX_PAIRS; 0 or 1)."""
+        """tvap_set_option: OPT_SOLVE_LOOKAHEAD and OPT_PFAFFIAN_BLOCKED, 0
+        or 1; OPT_COMPLEX_PAIRS, the contraction length from which complex
+        products take the paired form (81 in a new context; 0: none)."""
         _check(lib().tvap_set_option(self.h, option, value), "tvap_set_option")
 
     def option(self, option):
