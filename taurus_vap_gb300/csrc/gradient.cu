@@ -11,6 +11,7 @@
 
 #include <cmath>
 
+#include "evolve_route.h"
 #include "tvap_internal.cuh"
 
 namespace tvap {
@@ -80,18 +81,18 @@ int rgemm(int M, int N, int K, View A, View B, double* C, int ldc, double alpha,
 
 // U1 = (U0 + V0 Z) L^{-T}, V1 = (V0 + U0 Z) L^{-T} with L L^T = 1 + Z^T Z, and
 // L^{-1} when Linv is not null; work holds evolve_work(n) doubles.  One
-// cooperative launch, which also forms the products where n allows it; above
-// its range the single-CTA inverse and two products.
+// cooperative launch, which also forms the products where n allows it; where
+// it does not run the single-CTA inverse and two products.
 int evolve_device(tvap_ctx* c, const double* Z, const double* U0, const double* V0, double* work, int n, double* U1,
                   double* V1, double* Linv) {
   cudaStream_t s = c->stream;
   const size_t nn = size_t(n) * n;
   double *A = work, *S = work + 2 * nn;
-  int rc;
   sec_begin(c, SEC_EVOLVE);
-  if (!evolve_forms_products(n)) {
+  auto products = [&]() -> int {
+    int r;
     const View Zv = view_cm(Z, n, 0);
-    if ((rc = rgemm(n, n, n, view_t(Zv), Zv, S, n, 1.0, 0.0, s))) return rc;
+    if ((r = rgemm(n, n, n, view_t(Zv), Zv, S, n, 1.0, 0.0, s))) return r;
     add_identity_kernel<<<(n + 255) / 256, 256, 0, tvap::counted(s)>>>(n, S);
     TVAP_CUDA(cudaMemcpyAsync(A, U0, sizeof(double) * nn, cudaMemcpyDeviceToDevice, s));
     TVAP_CUDA(cudaMemcpyAsync(A + nn, V0, sizeof(double) * nn, cudaMemcpyDeviceToDevice, s));
@@ -107,20 +108,23 @@ int evolve_device(tvap_ctx* c, const double* Z, const double* U0, const double* 
     g.alpha = make_double2(1.0, 0.0);
     g.beta = make_double2(1.0, 0.0);
     g.a_real = g.b_real = g.c_real = true;
-    if ((rc = gemm(g, s))) return rc;
-  }
-  const int skip = c->test_skip_arrival ? 1 : -1;
-  c->test_skip_arrival = false;
-  rc = thouless_evolve(n, Z, U0, V0, work, U1, V1, Linv, c->d_bar, c->d_flags, s, skip);
-  if (rc == TVAP_ERR_ARG) {
-    if ((rc = cholesky_inverse(n, S, c->d_flags, s))) return rc;
+    return gemm(g, s);
+  };
+  auto coop = [&]() -> int {
+    const int skip = c->test_skip_arrival ? 1 : -1;
+    c->test_skip_arrival = false;
+    return thouless_evolve(n, Z, U0, V0, work, U1, V1, Linv, c->d_bar, c->d_flags, s, skip);
+  };
+  auto single = [&]() -> int {
+    int r;
+    if ((r = cholesky_inverse(n, S, c->d_flags, s))) return r;
     const View LinvT = view_t(view_cm(S, n, 0));
-    if ((rc = rgemm(n, n, n, view_cm(A, n, 0), LinvT, U1, n, 1.0, 0.0, s))) return rc;
-    if ((rc = rgemm(n, n, n, view_cm(A + nn, n, 0), LinvT, V1, n, 1.0, 0.0, s))) return rc;
+    if ((r = rgemm(n, n, n, view_cm(A, n, 0), LinvT, U1, n, 1.0, 0.0, s))) return r;
+    if ((r = rgemm(n, n, n, view_cm(A + nn, n, 0), LinvT, V1, n, 1.0, 0.0, s))) return r;
     if (Linv) TVAP_CUDA(cudaMemcpyAsync(Linv, S, sizeof(double) * nn, cudaMemcpyDeviceToDevice, s));
-  } else if (rc) {
-    return rc;
-  }
+    return TVAP_OK;
+  };
+  if (const int rc = evolve_route(evolve_forms_products(n), products, coop, single)) return rc;
   sec_end(c, SEC_EVOLVE);
   return TVAP_OK;
 }
