@@ -269,11 +269,15 @@ def run_ours(args):
         proposed = ctx.tuning()
         # the tuner ranks projections, whose best shapes lie within about 1 %
         # of each other; the timed step also evolves the state and reads its
-        # results back.  Its three best and the context's defaults are timed
-        # again on whole iterations (3 alternating rounds of 8) and the
-        # fastest is kept.
-        cands = [k for k, _ in sorted(tune_table.items(), key=lambda kv: kv[1])[:3]]
-        if DEFAULT_TUNING not in cands:
+        # results back.  Its three best programs (candidates that launch the
+        # same one share its time) and the context's defaults are timed again
+        # on whole iterations (3 alternating rounds of 8) and the fastest is
+        # kept.
+        by_time = {}
+        for k, t in tune_table.items():
+            by_time.setdefault(t, k)
+        cands = [by_time[t] for t in sorted(by_time)[:3]]
+        if by_time[tune_table[DEFAULT_TUNING]] not in cands:
             cands.append(DEFAULT_TUNING)
         it_ms = {cnd: [] for cnd in cands}
         itc = DeviceIteration(ctx, U, V, 0, torch)

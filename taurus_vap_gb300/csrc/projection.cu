@@ -2264,24 +2264,64 @@ int gj_solve_range(tvap_ctx* c, int g0, int gc, int nb, cudaStream_t s, cudaEven
   return TVAP_OK;
 }
 
+namespace {
+
+// The panels of the solve: at most kPanelMax columns, equal widths; the
+// shared-memory panel (n x nb complex) must fit, else the former wider
+// kernels run from global memory.  With the emulated products, the triangular
+// solves of the block rows and of the back substitution run as products with
+// the inverted diagonal blocks (computed by the panel kernel) on the tensor
+// cores; on the FP64 pipe they stay one-thread-per-column substitutions.
+struct Panels {
+  int nb;
+  size_t bytes;
+  bool smem_path, use_inv;
+};
+Panels solve_panels(int n, int gemm_mode) {
+  const int npanels = (n + kPanelMax - 1) / kPanelMax, nb = (n + npanels - 1) / npanels;
+  const bool inv_path = gemm_mode >= 1;
+  Panels p{};
+  p.bytes = sizeof(double2) * (size_t(n) * nb + (inv_path ? 2 * size_t(nb) * nb : 0));
+  p.smem_path = p.bytes <= size_t(jacobi32_smem_limit());
+  p.use_inv = inv_path && p.smem_path;
+  p.nb = p.smem_path ? nb : (n <= 64) ? n : 28;
+  return p;
+}
+
+}  // namespace
+
+// Blocked Gauss-Jordan: the emulated products, panels of up to 384 rows.
+// More angles than SMs: two halves of them on two streams, the second
+// started after the first half's first panel, so that one half's panel
+// factorisations (one CTA and SM an angle) run beside the other half's
+// products.  The products leave SMs for them (their CTAs are capped at
+// the SMs the other half's panels do not hold: a panel CTA and a product
+// CTA do not fit one SM).  While the panels of all angles run at once,
+// twice the launches of half the size cost more than the overlap gives.
+// Iterations in one and in two halves: n = 24, 113 angles 0.640 / 0.665
+// ms; n = 80, 39 angles 1.54 / 1.60; n = 140, 41 angles 2.96 / 3.03, 113
+// 4.11 / 4.13, 221 6.51 / 6.47.
+// The look-ahead has a panel to work on where there are two.
+SolveShape solve_shape(int n, int G, int gemm_mode, int groups, int cap, int lookahead) {
+  const Panels p = solve_panels(n, gemm_mode);
+  SolveShape q{};
+  q.gauss_jordan = p.use_inv && (n + 31) / 32 <= kGjMaxSlots && p.nb <= kPanelMax;
+  if (!q.gauss_jordan) return q;
+  const int sms = device_sms();
+  q.split = G > sms && groups != 1;
+  if (q.split) q.cap = cap == 2 ? 0 : cap == 1 ? sms / 2 : std::max(sms - (G + 1) / 2, sms / 2);
+  q.lookahead = lookahead != 0 && p.nb < n;
+  return q;
+}
+
 int blocked_thouless_solve(tvap_ctx* c, int G, cudaStream_t s) {
   Workspace* w = c->ws;
   const int n = c->n;
   const long long bsW = 2LL * n * n;
-  // panels of at most kPanelMax columns, equal widths; the shared-memory panel
-  // (n x nb complex) must fit, else the former wider kernels run from global
-  const int npanels = (n + kPanelMax - 1) / kPanelMax;
-  const int nb_smem = (n + npanels - 1) / npanels;
-  // with the emulated products, the triangular solves of the block rows and
-  // of the back substitution run as products with the inverted diagonal
-  // blocks (computed by the panel kernel) on the tensor cores; on the FP64
-  // pipe they stay one-thread-per-column substitutions
-  const bool inv_path = g_gemm_mode >= 1;
-  const size_t panel_bytes =
-      sizeof(double2) * (size_t(n) * nb_smem + (inv_path ? 2 * size_t(nb_smem) * nb_smem : 0));
-  const bool smem_path = panel_bytes <= size_t(jacobi32_smem_limit());
-  const bool use_inv = inv_path && smem_path;
-  const int nb = smem_path ? nb_smem : ((n <= 64) ? n : 28);
+  const Panels panels = solve_panels(n, g_gemm_mode);
+  const size_t panel_bytes = panels.bytes;
+  const bool smem_path = panels.smem_path, use_inv = panels.use_inv;
+  const int nb = panels.nb;
   const long long tstride = (long long)tinv_stride(n);
   int rc;
   if (smem_path && panel_bytes > 48 * 1024) {
@@ -2307,28 +2347,16 @@ int blocked_thouless_solve(tvap_ctx* c, int G, cudaStream_t s) {
     g.beta = make_double2(0.0, 0.0);
     return gemm_ozaki(g, s);
   };
-  // Blocked Gauss-Jordan (the emulated products, panels of up to 192 rows):
-  // per panel the factor kernel chooses the pivots and forms T = A11^{-1},
-  // the block row becomes T [A12 | B1] and one product eliminates the panel
-  // columns from all other rows; no back substitution follows.
-  if (use_inv && (n + 31) / 32 <= kGjMaxSlots && nb <= kPanelMax) {
-    // More angles than SMs: two halves of them on two streams, the second
-    // started after the first half's first panel, so that one half's panel
-    // factorisations (one CTA and SM an angle) run beside the other half's
-    // products.  The products leave SMs for them (their CTAs are capped at
-    // the SMs the other half's panels do not hold: a panel CTA and a product
-    // CTA do not fit one SM).  While the panels of all angles run at once,
-    // twice the launches of half the size cost more than the overlap gives.
-    // Iterations in one and in two halves: n = 24, 113 angles 0.640 / 0.665
-    // ms; n = 80, 39 angles 1.54 / 1.60; n = 140, 41 angles 2.96 / 3.03, 113
-    // 4.11 / 4.13, 221 6.51 / 6.47.
-    const int sms = device_sms();
-    const bool split = c->streamM2 && G > sms && c->tune_groups != 1;
-    const bool la = c->tune_lookahead != 0;
-    if (!split)
+  // Gauss-Jordan: per panel the factor kernel chooses the pivots and forms T =
+  // A11^{-1}, the block row becomes T [A12 | B1] and one product eliminates the
+  // panel columns from all other rows; no back substitution follows.
+  const SolveShape shape = solve_shape(n, G, g_gemm_mode, c->tune_groups, c->tune_cap, c->tune_lookahead);
+  if (shape.gauss_jordan) {
+    const bool la = shape.lookahead;
+    if (!shape.split)
       return gj_solve_range(c, 0, G, nb, s, nullptr, la ? c->streamB[0] : nullptr, c->ev_la[0][0], c->ev_la[0][1]);
     const int G1 = (G + 1) / 2, G2 = G - G1;
-    TcGridCap cap(c->tune_cap == 2 ? 0 : c->tune_cap == 1 ? sms / 2 : std::max(sms - G1, sms / 2));
+    TcGridCap cap(shape.cap);
     if ((rc = gj_solve_range(c, 0, G1, nb, s, c->ev_stagger, la ? c->streamB[0] : nullptr, c->ev_la[0][0],
                              c->ev_la[0][1])))
       return rc;

@@ -654,14 +654,40 @@ int tvap_autotune(tvap_ctx* c, const double* U0, const double* V0, const tvap_pr
       for (int groups = 2; groups >= 1; --groups)
         for (int cap = 0; cap < (groups == 2 ? 3 : 1); ++cap)
           for (int bn = 0; bn < 3; ++bn) cands.push_back({bn, groups, cap, la, pf});
+  // Candidates differ only where the size, the angles and the arithmetic let
+  // them: those that launch the same program are timed once and share its
+  // time, so that the choice is one between programs.
+  struct Program {
+    SolveShape solve;
+    bool one_half, pf_blocked;
+    double ms;
+  };
+  std::vector<Program> programs;
+  tvap_pnp out{};
+  int rc;
+  if ((rc = tvap_project(c, U0, V0, opts, &out, nullptr))) return rc;  // (the order of its Pfaffians)
+  const int G = opts->mode == 0 ? angle_count(*opts) : 1, npf = c->n - out.nocc - out.nemp;
+  auto program = [&](const Cand& k) -> Program& {
+    const SolveShape q = solve_shape(c->n, G, c->gemm_mode, k.groups, k.cap, k.la);
+    const bool one_half = c->gemm_mode == 2 && k.bn == 2, pf = k.pf != 0 || !pfaffian_in_smem(npf);
+    for (Program& p : programs)
+      if (p.solve.split == q.split && p.solve.cap == q.cap && p.solve.lookahead == q.lookahead &&
+          p.one_half == one_half && p.pf_blocked == pf)
+        return p;
+    programs.push_back({q, one_half, pf, 0.0});
+    return programs.back();
+  };
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   TVAP_CUDA(cudaEventCreate(&e0));
   TVAP_CUDA(cudaEventCreate(&e1));
-  int rc = TVAP_OK;
   double best = 1e300;
   Cand chosen = {c->tune_bn, c->tune_groups, c->tune_cap, c->tune_lookahead, c->tune_pf_blocked};
-  tvap_pnp out{};
   for (size_t k = 0; k < cands.size() && rc == TVAP_OK; ++k) {
+    Program& p = program(cands[k]);
+    if (p.ms > 0.0) {
+      if (table_ms && int(k) < ntable) table_ms[k] = p.ms;
+      continue;
+    }
     c->tune_bn = cands[k].bn;
     c->tune_groups = cands[k].groups;
     c->tune_cap = cands[k].cap;
@@ -675,6 +701,7 @@ int tvap_autotune(tvap_ctx* c, const double* U0, const double* V0, const tvap_pr
     float ms = 0.f;
     cudaEventElapsedTime(&ms, e0, e1);
     const double per = double(ms) / reps;
+    p.ms = per;
     if (table_ms && int(k) < ntable) table_ms[k] = per;
     if (per < best) {
       best = per;

@@ -391,6 +391,17 @@ enum Section : int {
   SEC_CANONICAL = 0, SEC_BLOCKS, SEC_SOLVE, SEC_UV, SEC_DENSITIES, SEC_FIELDS_GAMMA, SEC_FIELDS_DELTA, SEC_TRACES,
   SEC_H20, SEC_OVERLAP, SEC_PFAFFIAN, SEC_SUMS, SEC_GRADIENT, SEC_EVOLVE, SEC_H20_TC, SEC_COUNT
 };
+// What the launch shapes of tvap_autotune come to in the Thouless solve of G
+// angles (projection.cu): candidates that agree here launch the same program.
+struct SolveShape {
+  bool gauss_jordan;  // blocked Gauss-Jordan; else none of the following
+  bool split;         // two groups of angles on two streams
+  int cap;            // tcgen05 CTAs beside the second group's panels (0: no cap), with split
+  bool lookahead;
+};
+SolveShape solve_shape(int n, int G, int gemm_mode, int groups, int cap, int lookahead);
+// pfaffian_batched takes the shared-memory form for matrices of n rows
+bool pfaffian_in_smem(int n);
 // Waits for every stream of the context.
 void sync_streams(tvap_ctx* c);
 // The result of a call that forks chains onto the context's streams: on an
