@@ -124,8 +124,9 @@ int tvap_set_timing(tvap_ctx* ctx, int on);
  * or column, exact FP32 partial sums, integer recombination; error bound at
  * tvap_zgemm) with warp-level mma.sync; 2 (default) = the same splitting
  * with tcgen05 MMAs and tensor-memory accumulators for the batched products
- * (those of few tiles keep the mma.sync kernel).  Products of up to 1.2 10^7
- * FP64 multiply-adds run on the FP64 pipe in every mode.  In modes 1 and 2 the
+ * (those of few tiles keep the mma.sync kernel).  Products of few FP64
+ * multiply-adds (at most 1.2 10^7; the rule stands in csrc/gemm_route.h) run on
+ * the FP64 pipe in every mode.  In modes 1 and 2 the
  * field contraction over 16 or more gauge angles also runs on the tensor
  * cores (dense symmetry blocks of the interaction); the factorisations and
  * all reductions run on the FP64 pipe in every mode. */
@@ -387,7 +388,9 @@ int tvap_zskpfa_batched(tvap_ctx* ctx, int batch, int64_t n, const double* A, do
  * arithmetic the context uses for the path's own products
  * (tvap_set_gemm_mode).  Host or device memory; the call returns when C is
  * written.  In modes 1 and 2 a product with K >= 16 and more than 1.2 10^7
- * FP64 multiply-adds (complex x complex counts 3 per element, tvap_dgemm 1)
+ * FP64 multiply-adds (complex x complex counts 3 per element, tvap_dgemm 1),
+ * or with at least 10^6 of M N K and so many outputs for its K that the FP64
+ * pipe is the slower side (csrc/gemm_route.h),
  * is emulated on the tensor cores: every row i of op(A) and
  * column j of op(B) gets one power-of-two scale 2^e (2^e <= its largest
  * entry), each entry is rounded to an integer multiple of 2^(e-53) (error

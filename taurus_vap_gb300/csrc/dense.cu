@@ -13,6 +13,7 @@
 #include <utility>
 #include <vector>
 
+#include "gemm_route.h"
 #include "tvap_internal.cuh"
 
 namespace tvap {
@@ -236,9 +237,6 @@ template <typename TA, typename TB>
 __host__ __device__ constexpr int small_kc() {
   return sizeof(TA) + sizeof(TB) > 24 ? 96 : sizeof(TA) + sizeof(TB) > 16 ? 128 : 192;
 }
-// double precision multiply-adds of a product up to which it runs here
-constexpr double kSmallWork = 1.2e7;
-
 template <typename T>
 __device__ __forceinline__ void stage_small(T* dst, const View& v, bool rows_first, int r0, int rows, int k0, int kt,
                                             long long b, bool conj) {
@@ -318,9 +316,13 @@ __global__ void __launch_bounds__(kSmallThreads) small_gemm_kernel(GemmArgs g, u
   }
 }
 
-// FP64 multiply-adds of a product (a complex one in the 3M form)
-double real_work(const GemmArgs& g) {
-  return double(g.M) * g.N * (double(g.K) + g.K2) * g.batch * ((g.a_real ? 1 : 2) + (g.b_real ? 1 : 2) - 1);
+// small_product for these arguments in the calling thread's arithmetic
+bool is_small(const GemmArgs& g) {
+  const int K = g.K + (g.K2 > 0 ? g.K2 : 0);
+  const Route other = g_gemm_mode == 0 || K < 16             ? Route::fp64_tiles
+                      : g_gemm_mode == 2 && tc_takes(g) ? Route::tcgen05
+                                                        : Route::mma_sync;
+  return small_product(g.M, g.N, K, g.batch, (g.a_real ? 1 : 2) + (g.b_real ? 1 : 2) - 1, g.upper_only, other);
 }
 
 void launch_small_gemm(const GemmArgs& g, cudaStream_t s) {
@@ -405,12 +407,7 @@ int gemm_split_k2(const GemmArgs& g, cudaStream_t s) {
 
 int gemm(const GemmArgs& g, cudaStream_t s) {
   if (g.M <= 0 || g.N <= 0 || g.batch <= 0) return TVAP_OK;
-  // Up to kSmallWork FP64 multiply-adds a product runs on the FP64 pipe in
-  // every mode (small_gemm_kernel): 1.2e7 take 20 us on the whole chip, about
-  // what the emulated form's two slicing passes and its product need at least
-  // (real n = 140, 2.7e6: 15.6 us against 27; n = 336, 3.8e7: at least 63 us
-  // against 50).  Larger ones run emulated on the tensor cores.
-  const bool small = real_work(g) <= kSmallWork;
+  const bool small = is_small(g);  // on the FP64 pipe in every mode
   if (g.K2 > 0) {
     if (g_gemm_mode == 2 && !small) return gemm_ozaki(g, s);
     return gemm_split_k2(g, s);

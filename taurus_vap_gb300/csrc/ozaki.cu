@@ -617,15 +617,39 @@ static_assert(kPairsMinK == oztc::kFoldKs * 16 / 2 + 1, "the paired form from ha
 
 inline bool g_alpha_unit(double a) { return a == 1.0 || a == -1.0; }
 
+// Tiles of 128 x 64 of the tcgen05 kernel for a product; 0 when it is not of a
+// supported kind.  The paired form has twice the tiles of half the k-steps; it
+// is counted in tiles of the real representation, so that both forms route
+// the same products here.
+long long tc_tiles(const GemmArgs& g) {
+  const bool real_scalars = g.alpha.y == 0.0 && g.beta.y == 0.0 && !g.alpha_vec;
+  if (!real_scalars || (g.a_real && g.b_real && !g.c_real)) return 0;
+  const bool a_sh = g.A.bs == 0 && g.batch > 1, b_sh = g.B.bs == 0 && g.batch > 1;
+  if (a_sh && b_sh) return 0;
+  if (g.K2 > 0 && ((g.A2.bs == 0) != (g.A.bs == 0) || (g.B2.bs == 0) != (g.B.bs == 0))) return 0;
+  // (the slicing pass holds 8 rows in shared memory at least)
+  const int K = g.K + (g.K2 > 0 ? g.K2 : 0);
+  if (sizeof(double2) * (size_t(K | 1) << slice_rshift(K, !g.a_real || !g.b_real)) > size_t(227) * 1024) return 0;
+  const bool stack = a_sh || b_sh, l_real = a_sh ? g.b_real : g.a_real, r_real = a_sh ? g.a_real : g.b_real;
+  const long long l_rows = a_sh ? g.N : g.M, r_rows = a_sh ? g.M : g.N;
+  const long long rows = l_rows * (l_real ? 1 : 2) * (stack ? g.batch : 1);
+  const long long cols = r_rows * (l_real && !r_real ? 2 : 1);
+  return (rows + oztc::kM - 1) / oztc::kM * ((cols + 2 * oztc::kHalf - 1) / (2 * oztc::kHalf)) * (stack ? 1 : g.batch);
+}
+
 // The tensor-memory path for one product (mode 2).  Returns TVAP_ERR_ARG
 // without launching anything when the product is not of a supported kind.
 // With upper_only the whole product is formed (the lower triangle is
 // written too; its readers ignore it).
 int gemm_tc(const GemmArgs& g, cudaStream_t s) {
-  const bool real_scalars = g.alpha.y == 0.0 && g.beta.y == 0.0 && !g.alpha_vec;
-  if (!real_scalars || (g.a_real && g.b_real && !g.c_real)) return TVAP_ERR_ARG;
+  // The tile route wins long before it has a tile for every SM (slicing and
+  // product, 32 x 32 mma.sync tiles / this route, us): 1024 x 640 x 140 real 53
+  // / 29, 512 x 384 x 336 real 60 / 38, 512 x 256 x 140 complex 42 / 23, 16 tiles
+  // of 512 x 256 x 140 real 28 / 29, 8 of 256 x 128 x 140 complex 43 / 23;
+  // products of fewer tiles that are not small ones (small_product) are thin
+  // ones.
+  if (tc_tiles(g) < kTcMinTiles) return TVAP_ERR_ARG;
   const bool a_sh = g.A.bs == 0 && g.batch > 1, b_sh = g.B.bs == 0 && g.batch > 1;
-  if (a_sh && b_sh) return TVAP_ERR_ARG;
   // rows of op(A): element (i, k) at A.p[i rs + k cs]; rows of op(B)^T:
   // element (j, k) at B.p[k rs + j cs].  With a shared A the transposed
   // product C^T = op(B)^T op(A)^T is formed, so that the per-batch operand is
@@ -638,7 +662,6 @@ int gemm_tc(const GemmArgs& g, cudaStream_t s) {
     const void* p2;
     long long sr2, sk2, bs2;
   };
-  if (g.K2 > 0 && ((g.A2.bs == 0) != (g.A.bs == 0) || (g.B2.bs == 0) != (g.B.bs == 0))) return TVAP_ERR_ARG;
   Side L{g.A.p, g.A.rs, g.A.cs, g.A.bs, g.M, g.a_real, g.conj_a, g.A2.p, g.A2.rs, g.A2.cs, g.A2.bs};
   Side R{g.B.p, g.B.cs, g.B.rs, g.B.bs, g.N, g.b_real, g.conj_b, g.B2.p, g.B2.cs, g.B2.rs, g.B2.bs};
   long long crs = g.crs, ccs = g.ccs;
@@ -697,16 +720,6 @@ int gemm_tc(const GemmArgs& g, cudaStream_t s) {
   if (nks > oztc::kMaxKs) return TVAP_ERR_ARG;
   const size_t asz = size_t(a_slots) * (a_rows_pad / oztc::kM) * nks * (oztc::kABytes / 2);
   const size_t bsz = size_t(b_slots) * b_halves * nks * (oztc::kBBytes / 2);
-  // The tile route wins long before it has a tile for every SM (slicing and
-  // product, 32 x 32 mma.sync tiles / this route, us): 1024 x 640 x 140 real 53
-  // / 29, 512 x 384 x 336 real 60 / 38, 512 x 256 x 140 complex 42 / 23, 16 tiles
-  // of 512 x 256 x 140 real 28 / 29, 8 of 256 x 128 x 140 complex 43 / 23;
-  // products of fewer tiles that are not small ones (small_gemm_kernel) are
-  // thin ones.  The paired form has twice the tiles of half the k-steps; it is
-  // counted in tiles of the real representation, so that both forms route the
-  // same products here.
-  if (size_t(a_rows_pad / oztc::kM) * ((b_halves + 1) / 2) * a_slots / (pairs ? 2 : 1) < size_t(kTcMinTiles))
-    return TVAP_ERR_ARG;
   int rc;
   OzScratch* sc = nullptr;
   if ((rc = oz_reserve(s, sizeof(__nv_bfloat16) * (asz + bsz), size_t(a_slots) * a_rows_pad +
@@ -720,7 +733,6 @@ int gemm_tc(const GemmArgs& g, cudaStream_t s) {
   const int rshift = slice_rshift(K, !L.real || !R.real);
   const size_t slice_shm = sizeof(double2) * (size_t(K | 1) << rshift);
   if (slice_shm > 48 * 1024) {
-    if (slice_shm > size_t(227) * 1024) return TVAP_ERR_ARG;
     if ((rc = smem_opt_in((const void*)slice_tc_kernel, slice_shm))) return rc;
   }
   LeftSlice left;
@@ -783,6 +795,8 @@ int gemm_tc(const GemmArgs& g, cudaStream_t s) {
 }
 
 }  // namespace
+
+bool tc_takes(const GemmArgs& g) { return tc_tiles(g) >= kTcMinTiles; }
 
 // Returns TVAP_OK after launching, or TVAP_ERR_ARG when the shape is not
 // supported (the caller then uses the FP64 pipe).

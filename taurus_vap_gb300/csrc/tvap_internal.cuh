@@ -200,6 +200,8 @@ int gemm(const GemmArgs& g, cudaStream_t s);
 int gemm_split_k2(const GemmArgs& g, cudaStream_t s);
 // the same product with the FP64 arithmetic emulated on the bf16 tensor cores
 int gemm_ozaki(const GemmArgs& g, cudaStream_t s);
+// in mode 2 the tcgen05 kernel takes the product (kind of operands, tiles)
+bool tc_takes(const GemmArgs& g);
 void oz_release(cudaStream_t s);
 // per-stream scratch of the emulated products (grown on demand, stream-ordered)
 int oz_scratch(cudaStream_t s, size_t bytes, size_t ex_count, __nv_bfloat16** buf, int** ex);
