@@ -19,7 +19,8 @@ namespace tvap {
 // 0 factors each diagonal block, all CTAs solve the panel rows below it and
 // apply the trailing update (CTA 0 updating and factoring the next diagonal
 // block meanwhile); then one warp per row of A1 / A2 runs the forward
-// substitution L x = a with L in shared memory.  Grid-wide barriers between
+// substitution L x = a, L read through L2 (beyond kNewtonMaxN it does not fit
+// shared memory).  Grid-wide barriers between
 // the phases are bounded spins (all CTAs are co-resident by the cooperative
 // launch); a barrier that gives up raises the status word and every CTA
 // returns.
@@ -127,10 +128,10 @@ __device__ bool coop_factor_diag(int n, double* S, double* rd, int j0, int nb, d
 // grid (coop_barrier with bar and the caller's generation).  X_m = A_m L^{-T}
 // for m = 0 (A at A, X at X) and m = 1 (A + a_stride, X + x_stride); with
 // Linv != null also L^{-1} (row r of L^{-T} solves for the unit row e_r).
-// coop_smem holds L (n x n, when l_smem; else the panel rows) and 1 / L_jj.
+// coop_smem holds the panel rows, then 1 / L_jj.
 template <int SLOTS>
 __device__ void evolve_by_blocks(int n, double* S, const double* A, long long a_stride, double* X, long long x_stride,
-                                 double* Linv, unsigned* bar, unsigned gen, int* flags, int skip_cta, int l_smem,
+                                 double* Linv, unsigned* bar, unsigned gen, int* flags, int skip_cta,
                                  double* coop_smem) {
   __shared__ double L11[kCoopNb][kCoopNb + 1];
   __shared__ double rdiag[kCoopNb];
@@ -222,24 +223,8 @@ __device__ void evolve_by_blocks(int n, double* S, const double* A, long long a_
   const int warps = blockDim.x >> 5, warp = t >> 5, lane = t & 31;
   const int rows = (Linv ? 3 : 2) * n;
   if (cta >= rows) return;
-  // L from shared memory when it fits (n <= 168), else from L2 (S is
-  // written by this grid before the last barrier: read through L2, not L1)
-  double* Ls = coop_smem;
-  double* dinv = l_smem ? Ls + size_t(n) * n : coop_smem;
-  if (l_smem) {
-    if ((reinterpret_cast<uintptr_t>(S) & 15) == 0) {
-      // 16-byte loads, many in flight
-      const int nn2 = (n * n) / 2;
-      const double2* S2 = reinterpret_cast<const double2*>(S);
-      double2* L2 = reinterpret_cast<double2*>(Ls);
-#pragma unroll 16
-      for (int idx = t; idx < nn2; idx += blockDim.x) L2[idx] = __ldcg(&S2[idx]);
-      if (((n * n) & 1) && t == 0) Ls[n * n - 1] = __ldcg(&S[n * n - 1]);
-    } else {
-#pragma unroll 16
-      for (int idx = t; idx < n * n; idx += blockDim.x) Ls[idx] = __ldcg(&S[idx]);
-    }
-  }
+  // S is written by this grid before the last barrier: read through L2, not L1
+  double* dinv = coop_smem;
   __syncthreads();
   for (int j = t; j < n; j += blockDim.x) dinv[j] = __ldcg(&rd[j]);
   __syncthreads();
@@ -269,16 +254,16 @@ __device__ void evolve_by_blocks(int n, double* S, const double* A, long long a_
         const int owner = j & 31;
         const double xj = __shfl_sync(0xffffffffu, v[qj], owner) * dinv[j];
         if (lane == owner) v[qj] = xj;
-        const double* lc = (l_smem ? Ls : S) + size_t(j) * n;
+        const double* lc = S + size_t(j) * n;
         {
           const int jj = lane + 32 * qj;
-          if (jj > j && jj < n) v[qj] = fma(-xj, l_smem ? lc[jj] : __ldcg(&lc[jj]), v[qj]);
+          if (jj > j && jj < n) v[qj] = fma(-xj, __ldcg(&lc[jj]), v[qj]);
         }
 #pragma unroll
         for (int q = qj + 1; q < kMaxPerLane; ++q) {
           if (32 * q >= n) break;
           const int jj = lane + 32 * q;
-          if (jj < n) v[q] = fma(-xj, l_smem ? lc[jj] : __ldcg(&lc[jj]), v[q]);
+          if (jj < n) v[q] = fma(-xj, __ldcg(&lc[jj]), v[q]);
         }
       }
     }
@@ -313,7 +298,7 @@ constexpr int kNewtonSteps = 6;
 constexpr float kNewtonLast = 1e-10f, kNewtonUsable = 0.05f;
 
 struct EvolveArgs {
-  int n, newton, skip_cta, l_smem;
+  int n, newton, skip_cta;
   const double *Z, *U0, *V0;
   double *S, *A, *X0, *X1, *T, *E;  // S: n^2 + n; A: A1 then A2; X0, X1, T, E: n^2 each (newton only)
   double *U1, *V1, *Linv;           // Linv may be null
@@ -638,7 +623,7 @@ __global__ void __launch_bounds__(kCoopThreads, 1) thouless_evolve_kernel(Evolve
   unsigned gen = 0;  // barriers passed
   if (!p.newton) {
     evolve_by_blocks<SLOTS>(n, p.S, p.A, (long long)n * n, p.U1, p.V1 - p.U1, p.Linv, p.bar, gen, p.flags, p.skip_cta,
-                            p.l_smem, evolve_smem);
+                            evolve_smem);
     return;
   }
   const size_t nn = size_t(n) * n;
@@ -741,7 +726,7 @@ __global__ void __launch_bounds__(kCoopThreads, 1) thouless_evolve_kernel(Evolve
     Xn = swap;
   }
   if (!good) {
-    evolve_by_blocks<SLOTS>(n, p.S, p.A, (long long)nn, p.U1, p.V1 - p.U1, p.Linv, p.bar, gen, p.flags, -1, 0,
+    evolve_by_blocks<SLOTS>(n, p.S, p.A, (long long)nn, p.U1, p.V1 - p.U1, p.Linv, p.bar, gen, p.flags, -1,
                             evolve_smem);
     return;
   }
@@ -784,19 +769,13 @@ int thouless_evolve(int n, const double* Z, const double* U0, const double* V0, 
   p.Linv = Linv;
   p.bar = bar;
   p.flags = flags;
-  // shared memory: the FP32 stage's steps, the tiles' operands, the
-  // blocks' panel rows; without Newton steps L for the blocks' solves when it
-  // fits (else the panel rows, L read from L2)
-  const size_t panel = sizeof(double) * (nn / n * kCoopNb + n);
-  size_t shm = panel;
+  // shared memory: the FP32 stage's steps, the tiles' operands, the blocks'
+  // panel rows
+  size_t shm = sizeof(double) * (size_t(n) * kCoopNb + n);
   if (p.newton) {
     static_assert(kNewtonMaxN <= 32 * kF32MaxSlots, "the FP32 stage holds the matrix");
     shm = std::max(shm, sizeof(double) * n + sizeof(float) * (kF32Ring * (64 * kF32MaxSlots + 2) + n + 1 + nn));
     shm = std::max(shm, sizeof(double) * kBatch * (size_t(n) * kTileElems + kCoopThreads));
-  } else {
-    const size_t full = sizeof(double) * (nn + n);
-    p.l_smem = full <= jacobi32_smem_limit() ? 1 : 0;
-    if (p.l_smem) shm = full;
   }
   if (n > 384 || shm > jacobi32_smem_limit()) return TVAP_ERR_ARG;
   const int slots = (n + 31) / 32;
