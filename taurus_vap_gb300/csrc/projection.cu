@@ -2297,10 +2297,13 @@ Panels solve_panels(int n, int gemm_mode) {
 // products.  The products leave SMs for them (their CTAs are capped at
 // the SMs the other half's panels do not hold: a panel CTA and a product
 // CTA do not fit one SM).  While the panels of all angles run at once,
-// twice the launches of half the size cost more than the overlap gives.
-// Iterations in one and in two halves: n = 24, 113 angles 0.640 / 0.665
-// ms; n = 80, 39 angles 1.54 / 1.60; n = 140, 41 angles 2.96 / 3.03, 113
-// 4.11 / 4.13, 221 6.51 / 6.47.
+// twice the launches of half the size cost more than the overlap gives:
+// iterations in one and in two halves n = 24, 113 angles 0.640 / 0.665 ms;
+// n = 80, 39 angles 1.54 / 1.60; n = 140, 41 angles 2.96 / 3.03, 113 4.11 /
+// 4.13.  Above the SMs the halves give little and only at the larger n (181,
+// 221 and 313 angles): n = 24 0.68 / 0.69, 0.71 / 0.72; n = 80 2.01 / 2.02,
+// 2.31 / 2.32, 3.06 / 3.06; n = 140 5.38 / 5.38, 6.26 / 6.25, 8.60 / 8.46; n =
+// 224 13.75 / 13.66, 16.4 / 16.3; n = 336 37.7 / 37.1, 44.7 / 44.6.
 // The look-ahead has a panel to work on where there are two.
 SolveShape solve_shape(int n, int G, int gemm_mode, int groups, int cap, int lookahead) {
   const Panels p = solve_panels(n, gemm_mode);
