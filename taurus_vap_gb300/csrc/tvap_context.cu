@@ -80,7 +80,8 @@ double* ws_V(tvap_ctx* c);
 double* ws_H20v(tvap_ctx* c);
 
 void sync_streams(tvap_ctx* c) {
-  for (cudaStream_t st : {c->stream, c->stream2, c->stream3, c->streamM, c->streamM2, c->streamB[0], c->streamB[1]})
+  cudaStreamSynchronize(c->stream);  // (null: the default stream, a caller's choice)
+  for (cudaStream_t st : {c->stream2, c->stream3, c->streamM, c->streamM2, c->streamB[0], c->streamB[1]})
     if (st) cudaStreamSynchronize(st);
 }
 

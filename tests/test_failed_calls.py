@@ -36,6 +36,18 @@ def test_chains_are_forked_under_settle():
     assert tail.index("settle(c, run())") < tail.index("return")
 
 
+def test_every_stream_is_waited_for():
+    src = open(os.path.join(CSRC, "tvap_context.cu")).read()
+    body = re.search(r"^void sync_streams\(.*?^\}", src, re.M | re.S).group(0)
+    ctx = open(os.path.join(CSRC, "tvap_internal.cuh")).read()
+    ctx = ctx[ctx.index("struct tvap_ctx {"):]
+    streams = set(re.findall(r"cudaStream_t (\w+)(?:\[\d\])? = ", ctx[:ctx.index("\n};")]))
+    assert streams == {"stream", "stream2", "stream3", "streamM", "streamM2", "streamB"}
+    assert all(f"c->{k}" in body for k in streams)
+    # the caller may have set the default stream, whose handle is null
+    assert re.search(r"^  cudaStreamSynchronize\(c->stream\);", body, re.M)
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("call", ["observables", "projection"])
 def test_projection_after_an_error(call):
