@@ -565,6 +565,7 @@ int oz_reserve(cudaStream_t s, size_t bytes, size_t ex_count, OzScratch** out) {
       cudaFree(sc->buf);
     }
     sc->buf = nullptr;
+    sc->bytes = 0;  // (a failed allocation must not leave the size of what was freed)
     TVAP_CUDA(cudaMalloc(&sc->buf, bytes));
     sc->bytes = bytes;
     sc->left.valid = false;
@@ -575,6 +576,7 @@ int oz_reserve(cudaStream_t s, size_t bytes, size_t ex_count, OzScratch** out) {
       cudaFree(sc->ex);
     }
     sc->ex = nullptr;
+    sc->ex_count = 0;
     TVAP_CUDA(cudaMalloc(&sc->ex, ex_count * sizeof(int)));
     sc->ex_count = ex_count;
     sc->left.valid = false;

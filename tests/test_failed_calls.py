@@ -48,6 +48,19 @@ def test_every_stream_is_waited_for():
     assert re.search(r"^  cudaStreamSynchronize\(c->stream\);", body, re.M)
 
 
+@pytest.mark.parametrize("source,pointer,size", [("ozaki.cu", "sc->buf", "sc->bytes"),
+                                                 ("ozaki.cu", "sc->ex", "sc->ex_count"),
+                                                 ("tvap_context.cu", "c->scratch", "c->scratch_count"),
+                                                 ("tvap_context.cu", "c->fields_buf", "c->fields_bytes")])
+def test_a_failed_growth_leaves_no_size_behind(source, pointer, size):
+    # grown buffers are freed first: were the old size kept when the allocation fails, the next call would find the
+    # null pointer large enough
+    src = open(os.path.join(CSRC, source)).read()
+    at = src.index(f"cudaMalloc(&{pointer},")
+    before = src[src.rindex(f"cudaFree({pointer})", 0, at):at]
+    assert re.search(re.escape(pointer) + r" = nullptr;", before) and re.search(re.escape(size) + r" = 0;", before)
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("call", ["observables", "projection"])
 def test_projection_after_an_error(call):
